@@ -617,6 +617,7 @@ __global__ void decode_end_gather_kernel(const TpExchange* xcp, DecodeState* sta
 #include "linear_stream.cuh"
 #include "linear_chain.cuh"
 #include "linear_gemm.cuh"
+#include "linear_gemm_pair.cuh"
 #include "linear_gemm_small.cuh"
 
 namespace kmll {
@@ -899,38 +900,17 @@ static void chain_plain_phase(ChainPhase& ph, int epi, const float* x, const uin
     ph.total_units = units;
 }
 
-// ---- tcgen05 GEMM path (linear_gemm.cuh) ------------------------------------------------------------------------
+// ---- tcgen05 GEMM path (linear_gemm_pair.cuh, linear_gemm_small.cuh) ---------------------------------------------
 struct GemmPlan {
-    int n_block, x_blocks, row_tiles, ksplit, stages;
-    size_t smem;
+    int n_block;  // rows of x that a partial tile of the workspace has room for
     size_t off_lo, off_inv, off_partial, off_counters, total;  // workspace layout in bytes
 };
 static bool gemm_plan(int fmt, int M, int K, int rows, GemmPlan* out) {
     if (M < 5 || K % kGKT != 0 || (fmt == FMT_W4 && K % 128 != 0) || rows <= 0) return false;
     GemmPlan pl;
-    pl.x_blocks = (M + kGMaxN - 1) / kGMaxN;
-    pl.n_block = (((M + pl.x_blocks - 1) / pl.x_blocks) + 15) & ~15;
-    pl.row_tiles = (rows + kGRows - 1) / kGRows;
-    const int tiles = pl.row_tiles * pl.x_blocks, kt_all = K / kGKT;
-    pl.ksplit = 1;
-    if (tiles < 148) {  // few tiles (a narrow matrix, or few rows of x): split K so that every multiprocessor has work
-        pl.ksplit = 148 / tiles;
-        if (pl.ksplit > kGMaxSplit) pl.ksplit = kGMaxSplit;
-        // a split must bring more than its merge costs (the last block of a tile reads every partial back): at least 8 k-tiles
-        // per split for narrow blocks of x, 32 for wide ones (measured: 3584 x 3584 at 256 rows loses with 5 splits of 11
-        // k-tiles, 3584 x 18944 doubles its rate with 5 splits of 59)
-        const int min_kt = pl.n_block <= 64 ? 8 : 32;
-        if (pl.ksplit > kt_all / min_kt) pl.ksplit = kt_all / min_kt;
-        if (pl.ksplit < 1) pl.ksplit = 1;
-    }
-    // (raw weight tiles with 128-byte rows in a ring of their own - 4 k-tiles of W4, 2 of RS-I8 per TMA box - were measured
-    // and brought nothing: the small-batch shapes are bound by the per-k-tile hand-offs, not by the row pieces TMA moves)
-    const size_t raw = fmt == FMT_W4 ? 4096 : 8192;
-    const size_t stage = (size_t)(fmt == FMT_W4 ? 2 : 1) * kGRows * 128 + (size_t)2 * pl.n_block * 128 + raw;
-    pl.stages = (int)((220 * 1024 - 2048) / stage);
-    if (pl.stages > 8) pl.stages = 8;
-    if (pl.stages < 2) return false;
-    pl.smem = (size_t)pl.stages * stage + (3 * pl.stages + 1) * 8 + 16 + 1024;  // + slack for the 1024-byte alignment
+    const int x_blocks = (M + kGMaxN - 1) / kGMaxN;
+    pl.n_block = (((M + x_blocks - 1) / x_blocks) + 15) & ~15;
+    const int tiles = (rows + 127) / 128 * x_blocks;
     auto up256 = [](size_t v) { return (v + 255) & ~(size_t)255; };
     pl.off_lo = (size_t)M * K * 2;  // the two f16 planes of x are contiguous: one 3-D tensor [2, M, K]
     pl.off_inv = up256(pl.off_lo * 2);
@@ -938,7 +918,7 @@ static bool gemm_plan(int fmt, int M, int K, int rows, GemmPlan* out) {
     // the layout depends on (M, K) only, so one workspace serves matrices of any height: split-K keeps tiles * splits
     // at or below 148 partial tiles; 16384 arrival counters
     if (tiles > 16384) return false;
-    size_t partial_bytes = (size_t)148 * pl.n_block * kGRows * 4;
+    size_t partial_bytes = (size_t)148 * pl.n_block * 128 * 4;
     if (M <= 32) {  // the small-batch kernel (linear_gemm_small.cuh) keeps up to kSMaxUnits partial tiles
         const size_t small = (size_t)kBtMaxUnits * (M <= 16 ? 16 : 32) * 128 * 4;
         partial_bytes = small > partial_bytes ? small : partial_bytes;
@@ -947,6 +927,43 @@ static bool gemm_plan(int fmt, int M, int K, int rows, GemmPlan* out) {
     pl.total = pl.off_counters + 16384 * 4;
     *out = pl;
     return true;
+}
+
+// Shape of one launch of linear_gemm_pair_kernel over `tiles` 256-row tiles: x blocks and k-splits that keep 74 pairs of
+// multiprocessors busy.  Cost in SM cycles, fitted to stamps inside the kernel: a 64-column k-tile is eight MMAs of n / 2 + 15
+// cycles (four of n + 15 up to 128 rows of x), but not less than the hand-over chain between the roles (W4: accumulator full ->
+// drained -> free, ~770 cycles per k-tile; RS-I8 ~560); a W4 unit ends in ~40 n cycles of stores that its successor's MMAs
+// can overlap only for two groups; a split adds the merge through L2.
+struct PairPlan { int n_block, x_blocks, ksplit, units, stages; size_t smem; };
+static PairPlan pair_plan(int fmt, int M, int K, int tiles, int n_max_split) {
+    PairPlan best;
+    memset(&best, 0, sizeof(best));
+    double best_cost = 1e30;
+    const int items = K / (fmt == FMT_W4 ? 128 : 64), kt_all = K / kGKT;
+    const int xb_min = (M + kGMaxN - 1) / kGMaxN, xb_max = xb_min * 4;
+    for (int xb = xb_min; xb <= xb_max; ++xb) {
+        const int n = (((M + xb - 1) / xb) + 15) & ~15;
+        if (xb > xb_min && n < 64) break;
+        const int xblocks = (M + n - 1) / n;
+        for (int ks = 1; ks <= kGMaxSplit && ks <= items; ++ks) {
+            const long long units = (long long)tiles * xblocks * ks;
+            if (ks > 1 && (units > kPClusters || n > n_max_split)) break;  // the workspace holds 148 partial tiles of 128 rows
+            const double rounds = (double)((units + kPClusters - 1) / kPClusters);
+            const double kt = (double)((kt_all + ks - 1) / ks), chain = fmt == FMT_W4 ? 770.0 : 560.0;
+            const double mma = 4.0 * n + (2 * n <= kGMaxN ? 60.0 : 120.0);
+            const double unit = kt * (mma > chain ? mma : chain) + (fmt == FMT_W4 ? 40.0 * n : 2000.0);
+            const double cost = rounds * unit + (ks > 1 ? 3000.0 + 12.0 * n * ks : 0.0);
+            if (cost < best_cost * 0.995) {
+                best_cost = cost;
+                best.n_block = n; best.x_blocks = xblocks; best.ksplit = ks; best.units = (int)units;
+            }
+        }
+    }
+    const size_t stage = (size_t)128 * 128 + (size_t)best.n_block * 128 + (fmt == FMT_W4 ? 4096 : 8192);
+    best.stages = (int)((size_t)(227 * 1024 - 1024 - 512) / stage);
+    if (best.stages > 8) best.stages = 8;
+    best.smem = best.stages * stage + (3 * best.stages + 4) * 8 + 16 + 1024;  // + slack for the 1024-byte alignment
+    return best;
 }
 
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -1127,40 +1144,47 @@ static int run_gemm(cudaStream_t stream, const float* x, int M, int K, int ldx, 
     cudaError_t e = launch(split_rows_kernel, dim3(M), dim3(512), 0, stream, true, x, ldx, K, norm_w, eps, x_hi, x_lo, inv, counters, n_counters,
                            FMT == FMT_W4 ? 1 : 0);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "split_rows: %s", cudaGetErrorString(e));
-    auto kern = linear_gemm_kernel<FMT>;
-    for (int i = 0; i < nmat; ++i) {
-        GemmPlan pl;
-        if (!gemm_plan(FMT, M, K, rows[i], &pl)) return fail(KMLL_ERR_UNSUPPORTED, "linear_batched: shape not supported by the tensor-core path");
-        CUtensorMap map_w, map_x;
-        if (FMT == FMT_W4) KMLL_TRY_RC(make_map_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w[i], (uint64_t)K / 2, (uint64_t)rows[i], (uint64_t)K / 2, 32, kGRows, CU_TENSOR_MAP_SWIZZLE_NONE));
-        else KMLL_TRY_RC(make_map_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w[i], (uint64_t)K, (uint64_t)rows[i], (uint64_t)K, 64, kGRows, CU_TENSOR_MAP_SWIZZLE_NONE));
-        {   // both f16 planes of x as one 3-D tensor [2, M, K]; box = [2, n_block, 64 columns], 128-byte swizzle
-            TensorMapEncodeFn enc = tensor_map_encoder();
-            if (enc == nullptr) return fail(KMLL_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-            const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, 2};
-            const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)M * K * 2};
-            const cuuint32_t box[3] = {kGKT, (cuuint32_t)pl.n_block, 2};
-            const cuuint32_t estr[3] = {1, 1, 1};
-            const CUresult r = enc(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, x_hi, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return fail(KMLL_ERR_CUDA, "cuTensorMapEncodeTiled (activations) failed (%d)", (int)r);
-        }
-        GemmParams gp;
-        memset(&gp, 0, sizeof(gp));
-        gp.fmt = FMT; gp.rows = rows[i]; gp.K = K; gp.M = M;
-        gp.n_block = pl.n_block; gp.stages = pl.stages;
-        gp.scales = scales[i];
-        gp.inv_xscale = inv;
-        gp.out = outs[i];
-        gp.residual = residuals[i];
-        gp.ldo = ldos[i];
-        gp.partial = partial;
-        gp.counters = counters;
-        e = allow_all_dynamic_smem(kern);
-        if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "cudaFuncSetAttribute(%zu): %s", pl.smem, cudaGetErrorString(e));
-        e = launch(kern, dim3(pl.row_tiles, pl.x_blocks, pl.ksplit), dim3(kGThreads), pl.smem, stream, true, gp, map_w, map_x);
-        if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "linear_gemm: %s", cudaGetErrorString(e));
+    TensorMapEncodeFn enc = tensor_map_encoder();
+    if (enc == nullptr) return fail(KMLL_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    PairParams pp;
+    memset(&pp, 0, sizeof(pp));
+    pp.K = K; pp.M = M; pp.nmat = nmat;
+    CUtensorMap map_w[kPMaxMats], map_x;
+    int tiles = 0;
+    for (int i = 0; i < kPMaxMats; ++i) {
+        const int src = i < nmat ? i : 0;  // unused tensor-map slots repeat the first matrix
+        const uint64_t pitch = FMT == FMT_W4 ? (uint64_t)K / 2 : (uint64_t)K;
+        KMLL_TRY_RC(make_map_2d(&map_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w[src], pitch, (uint64_t)rows[src], pitch, FMT == FMT_W4 ? 32 : 64, 128,
+                                CU_TENSOR_MAP_SWIZZLE_NONE));
+        if (i >= nmat) continue;
+        pp.mat[i].scales = scales[i];
+        pp.mat[i].out = outs[i];
+        pp.mat[i].residual = residuals[i];
+        pp.mat[i].rows = rows[i];
+        pp.mat[i].ldo = ldos[i];
+        pp.mat[i].tile_start = tiles;
+        tiles += (rows[i] + 255) / 256;
     }
+    const PairPlan pl = pair_plan(FMT, M, K, tiles, big.n_block);
+    pp.n_block = pl.n_block; pp.x_blocks = pl.x_blocks; pp.ksplit = pl.ksplit; pp.units = pl.units; pp.stages = pl.stages;
+    pp.inv_xscale = inv;
+    pp.partial = partial;
+    pp.counters = counters;
+    {   // both f16 planes of x as one 3-D tensor [2, M, K]; box = [2, n_block / 2, 64 columns], 128-byte swizzle
+        const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, 2};
+        const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)M * K * 2};
+        const cuuint32_t box[3] = {kGKT, (cuuint32_t)pl.n_block / 2, 2};
+        const cuuint32_t estr[3] = {1, 1, 1};
+        const CUresult r = enc(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, x_hi, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(KMLL_ERR_CUDA, "cuTensorMapEncodeTiled (activations) failed (%d)", (int)r);
+    }
+    auto kern = 2 * pl.n_block <= kGMaxN ? linear_gemm_pair_kernel<FMT, true> : linear_gemm_pair_kernel<FMT, false>;
+    e = allow_all_dynamic_smem(kern);
+    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "cudaFuncSetAttribute(%zu): %s", pl.smem, cudaGetErrorString(e));
+    const int clusters = pl.units < kPClusters ? pl.units : kPClusters;
+    e = launch_cluster(kern, dim3(2 * clusters), 2, dim3(kPThreads), pl.smem, stream, true, pp, map_w[0], map_w[1], map_w[2], map_x);
+    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "linear_gemm_pair: %s", cudaGetErrorString(e));
     return KMLL_OK;
 }
 

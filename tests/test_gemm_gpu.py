@@ -129,3 +129,42 @@ def test_gemm_without_workspace_still_works(cuda):
     check(load().kmll_linear_batched_w4g128(torch.cuda.current_stream().cuda_stream, xd.data_ptr(), w.packed.data_ptr(), w.gscales.data_ptr(), m, k,
                                             n, None, out.data_ptr()))
     assert float(np.max(np.abs(host(out) - ref))) <= 1e-4 * np.sqrt(k)
+
+
+# 33 and more rows of x: pairs of blocks, 256 weight rows against up to 256 rows of x.  One row of weights, one k-tile, one group,
+# both sides of the one-MMA form (128 rows of x), ragged last tiles on either side, split K, several units per pair.
+PAIR = [("w4", 33, 1, 128), ("w4", 128, 257, 256), ("w4", 129, 300, 384), ("w4", 256, 256, 384), ("w4", 257, 255, 128), ("w4", 40, 600, 16384),
+        ("w4", 700, 3000, 1152), ("i8", 33, 1, 64), ("i8", 65, 300, 192), ("i8", 300, 257, 320), ("i8", 48, 130, 8192), ("i8", 1100, 5000, 128)]
+
+
+@pytest.mark.parametrize("fmt,m,n,k", PAIR)
+def test_pair_gemm_error_bound(cuda, fmt, m, n, k):
+    """Against 64-bit sums of the dequantized weights.  Bound per output: two binary16 planes of x (2^-22 of every product) and
+    f32 sums in steps of 16 columns (2^-23 of the partial sum each), times sum |w x|."""
+    rng = np.random.default_rng(m * 7 + n + k)
+    x = rng.normal(0, 1, (m, k)).astype(F)
+    x[m // 3] *= F(1e-3)
+    if fmt == "w4":
+        w = w4_weight(rng, n, k)[3]
+    else:
+        w = i8_weight(rng, n, k)[3]
+    w64 = host(w.dequantize()).astype(np.float64).reshape(n, k)
+    x64 = x.astype(np.float64)
+    got = host(ops.linear_batched(dev(x), w, m, k, n, workspace=ops.linear_batched_workspace(m, k))).reshape(m, n)
+    bound = (2.0 ** -22 + (k / 16 + 16) * 2.0 ** -23) * (np.abs(x64) @ np.abs(w64).T) + 1e-30
+    assert np.all(np.abs(got - x64 @ w64.T) <= bound)
+    again = host(ops.linear_batched(dev(x), w, m, k, n, workspace=ops.linear_batched_workspace(m, k))).reshape(m, n)
+    assert np.array_equal(got, again)
+
+
+def test_pair_gemm_three_matrices(cuda):
+    """Matrices of different, ragged heights in one launch, against 64-bit sums, bound as above."""
+    rng = np.random.default_rng(12)
+    m, k = 130, 512
+    mats = [w4_weight(rng, rows, k)[3] for rows in (513, 300, 300)]
+    xd = dev(rng.normal(0, 1, (m, k)).astype(F))
+    for got, w in zip(ops.linear_qkv_batched(xd, *mats, m, k), mats):
+        w64 = host(w.dequantize()).astype(np.float64).reshape(-1, k)
+        x64 = host(xd).astype(np.float64)
+        bound = (2.0 ** -22 + (k / 16 + 16) * 2.0 ** -23) * (np.abs(x64) @ np.abs(w64).T) + 1e-30
+        assert np.all(np.abs(host(got).reshape(m, -1) - x64 @ w64.T) <= bound)
