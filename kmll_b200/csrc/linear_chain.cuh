@@ -642,47 +642,63 @@ __global__ void __launch_bounds__(kSBlock, 1) linear_chain_kernel(const __grid_c
 }
 
 // ---- canonical W4-G128 -> prepared records --------------------------------------------------------------------
-// One thread per 32-bit word of the output.  pair != 0: the A rows of unit u are rows 16u.. of matrix a (gate) and
-// the B rows the same rows of matrix b (up); else A rows = 32u.., B rows = 32u + 16.. of matrix a.
-__global__ void w4_prepare_kernel(const uint8_t* __restrict__ pa, const uint16_t* __restrict__ sa, const uint8_t* __restrict__ pb,
-                                  const uint16_t* __restrict__ sb, int rows, int cols, int pair, size_t total_words,
-                                  uint32_t* __restrict__ out) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total_words) return;
-    constexpr int kWords = kCRecBytes / 4;  // 528
+// pair != 0: the A rows of unit u are rows 16u.. of matrix a (gate) and the B rows the same rows of matrix b (up); else A rows =
+// 32u.., B rows = 32u + 16.. of matrix a.  Bound by HBM: one warp per record; lane (g, t) reads 16 bytes (32 columns) of the four rows
+// g, g + 8 of both halves and writes four 16-byte words, so a warp's stores are 512 contiguous bytes.  14336 x 4096: 49 us (one
+// thread per output word, eight byte loads each) -> 19 us = 3.2 TB/s.  ALIGNED: the packed rows start on 16 bytes.
+template <bool ALIGNED>
+__global__ void __launch_bounds__(256) w4_prepare_kernel(const uint8_t* __restrict__ pa, const uint16_t* __restrict__ sa, const uint8_t* __restrict__ pb,
+                                                         const uint16_t* __restrict__ sb, int rows, int cols, int pair, size_t records,
+                                                         uint8_t* __restrict__ out) {
+    const size_t rec = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (rec >= records) return;
+    const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
     const int ngroups = cols >> 7;
-    const size_t rec = idx / kWords;
-    const int wi = (int)(idx - rec * kWords);
     const int unit = (int)(rec / ngroups), grp = (int)(rec - (size_t)unit * ngroups);
     const int rowA0 = pair ? unit * 16 : unit * 32, rowB0 = pair ? unit * 16 : unit * 32 + 16;
     const uint8_t* pB = pair ? pb : pa;
     const uint16_t* sB = pair ? sb : sa;
     const size_t rowbytes = (size_t)cols >> 1;
-    uint32_t word = 0;
-    if (wi < 512) {
-        const int i = wi >> 7, l = (wi >> 2) & 31, a = wi & 3;
-        const int gq = l >> 2, tq = l & 3;
-        const int rp = gq + 8 * (a & 1), h = a >> 1;
+    uint32_t n[2][2][4];  // [A / B][row g / g + 8][word of 8 columns]; rows past the end: q = 0
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int col = grp * 128 + tq * 32 + i * 8 + h * 4 + e;
-            const int ra = rowA0 + rp, rb = rowB0 + rp;
-            uint32_t na = 8u, nb = 8u;  // rows past the end: q = 0
-            if (ra < rows) { const uint8_t b = pa[(size_t)ra * rowbytes + (col >> 1)]; na = (col & 1) ? (b >> 4) : (b & 15u); }
-            if (rb < rows) { const uint8_t b = pB[(size_t)rb * rowbytes + (col >> 1)]; nb = (col & 1) ? (b >> 4) : (b & 15u); }
-            const uint32_t byte = (((na - 8u) & 15u) << 4) | nb;  // high nibble: two's complement q_A; low nibble: q_B + 8
-            word |= byte << (8 * e);
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int row = (m ? rowB0 : rowA0) + gq + 8 * r;
+            const uint8_t* src = (m ? pB : pa) + (size_t)row * rowbytes + grp * 64 + tq * 16;
+            uint4 v = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);
+            if (row < rows) {
+                if (ALIGNED) {
+                    v = __ldg(reinterpret_cast<const uint4*>(src));
+                } else {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) w[i] = src[4 * i] | (src[4 * i + 1] << 8) | (src[4 * i + 2] << 16) | ((uint32_t)src[4 * i + 3] << 24);
+                    v = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
+            n[m][r][0] = v.x; n[m][r][1] = v.y; n[m][r][2] = v.z; n[m][r][3] = v.w;
         }
-    } else {
-        const int si = wi - 512;  // (g, which): g = si / 2; which = 0: A rows g, g + 8; 1: B rows g, g + 8
-        const int gq = si >> 1;
-        const int r0 = (si & 1) ? rowB0 + gq : rowA0 + gq, r1 = r0 + 8;
-        const uint16_t* s = (si & 1) ? sB : sa;
+    uint8_t* to = out + rec * kCRecBytes;
+    // four columns (16 bits of nibbles) spread over the low nibbles of a word's bytes
+    auto spread = [](uint32_t h) { h = (h | (h << 8)) & 0x00ff00ffu; return (h | (h << 4)) & 0x0f0f0f0fu; };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t o[4];  // word a: row g + 8 (a & 1), columns 32 t + 8 i + 4 (a >> 1) ..; high nibble: two's complement q_A, low nibble: q_B + 8
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const uint32_t na = (n[0][a & 1][i] >> (16 * (a >> 1))) & 0xffffu, nb = (n[1][a & 1][i] >> (16 * (a >> 1))) & 0xffffu;
+            o[a] = (spread(na ^ 0x8888u) << 4) | spread(nb);
+        }
+        reinterpret_cast<uint4*>(to)[i * 32 + lane] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    if (lane < 16) {  // (g, which): g = lane / 2; which = 0: A rows g, g + 8; 1: B rows g, g + 8
+        const int r0 = ((lane & 1) ? rowB0 : rowA0) + (lane >> 1), r1 = r0 + 8;
+        const uint16_t* s = (lane & 1) ? sB : sa;
         const uint32_t lo = r0 < rows ? s[(size_t)r0 * ngroups + grp] : 0u;
         const uint32_t hi = r1 < rows ? s[(size_t)r1 * ngroups + grp] : 0u;
-        word = lo | (hi << 16);
+        reinterpret_cast<uint32_t*>(to)[512 + lane] = lo | (hi << 16);
     }
-    out[idx] = word;
 }
 
 }  // namespace kmll

@@ -83,6 +83,42 @@ def test_quantize_w4_bit_exact(cuda, rows, cols, golden):
         assert np.array_equal(host(m.packed), golden["w4_packed"])
 
 
+@pytest.mark.parametrize("rows,cols", [(3, 8), (5, 40), (2, 4100), (2, 16384), (2, 16520)])
+def test_quantize_rs_i8_ties_and_limits(cuda, rows, cols):
+    """Rows of 16-byte pieces (held in registers, or longer), of quads only; quotients on and next to ties, tiny and huge scales,
+    unaligned rows."""
+    rng = np.random.default_rng(cols)
+    w = (rng.integers(-254, 255, (rows, cols)) * F(0.5)).astype(F)  # scale 1: halves are ties
+    w[:, 0] = F(127.0)
+    w[1] *= F(2.0 ** -133)
+    if rows > 2:
+        w[2] = rng.normal(0, 1, cols).astype(F) * F(1e37)
+    wb = oracle.bf16_from_f32(w)
+    q, sc = oracle.rs_i8_quantize(wb)
+    room = torch.empty(rows * cols + 1, dtype=torch.bfloat16, device="cuda")
+    for shift in (0, 1):
+        view = room[shift:shift + rows * cols].view(rows, cols)
+        view.copy_(torch.from_numpy(wb.view(np.int16)).view(torch.bfloat16).view(rows, cols).cuda())
+        m = ops.DeviceRowwiseScaledI8Matrix.from_bf16_rows_symmetric(view)
+        assert np.array_equal(host(m.values), q)
+        assert np.array_equal(host(m.scales).view(np.uint32), sc.view(np.uint32))
+        assert np.array_equal(host(m.dequantize()).view(np.uint32), oracle.rs_i8_dequant(q, sc).view(np.uint32))
+
+
+def test_quantize_w4_ties_and_limits(cuda):
+    """33 groups (one past a block); ties, group maxima that round the f16 scale down, to a subnormal, to zero."""
+    rng = np.random.default_rng(3)
+    w = (rng.integers(-14, 15, (33, 128)) * F(0.5)).astype(F)
+    w[:, 5] = F(7.0)
+    w *= np.exp2(np.linspace(-30, 12, 33)).astype(F)[:, None]
+    w[7:20] *= F(1.0007)
+    m = ops.DeviceW4G128Matrix.from_f32_rows(dev(w))
+    packed, gs = oracle.w4_quantize(w)
+    assert np.array_equal(host(m.packed), packed)
+    assert np.array_equal(host(m.gscales.view(torch.int16)).view(np.uint16), gs)
+    assert np.array_equal(host(m.dequantize()).view(np.uint32), oracle.w4_dequant(packed, gs).view(np.uint32))
+
+
 def test_w4_requires_group_multiple(cuda):
     with pytest.raises(KmllError):
         ops.DeviceW4G128Matrix.from_f32_rows(torch.zeros((4, 100), device="cuda"))
