@@ -91,6 +91,8 @@ struct Decoder {
     bool chain_words = false;      // one GPU, one launch per projection: still hand the vectors over as exchange words (KMLL_CHAIN=words)
     bool prepared_valid = false;   // the prepared buffers match the canonical tensors
     unsigned int* top1_counter = nullptr;
+    void* prompt_scratch = nullptr;  // scratch of the batched prompt path, as large as the longest prompt so far needed
+    size_t prompt_scratch_bytes = 0;
     Layered* lay = nullptr;  // a decoder over a list of layer descriptions (layered.cu); null = kmll's uniform layers
 };
 

@@ -861,6 +861,35 @@ static int setup_exchange(Decoder* d) {
     return KMLL_OK;
 }
 
+// Scratch of a prompt, kept by the decoder: its calls are one after another, and each ends in a stream synchronisation.  Allocating
+// and freeing 14 buffers per call (with the synchronisations inside) took 10 ms of the 13.9 ms of a 200-token prompt of an 8-layer
+// 4096 / 14336 wide decoder (45 ms in some runs); now 2.6 ms in all.
+// Above 2 GiB (more than ~5500 positions at that width, whose prompt takes 20 ms and more) it is allocated for the call and given back.
+static int prefill_scratch(Decoder* d, size_t bytes, unsigned char** out, bool* kept) {
+    constexpr size_t kKeep = (size_t)2 << 30;
+    *kept = bytes <= kKeep;
+    if (*kept && bytes <= d->prompt_scratch_bytes) {
+        *out = static_cast<unsigned char*>(d->prompt_scratch);
+        return KMLL_OK;
+    }
+    if (d->prompt_scratch != nullptr) {
+        cudaFree(d->prompt_scratch);
+        d->resident_bytes -= d->prompt_scratch_bytes;
+        d->prompt_scratch = nullptr;
+        d->prompt_scratch_bytes = 0;
+    }
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "prefill scratch: %s", cudaGetErrorString(e));
+    if (*kept) {
+        d->prompt_scratch = p;
+        d->prompt_scratch_bytes = bytes;
+        d->resident_bytes += bytes;
+    }
+    *out = static_cast<unsigned char*>(p);
+    return KMLL_OK;
+}
+
 extern "C" {
 
 size_t kmll_decoder_config_bytes(void) { return sizeof(kmll_decoder_config); }
@@ -973,6 +1002,7 @@ int kmll_decoder_destroy(kmll_decoder_t dec) {
         if (d->xc_peer_base[r]) cudaIpcCloseMemHandle(d->xc_peer_base[r]);
     if (d->xc_local) cudaFree(d->xc_local);
     for (void* p : d->allocs) cudaFree(p);
+    cudaFree(d->prompt_scratch);
     if (d->pinned) cudaFreeHost(d->pinned);
     layered_destroy(d);
     delete d;
@@ -1181,53 +1211,47 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
     const int q_len = d->n_heads_l * c.head_dim, kv_len = d->n_kv_l * c.head_dim;
     d->host_position = 0;
     d->have_next = false;
-    // batched scratch (prefill_batched_i8_hidden, crates/inference/src/model.rs:5849-5943)
-    std::vector<void*> tmp;
-    auto talloc = [&](float** p, size_t count) -> int {
-        void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, count * sizeof(float));
-        if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "prefill scratch: %s", cudaGetErrorString(e));
-        tmp.push_back(q);
-        *p = (float*)q;
-        return KMLL_OK;
-    };
-    float *xb = nullptr, *x2b = nullptr, *nb = nullptr, *ob = nullptr, *qb = nullptr, *kb = nullptr, *vb = nullptr, *qrb = nullptr,
-          *ab = nullptr, *gb = nullptr, *ub = nullptr, *actb = nullptr;
-    uint32_t* dtok = nullptr;
+    // batched scratch (prefill_batched_i8_hidden, crates/inference/src/model.rs:5849-5943): one buffer, cut into 256-byte aligned parts
+    const int widest = d->hidden_l > c.dim ? (d->hidden_l > q_len ? d->hidden_l : q_len) : (c.dim > q_len ? c.dim : q_len);
+    const size_t ws_bytes = kmll_linear_batched_workspace_bytes(n, widest);
+    // One GPU, every projection on the batched tensor-core path: norms, residuals and SiLU * up ride on the projections (the same
+    // f32 operations per element).  Other shapes, tensor parallelism and kmll's operator order run one operator at a time.
+    const int kmult = c.format == KMLL_FORMAT_W4G128 ? 128 : 64;
+    const bool forms = c.tp_size == 1 && c.fused && ws_bytes > 0 && c.dim % kmult == 0 && q_len % kmult == 0 && d->hidden_l % kmult == 0;
+    size_t scratch_bytes = 0;
+    auto part = [&](size_t bytes) { const size_t at = scratch_bytes; scratch_bytes += (bytes + 255) & ~(size_t)255; return at; };
+    const size_t row = (size_t)n * sizeof(float);
+    const size_t o_x = part(row * c.dim), o_x2 = part(row * c.dim), o_q = part(row * q_len), o_qr = part(row * q_len), o_a = part(row * q_len);
+    const size_t o_k = part(row * kv_len), o_v = part(row * kv_len), o_g = part(row * d->hidden_l), o_u = part(row * d->hidden_l), o_act = part(row * d->hidden_l);
+    const size_t o_tok = part(row), o_ws = part(ws_bytes), o_n = part(forms ? 0 : row * c.dim), o_o = part(forms ? 0 : row * c.dim);
+    unsigned char* base = nullptr;
+    bool kept = false;
+    KMLL_TRY(prefill_scratch(d, scratch_bytes, &base, &kept));
+    auto at = [&](size_t o) { return reinterpret_cast<float*>(base + o); };
+    float *xb = at(o_x), *x2b = at(o_x2), *nb = at(o_n), *ob = at(o_o), *qb = at(o_q), *qrb = at(o_qr), *ab = at(o_a), *kb = at(o_k), *vb = at(o_v),
+          *gb = at(o_g), *ub = at(o_u), *actb = at(o_act);
+    uint32_t* dtok = reinterpret_cast<uint32_t*>(base + o_tok);
+    void* ws = ws_bytes > 0 ? base + o_ws : nullptr;
     auto body = [&]() -> int {
-        KMLL_TRY(talloc(&xb, (size_t)n * c.dim));
-        KMLL_TRY(talloc(&x2b, (size_t)n * c.dim));
-        KMLL_TRY(talloc(&nb, (size_t)n * c.dim));
-        KMLL_TRY(talloc(&ob, (size_t)n * c.dim));
-        KMLL_TRY(talloc(&qb, (size_t)n * q_len));
-        KMLL_TRY(talloc(&qrb, (size_t)n * q_len));
-        KMLL_TRY(talloc(&ab, (size_t)n * q_len));
-        KMLL_TRY(talloc(&kb, (size_t)n * kv_len));
-        KMLL_TRY(talloc(&vb, (size_t)n * kv_len));
-        KMLL_TRY(talloc(&gb, (size_t)n * d->hidden_l));
-        KMLL_TRY(talloc(&ub, (size_t)n * d->hidden_l));
-        KMLL_TRY(talloc(&actb, (size_t)n * d->hidden_l));
-        float* tokf = nullptr;
-        KMLL_TRY(talloc(&tokf, (size_t)n));
-        dtok = (uint32_t*)tokf;
-        // scratch of the batched linears (f16 planes of the activations), sized for the widest input
-        float* wsf = nullptr;
-        const int widest = d->hidden_l > c.dim ? (d->hidden_l > q_len ? d->hidden_l : q_len) : (c.dim > q_len ? c.dim : q_len);
-        const size_t ws_bytes = kmll_linear_batched_workspace_bytes(n, widest);
-        if (ws_bytes > 0) KMLL_TRY(talloc(&wsf, ws_bytes / sizeof(float) + 64));
-        void* ws = wsf;
         KMLL_CUDA(cudaMemcpyAsync(dtok, tokens, (size_t)n * 4, cudaMemcpyHostToDevice, s));
         KMLL_TRY(kmll_embedding_tokens(s, d->embedding, c.vocab_size, c.dim, dtok, n, xb));
         const bool w4 = c.format == KMLL_FORMAT_W4G128;
         for (int l = 0; l < c.n_layers; ++l) {
             Layer& L = d->layers[l];
             // run_prefill_rowwise_scaled_layer_device_with_cache, crates/inference/src/model.rs:9803-10017
-            KMLL_TRY(kmll_rmsnorm_batched(s, xb, L.attention_norm, n, c.dim, c.norm_eps, nb));
-            if (w4) {
+            if (forms) {
+                const void* w[3] = {L.wq.w, L.wk.w, L.wv.w};
+                const void* sc[3] = {L.wq.scales, L.wk.scales, L.wv.scales};
+                const int rows[3] = {q_len, kv_len, kv_len};
+                float* outs[3] = {qb, kb, vb};
+                KMLL_TRY(linear_batched_form(0, s, c.format, xb, n, L.attention_norm, c.norm_eps, w, sc, rows, c.dim, outs, nullptr, ws));
+            } else if (w4) {
+                KMLL_TRY(kmll_rmsnorm_batched(s, xb, L.attention_norm, n, c.dim, c.norm_eps, nb));
                 KMLL_TRY(kmll_linear_qkv_batched_w4g128(s, nb, (const uint8_t*)L.wq.w, (const uint16_t*)L.wq.scales, (const uint8_t*)L.wk.w,
                                                         (const uint16_t*)L.wk.scales, (const uint8_t*)L.wv.w, (const uint16_t*)L.wv.scales, n,
                                                         c.dim, q_len, kv_len, ws, qb, kb, vb));
             } else {
+                KMLL_TRY(kmll_rmsnorm_batched(s, xb, L.attention_norm, n, c.dim, c.norm_eps, nb));
                 KMLL_TRY(kmll_linear_qkv_batched_i8(s, nb, (const int8_t*)L.wq.w, (const float*)L.wq.scales, (const int8_t*)L.wk.w,
                                                     (const float*)L.wk.scales, (const int8_t*)L.wv.w, (const float*)L.wv.scales, n, c.dim,
                                                     q_len, kv_len, ws, qb, kb, vb));
@@ -1237,6 +1261,23 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
                                             L.value_cache, c.kv_bf16));
             KMLL_TRY(prefill_attention_launch(s, qrb, L.key_cache, L.value_cache, n, d->n_heads_l, d->n_kv_l, c.head_dim, ab, c.kv_bf16,
                                               c.sliding_window, c.fused ? 1 : 0));  // fused = 0: kmll's f32 operator arithmetic throughout
+            if (forms) {
+                auto residual = [&](const float* x, const QWeight& m, int cols, const float* r, float* out) -> int {
+                    const void* w[1] = {m.w};
+                    const void* sc[1] = {m.scales};
+                    const int rows[1] = {c.dim};
+                    float* outs[1] = {out};
+                    return linear_batched_form(2, s, c.format, x, n, nullptr, 0.f, w, sc, rows, cols, outs, r, ws);
+                };
+                KMLL_TRY(residual(ab, L.wo, q_len, xb, x2b));
+                const void* w[2] = {L.w1.w, L.w3.w};
+                const void* sc[2] = {L.w1.scales, L.w3.scales};
+                const int rows[1] = {d->hidden_l};
+                float* outs[1] = {actb};
+                KMLL_TRY(linear_batched_form(1, s, c.format, x2b, n, L.ffn_norm, c.norm_eps, w, sc, rows, c.dim, outs, nullptr, ws, gb, ub));
+                KMLL_TRY(residual(actb, L.w2, d->hidden_l, x2b, xb));
+                continue;
+            }
             KMLL_TRY(op_linear_batched(d, s, ab, L.wo, n, ws, ob));
             KMLL_TRY(tp_allreduce(d, s, ob, (size_t)n * c.dim));
             KMLL_TRY(kmll_add_prefix(s, xb, ob, (size_t)n * c.dim, x2b));
@@ -1259,7 +1300,7 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
     };
     const int rc = body();
     cudaStreamSynchronize(s);
-    for (void* p : tmp) cudaFree(p);
+    if (!kept) cudaFree(base);
     if (rc != KMLL_OK) return rc;
     d->host_position = n;
     d->have_next = true;
