@@ -583,3 +583,26 @@ def test_one_thread_two_devices(cuda):
             assert float(np.max(np.abs(got - refb))) <= 1e-4 * np.sqrt(4096)
     finally:
         torch.cuda.set_device(0)
+
+
+# one to eight rows per thread (by the number of blocks), both head sizes, edges of the 16 / 32 / 64-row and 64-key tiles, pointers
+# that are not 16-byte aligned
+@pytest.mark.parametrize("n,h,g,d,shift", [(1, 2, 1, 128, 0), (17, 8, 2, 64, 0), (63, 4, 4, 128, 1), (65, 14, 2, 64, 0), (129, 32, 8, 128, 0), (160, 32, 4, 64, 3),
+                                           (320, 64, 8, 128, 0), (577, 32, 8, 64, 1), (1025, 32, 32, 128, 0)])
+def test_prefill_attention_against_64_bits(cuda, n, h, g, d, shift):
+    """Bound: scores carry 2^-24 of sum |q k| per step, weights twice that relative error, sums over keys 2^-23 per step."""
+    gen = torch.Generator(device="cuda").manual_seed(n + h)
+
+    def rows(width):
+        return torch.randn(n * width + shift, generator=gen, device="cuda")[shift:]
+
+    q, k, v = rows(h * d), rows(g * d), rows(g * d)
+    got = ops.prefill_causal_attention(q, k, v, n, n, h, g, d).view(n, h, d).double()
+    q64, k64, v64 = (t.view(n, -1, d).double().transpose(0, 1) for t in (q, k, v))
+    hidden = torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1)
+    for head in range(0, h, max(1, h // 4)):
+        kh, vh = k64[head // (h // g)], v64[head // (h // g)]
+        w = torch.softmax((q64[head] @ kh.T * d ** -0.5).masked_fill(hidden, float("-inf")), -1)
+        step = float((q64[head].abs() @ kh.abs().T).max()) * d ** -0.5
+        bound = (2 * (d + 8) * 2.0 ** -24 * step + (n + 64) * 2.0 ** -23) * float(vh.abs().max())
+        assert float((got[:, head] - w @ vh).abs().max()) <= bound
