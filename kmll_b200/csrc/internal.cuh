@@ -193,7 +193,8 @@ int linear_top1_offset(cudaStream_t stream, int fmt, const float* x, const uint1
                        float* partial_logits, uint64_t* packed_out, const TpExchange* xc = nullptr);
 // Batched fused linear forms for rows of x that are independent sequences (batch <= 16 per pass):
 // form 0 = RMSNorm + QKV (3 matrices, rows[0..2]), 1 = RMSNorm + gate/up + SiLU*up (2 matrices of rows[0]),
-// 2 = projection + residual, 3 = (RMSNorm +) projection.  Outputs are [batch, rows] row-major.
+// 2 = projection + residual, 3 = (RMSNorm +) projection, 4 = RMSNorm + gate/up into gate_tmp and up_tmp, 5 = SiLU(gate_tmp) *
+// up_tmp + projection + residual (overwrites gate_tmp).  Outputs are [batch, rows] row-major.
 // `workspace` (linear_batched_workspace_bytes(batch, cols) bytes) enables the tensor-core path for 5 or more rows; form 1
 // then also needs two [batch, rows] scratch matrices for the gate and up projections.
 int linear_batched_form(int form, cudaStream_t stream, int fmt, const float* x, int batch, const uint16_t* norm_w, float eps,

@@ -1123,9 +1123,10 @@ static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, int M, i
     return KMLL_OK;
 }
 
-// y[m, :] (+= residual) = dequant(W_i) x[m, :] for every matrix i; x is split into f16 planes once for all of them
+// y[m, :] (+= residual) = dequant(W_i) x[m, :] for every matrix i; x is split into f16 planes once for all of them.  With `up` (more
+// than 32 rows only) the input is SiLU(x) * up.
 template <int FMT>
-static int run_gemm(cudaStream_t stream, const float* x, int M, int K, int ldx, const uint16_t* norm_w, float eps, const void* const* w,
+static int run_gemm(cudaStream_t stream, const float* x, const float* up, int M, int K, int ldx, const uint16_t* norm_w, float eps, const void* const* w,
                     const void* const* scales, const int* rows, float* const* outs, const float* const* residuals, const int* ldos, int nmat,
                     void* workspace) {
     int max_rows = 0;
@@ -1143,7 +1144,7 @@ static int run_gemm(cudaStream_t stream, const float* x, int M, int K, int ldx, 
     float* partial = reinterpret_cast<float*>(ws + big.off_partial);
     unsigned int* counters = reinterpret_cast<unsigned int*>(ws + big.off_counters);
     const int n_counters = 16384;
-    cudaError_t e = launch(split_rows_kernel, dim3(M), dim3(512), 0, stream, true, x, ldx, K, norm_w, eps, x_hi, x_lo, inv, counters, n_counters,
+    cudaError_t e = launch(K <= 4096 ? split_rows_kernel<1> : K <= 8192 ? split_rows_kernel<2> : split_rows_kernel<4>, dim3(M), dim3(512), 0, stream, true, x, up, ldx, K, norm_w, eps, x_hi, x_lo, inv, counters, n_counters,
                            FMT == FMT_W4 ? 1 : 0);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "split_rows: %s", cudaGetErrorString(e));
     TensorMapEncodeFn enc = tensor_map_encoder();
@@ -1288,7 +1289,7 @@ static int run_linear(const char* name, cudaStream_t stream, const float* x, int
                 res_[i] = EPI == EPI_RESIDUAL ? mats[i].residual : nullptr;
                 ldos_[i] = ldo_override > 0 ? ldo_override : mats[i].rows;
             }
-            return run_gemm<FMT>(stream, x, M, K, ldx, norm_w, eps, w_, s_, rows_, outs_, res_, ldos_, nmat, workspace);
+            return run_gemm<FMT>(stream, x, nullptr, M, K, ldx, norm_w, eps, w_, s_, rows_, outs_, res_, ldos_, nmat, workspace);
         }
     }
     // Batches above one row: the streaming kernel takes up to 4 rows of x per pass when its shared-memory plan fits
@@ -1421,6 +1422,22 @@ static int batched_forms(int form, cudaStream_t stream, const float* x, int batc
             }
             MatArg m[2] = {{w[0], scales[0], rows[0], outs[0], nullptr}, {w[1], scales[1], rows[0], nullptr, nullptr}};
             return run_linear<FMT, EPI_SILU>("silu_gate_up_batched_norm", stream, x, batch, cols, cols, norm_w, eps, m, 2, 0, nullptr, nullptr);
+        }
+        case 4: {  // RMSNorm + gate / up, for form 5
+            MatArg m[2] = {{w[0], scales[0], rows[0], gate_tmp, nullptr}, {w[1], scales[1], rows[0], up_tmp, nullptr}};
+            return run_linear<FMT, EPI_STORE>("gate_up_batched_norm", stream, x, batch, cols, cols, norm_w, eps, m, 2, 0, nullptr, nullptr, nullptr, 0, 0,
+                                              workspace);
+        }
+        case 5: {  // SiLU(gate) * up + projection + residual: the activation is formed where the tensor-core path splits its input
+            GemmPlan pl;
+            if (batch > 32 && workspace != nullptr && gemm_enabled() && (cols & 3) == 0 && aligned16(gate_tmp) && aligned16(up_tmp) && aligned16(workspace) &&
+                aligned16(w[0]) && gemm_plan(FMT, batch, cols, rows[0], &pl)) {
+                const int ldo = rows[0];
+                return run_gemm<FMT>(stream, gate_tmp, up_tmp, batch, cols, cols, nullptr, 0.f, w, scales, rows, outs, &residual, &ldo, 1, workspace);
+            }
+            const int rc = kmll_silu_mul_prefix(stream, gate_tmp, up_tmp, (size_t)batch * cols, gate_tmp);
+            if (rc != KMLL_OK) return rc;
+            return batched_forms<FMT>(2, stream, gate_tmp, batch, nullptr, 0.f, w, scales, rows, cols, outs, residual, workspace, nullptr, nullptr);
         }
         case 2: {  // projection + residual
             MatArg m = {w[0], scales[0], rows[0], outs[0], residual};

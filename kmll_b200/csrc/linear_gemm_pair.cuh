@@ -421,15 +421,24 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
 #pragma unroll 1
                     for (int c = 0; c < n_half; c += 32) {
                         const int n_ok = n_half - c;
+                        // four splits' loads in flight (a round of loads costs ~1 us whatever it carries)
+                        auto part_of = [&](int z, int j) {
+                            return (z < p.ksplit && j < n_ok) ? __ldcg(base + ((size_t)z * p.n_block + c_first + c + j) * 128 + rl) : 0.0f;
+                        };
                         uint32_t d[32];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) d[j] = 0u;
+                        for (int j = 0; j < 32; ++j) d[j] = __float_as_uint(part_of(0, j));
 #pragma unroll 1
-                        for (int z = 0; z < p.ksplit; ++z) {
-                            const float* from = base + ((size_t)z * p.n_block + c_first + c) * 128 + rl;
+                        for (int z0 = 1; z0 < p.ksplit; z0 += 3) {
+                            float t[3][32];
 #pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (j < n_ok) d[j] = __float_as_uint(__uint_as_float(d[j]) + __ldcg(from + j * 128));
+                            for (int z = 0; z < 3; ++z)
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) t[z][j] = part_of(z0 + z, j);
+#pragma unroll
+                            for (int z = 0; z < 3; ++z)
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) d[j] = __float_as_uint(__uint_as_float(d[j]) + t[z][j]);
                         }
                         store_columns(mat, row, row_ok, u.m0 + c_first + c, min(n_ok, p.M - (u.m0 + c_first + c)), p.inv_xscale, rscale, lane, d);
                     }

@@ -1222,7 +1222,7 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
     auto part = [&](size_t bytes) { const size_t at = scratch_bytes; scratch_bytes += (bytes + 255) & ~(size_t)255; return at; };
     const size_t row = (size_t)n * sizeof(float);
     const size_t o_x = part(row * c.dim), o_x2 = part(row * c.dim), o_q = part(row * q_len), o_qr = part(row * q_len), o_a = part(row * q_len);
-    const size_t o_k = part(row * kv_len), o_v = part(row * kv_len), o_g = part(row * d->hidden_l), o_u = part(row * d->hidden_l), o_act = part(row * d->hidden_l);
+    const size_t o_k = part(row * kv_len), o_v = part(row * kv_len), o_g = part(row * d->hidden_l), o_u = part(row * d->hidden_l), o_act = part(forms ? 0 : row * d->hidden_l);
     const size_t o_tok = part(row), o_ws = part(ws_bytes), o_n = part(forms ? 0 : row * c.dim), o_o = part(forms ? 0 : row * c.dim);
     unsigned char* base = nullptr;
     bool kept = false;
@@ -1262,20 +1262,22 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
             KMLL_TRY(prefill_attention_launch(s, qrb, L.key_cache, L.value_cache, n, d->n_heads_l, d->n_kv_l, c.head_dim, ab, c.kv_bf16,
                                               c.sliding_window, c.fused ? 1 : 0));  // fused = 0: kmll's f32 operator arithmetic throughout
             if (forms) {
-                auto residual = [&](const float* x, const QWeight& m, int cols, const float* r, float* out) -> int {
-                    const void* w[1] = {m.w};
-                    const void* sc[1] = {m.scales};
+                {
+                    const void* w[1] = {L.wo.w};
+                    const void* sc[1] = {L.wo.scales};
                     const int rows[1] = {c.dim};
-                    float* outs[1] = {out};
-                    return linear_batched_form(2, s, c.format, x, n, nullptr, 0.f, w, sc, rows, cols, outs, r, ws);
-                };
-                KMLL_TRY(residual(ab, L.wo, q_len, xb, x2b));
+                    float* outs[1] = {x2b};
+                    KMLL_TRY(linear_batched_form(2, s, c.format, ab, n, nullptr, 0.f, w, sc, rows, q_len, outs, xb, ws));
+                }
                 const void* w[2] = {L.w1.w, L.w3.w};
                 const void* sc[2] = {L.w1.scales, L.w3.scales};
                 const int rows[1] = {d->hidden_l};
-                float* outs[1] = {actb};
-                KMLL_TRY(linear_batched_form(1, s, c.format, x2b, n, L.ffn_norm, c.norm_eps, w, sc, rows, c.dim, outs, nullptr, ws, gb, ub));
-                KMLL_TRY(residual(actb, L.w2, d->hidden_l, x2b, xb));
+                KMLL_TRY(linear_batched_form(4, s, c.format, x2b, n, L.ffn_norm, c.norm_eps, w, sc, rows, c.dim, nullptr, nullptr, ws, gb, ub));
+                const void* w2[1] = {L.w2.w};
+                const void* sc2[1] = {L.w2.scales};
+                const int rows2[1] = {c.dim};
+                float* outs[1] = {xb};
+                KMLL_TRY(linear_batched_form(5, s, c.format, nullptr, n, nullptr, 0.f, w2, sc2, rows2, d->hidden_l, outs, x2b, ws, gb, ub));
                 continue;
             }
             KMLL_TRY(op_linear_batched(d, s, ab, L.wo, n, ws, ob));
