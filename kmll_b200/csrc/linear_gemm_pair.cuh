@@ -27,7 +27,7 @@
 //   warp 2      TMA of the raw weight tile (ahead of the grid dependency: weights are constants)
 //   warps 4-7   expand raw weights to swizzled binary16 rows of the MMA operand
 //   warps 8-15  drain accumulators, epilogue
-// setmaxnreg moves registers to the drain warps (48 + 48 + 2 x 208 = 4 x 128 per thread of a warpgroup).
+// setmaxnreg moves registers to the drain warps (40 + 40 + 2 x 216 = 4 x 128 per thread of a warpgroup).
 // Barriers: `full` (own block's copies of a stage landed), `a_ready` (in the leader: both blocks' operands of a stage are
 // written), `empty` (in each block, multicast commit), `acc_full` (in each block, multicast commit), `acc_empty` (in the leader).
 // Every wait is bounded; on a time-out the role raises the device status word and walks to the cluster barrier at the end.
@@ -94,32 +94,40 @@ __device__ inline void fma_pair(unsigned long long& acc, unsigned long long s2, 
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(s2), "l"(d));
 }
 
-// 32 columns (rows of x m .. m + n_ok - 1) of one weight row: y = d 2^-sh scale (+ residual).  A lane holds the 2^-sh of one
-// column; loads are issued together (one at a time the epilogue of a 256 x 256 unit took 32000 cycles, this way 12000).
-__device__ inline void store_columns(const PairMat& mat, int row, bool row_ok, int m, int n_ok, const float* inv_xscale, float rscale, int lane,
-                                     const uint32_t (&d)[32]) {
-    const float iv = lane < n_ok ? __ldg(inv_xscale + m + lane) : 0.0f;
+// The 2^-sh of up to 128 rows of x, one per lane and register.  Loaded at the start of a unit: a load waits behind the tile copies in
+// flight (~3000 cycles), and one in front of every 16 columns made the epilogue 23000 cycles long.
+struct PairScales {
+    float v[4];
+    __device__ PairScales(const float* inv_xscale, int m, int n, int lane) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = c * 32 + lane < n ? __ldg(inv_xscale + m + c * 32 + lane) : 0.0f;
+    }
+    __device__ float chunk(int c) const { return c < 32 ? v[0] : c < 64 ? v[1] : c < 96 ? v[2] : v[3]; }
+};
+// 16 columns (rows of x m .. m + n_ok - 1) of one weight row: y = d 2^-sh scale (+ residual); `iv`: the 2^-sh of 32 columns, these from
+// lane `iv0`; the loads of the residual are issued together
+__device__ inline void store_columns(const PairMat& mat, int row, bool row_ok, int m, int n_ok, float iv, int iv0, float rscale, const uint32_t (&d)[16]) {
     const size_t o = (size_t)m * mat.ldo + row;
     const int ldo = mat.ldo;
-    const bool add = mat.residual != nullptr;
-    const float* res = mat.residual + o;
     float* out = mat.out + o;
-#pragma unroll
-    for (int h = 0; h < 32; h += 16) {
+    if (mat.residual != nullptr) {
+        const float* res = mat.residual + o;
         float r[16];
-        if (add) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j, res += ldo) r[j] = (row_ok && h + j < n_ok) ? *res : 0.0f;
-        }
+        for (int j = 0; j < 16; ++j, res += ldo) r[j] = (row_ok && j < n_ok) ? *res : 0.0f;
 #pragma unroll
         for (int j = 0; j < 16; ++j, out += ldo) {
-            float v = __uint_as_float(d[h + j]) * __shfl_sync(0xffffffffu, iv, h + j) * rscale;
-            if (add) v = r[j] + v;
-            if (row_ok && h + j < n_ok) *out = v;
+            const float v = r[j] + __uint_as_float(d[j]) * __shfl_sync(0xffffffffu, iv, iv0 + j) * rscale;
+            if (row_ok && j < n_ok) *out = v;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j, out += ldo) {
+            const float v = __uint_as_float(d[j]) * __shfl_sync(0xffffffffu, iv, iv0 + j) * rscale;
+            if (row_ok && j < n_ok) *out = v;
         }
     }
 }
-
 // Position in the ring of stages: counted, not divided (a division by a run-time number per k-tile costs the issuing thread ~600 cycles).
 struct PairRing {
     int stage = 0, stages;
@@ -201,7 +209,7 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
     bool ok = true;
 
     if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (warp != 2) pdl_wait();  // the planes of x come from the previous kernel
         if (warp == 0 || warp == 2) {
             if (lane == 0) {
@@ -270,7 +278,7 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
         }
     } else if (warp < 8) {
         // ---- weight expansion: thread pair (row, half) turns 32 columns of two raw rows into binary16 in the swizzled tile
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         pdl_wait();
         const int et = tid - 128, h = et & 1;
         PairRing ring(stages);
@@ -331,7 +339,7 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
         }
     } else {
         // ---- drain and epilogue: warp w reads tensor-memory lanes 32 (w % 4) .., warps 8-11 the first half of the columns
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         pdl_wait();
         const int q = warp & 3, half = (warp - 8) >> 2, rl = q * 32 + lane;
         const int c_first = half * n_half;
@@ -360,6 +368,8 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
             } else {
                 buffer = 0u;
             }
+            const PairScales scales(p.inv_xscale, u.m0 + c_first, min(n_half, p.M - (u.m0 + c_first)), lane);
+            const float rscale = W4 ? 1.0f : reinterpret_cast<const float*>(mat.scales)[srow];
             unsigned long long acc[16 * kChunks];  // pairs of f32 sums
 #pragma unroll
             for (int j = 0; j < 16 * kChunks; ++j) acc[j] = 0ull;
@@ -387,24 +397,22 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
                 if (lane == 0) mbar_arrive_leader(&acc_empty[buffer]);
             }
             if (!ok) break;
-            const float rscale = W4 ? 1.0f : reinterpret_cast<const float*>(mat.scales)[srow];
             const bool split = p.ksplit > 1, row_ok = row < mat.rows;
             float* part = p.partial + ((size_t)u.slot * p.ksplit + u.z) * (size_t)p.n_block * 128;
 #pragma unroll
-            for (int c = 0; c < kChunks; ++c) {
-                if (c * 32 < n_half) {
-                    uint32_t d[32];
+            for (int c = 0; c < 32 * kChunks; c += 16) {
+                const int n_ok = n_half - c;
+                if (n_ok <= 0) break;
+                uint32_t d[16];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) d[j] = (uint32_t)(acc[c * 16 + j / 2] >> (32 * (j & 1)));
-                    if (split) {
-                        const int n_ok = n_half - c * 32;
-                        float* to = part + (size_t)(c_first + c * 32) * 128 + rl;
+                for (int j = 0; j < 16; ++j) d[j] = (uint32_t)(acc[(c + j) / 2] >> (32 * (j & 1)));
+                if (split) {
+                    float* to = part + (size_t)(c_first + c) * 128 + rl;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (j < n_ok) to[j * 128] = __uint_as_float(d[j]);  // scales and residual are applied after the merge
-                    } else {
-                        store_columns(mat, row, row_ok, u.m0 + c_first + c * 32, min(n_half - c * 32, p.M - (u.m0 + c_first + c * 32)), p.inv_xscale, rscale, lane, d);
-                    }
+                    for (int j = 0; j < 16; ++j)
+                        if (j < n_ok) to[j * 128] = __uint_as_float(d[j]);  // scales and residual are applied after the merge
+                } else {
+                    store_columns(mat, row, row_ok, u.m0 + c_first + c, min(n_ok, p.M - (u.m0 + c_first + c)), scales.chunk(c), c & 31, rscale, d);
                 }
             }
             if (split) {
@@ -419,28 +427,25 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
                     __threadfence();
                     const float* base = p.partial + (size_t)u.slot * p.ksplit * (size_t)p.n_block * 128;
 #pragma unroll 1
-                    for (int c = 0; c < n_half; c += 32) {
+                    for (int c = 0; c < n_half; c += 16) {  // four splits' loads in flight (a round of loads costs ~1 us whatever it carries)
                         const int n_ok = n_half - c;
-                        // four splits' loads in flight (a round of loads costs ~1 us whatever it carries)
-                        auto part_of = [&](int z, int j) {
-                            return (z < p.ksplit && j < n_ok) ? __ldcg(base + ((size_t)z * p.n_block + c_first + c + j) * 128 + rl) : 0.0f;
-                        };
-                        uint32_t d[32];
+                        const float* from = base + (size_t)(c_first + c) * 128 + rl;
+                        uint32_t d[16];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) d[j] = __float_as_uint(part_of(0, j));
+                        for (int j = 0; j < 16; ++j) d[j] = 0u;
 #pragma unroll 1
-                        for (int z0 = 1; z0 < p.ksplit; z0 += 3) {
-                            float t[3][32];
+                        for (int z0 = 0; z0 < p.ksplit; z0 += 4) {
+                            float t[4][16];
 #pragma unroll
-                            for (int z = 0; z < 3; ++z)
+                            for (int z = 0; z < 4; ++z, from += (size_t)p.n_block * 128)
 #pragma unroll
-                                for (int j = 0; j < 32; ++j) t[z][j] = part_of(z0 + z, j);
+                                for (int j = 0; j < 16; ++j) t[z][j] = (z0 + z < p.ksplit && j < n_ok) ? __ldcg(from + j * 128) : 0.0f;
 #pragma unroll
-                            for (int z = 0; z < 3; ++z)
+                            for (int z = 0; z < 4; ++z)
 #pragma unroll
-                                for (int j = 0; j < 32; ++j) d[j] = __float_as_uint(__uint_as_float(d[j]) + t[z][j]);
+                                for (int j = 0; j < 16; ++j) d[j] = __float_as_uint(__uint_as_float(d[j]) + t[z][j]);
                         }
-                        store_columns(mat, row, row_ok, u.m0 + c_first + c, min(n_ok, p.M - (u.m0 + c_first + c)), p.inv_xscale, rscale, lane, d);
+                        store_columns(mat, row, row_ok, u.m0 + c_first + c, min(n_ok, p.M - (u.m0 + c_first + c)), scales.chunk(c), c & 31, rscale, d);
                     }
                     if (lane == 0) *counter = 0u;
                 }
