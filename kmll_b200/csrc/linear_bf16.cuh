@@ -405,14 +405,14 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
     bool ok = true;
     if (warp == 0) {
         if (lane == 0) {
-            int it = 0;
+            PairRing ring(stages);
             for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
                 const int tile = item / p.ksplit, kt0 = (item % p.ksplit) * kt_per, kt1 = min(kt0 + kt_per, KT);
                 const int row0 = (tile / p.x_tiles) * kHRows, t0 = (tile % p.x_tiles) * p.n_block;
 #pragma unroll 1
-                for (int kt = kt0; kt < kt1; ++kt, ++it) {
-                    const int s = it % stages, use = it / stages;
-                    if (use > 0 && !mbar_wait<false>(&empty[s], (uint32_t)(use - 1) & 1u)) { ok = false; break; }
+                for (int kt = kt0; kt < kt1; ++kt, ring.next()) {
+                    const int s = ring.stage;
+                    if (ring.wrapped && !mbar_wait<false>(&empty[s], ring.phase ^ 1u)) { ok = false; break; }
                     const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
                     mbar_arrive_expect_tx(&full[s], (uint32_t)stage_bytes);
                     tma_load_2d(st, &map_w, kt * kHKT, row0, &full[s]);
@@ -422,16 +422,17 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            int it = 0, n = 0;
+            PairRing ring(stages);
+            int n = 0;
             for (int item = blockIdx.x; ok && item < items; item += gridDim.x, ++n) {
                 const int buf = n & 1, kt0 = (item % p.ksplit) * kt_per, kt1 = min(kt0 + kt_per, KT);
                 if (n >= 2 && !mbar_wait<false>(&acc_free[buf], (uint32_t)((n >> 1) - 1) & 1u)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t acc = tmem_base + (uint32_t)buf * 256u;
 #pragma unroll 1
-                for (int kt = kt0; kt < kt1; ++kt, ++it) {
-                    const int s = it % stages, use = it / stages;
-                    if (!mbar_wait<false>(&full[s], (uint32_t)use & 1u)) { ok = false; break; }
+                for (int kt = kt0; kt < kt1; ++kt, ring.next()) {
+                    const int s = ring.stage;
+                    if (!mbar_wait<false>(&full[s], ring.phase)) { ok = false; break; }
                     tcgen05_fence_after();
                     const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
 #pragma unroll
@@ -531,6 +532,247 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
     if (!ok) atomicCAS(&g_device_status, 0, 1);
 }
 
+// ---- more than 256 rows of x: pairs of multiprocessors ------------------------------------------------------------------------
+// The same contraction as linear_gemm_bf16_kernel on tcgen05.mma.cta_group::2: 256 weight rows (128 per block of a cluster of two)
+// against up to 256 rows of x, half of them in each block's shared memory - 32 KB per 64-column k-tile and block instead of 48.
+// Bound by the tensor cores.  What kept the one-block kernel at 0.43 of their rate on a prompt was its issuing thread: a commit holds it
+// for ~500 cycles, as long as the four MMAs of a k-tile take.  So two threads issue, even and odd k-tiles into an accumulator each;
+// the drain warps add the two in registers, give both back and store while the next unit's MMAs run (linear_gemm_pair.cuh has the
+// same structure and the reasons for its barriers).  Roles of a block: warp 0 TMA of x, warp 2 TMA of the weights,
+// warps 1 and 3 the issuers in the leader block; in the other block warp 1 tells the leader that a stage has landed;
+// warps 4-11 drain and store.  Registers: 56 + 2 x 224 = 3 x 168 per thread of a warpgroup.
+// Measured against the one-block kernel: 1024 x 4096 x 4096 93 -> 37 us, 1024 x 4096 x 14336 163 -> 91 (1317 TFLOP/s), 1024 x 14336 x
+// 4096 128 -> 98, 2048 x 28672 x 4096 404 -> 339 (1421), 300 x 4096 x 4096 38 -> 26.
+constexpr int kHPairThreads = 384;
+
+// The sums of a unit leave their registers 16 columns at a time in a ROLLED loop: a pass takes the first eight pairs and moves the
+// others down.  Unrolled over 128 columns, with every option of the epilogue in every column, it is code that a unit runs once, and
+// fetching its instructions took longer than anything else there (15 to 38 us for a 256 x 256 unit, now 5).
+template <int N>
+__device__ inline void take_columns(unsigned long long (&acc)[N], uint32_t (&d)[16]) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) d[j] = (uint32_t)(acc[j / 2] >> (32 * (j & 1)));
+#pragma unroll
+    for (int j = 0; j + 8 < N; ++j) acc[j] = acc[j + 8];
+}
+
+// 16 rows of x (t .. t + n_ok - 1) of one weight row; `warp_row`: the first of the warp's 32 rows
+__device__ inline void store_bf16_columns(const GemmBf16Params& p, int warp_row, int lane, int t, int n_ok, uint32_t (&d)[16]) {
+    const int row = warp_row + lane;
+    bool live = row < p.rows;
+    size_t o = (size_t)t * p.ldo + row;
+    if (p.pair_act != 0) {  // even lanes hold the gate, odd lanes its value
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float v = __shfl_xor_sync(0xffffffffu, __uint_as_float(d[j]), 1);
+            d[j] = __float_as_uint(apply_act(__uint_as_float(d[j]), p.pair_act) * v);
+        }
+        live = live && (lane & 1) == 0;
+        o = (size_t)t * p.ldo + (row >> 1);
+    } else if (warp_row < p.silu_rows) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (row < p.silu_rows) d[j] = __float_as_uint(act_silu(__uint_as_float(d[j])));
+    }
+    if (p.out_scale != 1.0f) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) d[j] = __float_as_uint(__uint_as_float(d[j]) * p.out_scale);
+    }
+    if (p.residual != nullptr) {
+        const float* res = p.residual + o;
+        float r[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j, res += p.ldo) r[j] = (live && j < n_ok) ? *res : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) d[j] = __float_as_uint(__uint_as_float(d[j]) + r[j]);
+    }
+    if (p.out_bf16) {
+        uint16_t* out = static_cast<uint16_t*>(p.out) + o;
+#pragma unroll
+        for (int j = 0; j < 16; ++j, out += p.ldo)
+            if (live && j < n_ok) *out = f32_to_bf16_bits(__uint_as_float(d[j]));
+    } else {
+        float* out = static_cast<float*>(p.out) + o;
+#pragma unroll
+        for (int j = 0; j < 16; ++j, out += p.ldo)
+            if (live && j < n_ok) *out = __uint_as_float(d[j]);
+    }
+}
+
+__global__ void __launch_bounds__(kHPairThreads, 1) linear_gemm_bf16_pair_kernel(const GemmBf16Params p, const __grid_constant__ CUtensorMap map_w,
+                                                                                 const __grid_constant__ CUtensorMap map_x) {
+    extern __shared__ unsigned char bpsmem_raw[];
+    unsigned char* smem = bpsmem_raw + ((1024u - (smem_u32(bpsmem_raw) & 1023u)) & 1023u);  // the same offset in both blocks
+    const int n_half = p.n_block / 2, a_bytes = kHRows * 128, b_bytes = n_half * 128, stage_bytes = a_bytes + b_bytes;  // multiples of 1024
+    const int stages = p.stages;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)stages * stage_bytes);  // own block's copies of a stage have landed
+    uint64_t* peer_full = full + stages;    // in the leader: the other block's have
+    uint64_t* empty = peer_full + stages;   // in each block: the MMAs that read a stage have completed
+    uint64_t* acc_full = empty + stages;    // [2], in each block
+    uint64_t* acc_empty = acc_full + 2;     // [2], in the leader: drained by both blocks' eight warps
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = (int)(blockIdx.x & 1u), cluster = (int)(blockIdx.x >> 1), n_clusters = (int)(gridDim.x >> 1);
+    const int KT = (p.K + kHKT - 1) / kHKT;
+
+    if (tid == 0) {
+        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 2); mbar_init(&peer_full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");  // the other block's barriers exist
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t smem_base = smem_u32(smem);
+    bool ok = true;
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        pdl_wait();
+        if (lane == 0) {
+            PairRing ring(stages);
+            if (warp == 0 || warp == 2) {
+                for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters) {
+                    const int rt = unit / p.x_tiles, row0 = rt * 256 + rank * 128, t0 = (unit - rt * p.x_tiles) * p.n_block + rank * n_half;
+#pragma unroll 1
+                    for (int kt = 0; kt < KT; ++kt, ring.next()) {
+                        const int s = ring.stage;
+                        if (ring.wrapped && !mbar_wait<false>(&empty[s], ring.phase ^ 1u)) { ok = false; break; }
+                        const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
+                        if (warp == 0) {
+                            mbar_arrive_expect_tx(&full[s], (uint32_t)b_bytes);
+                            tma_load_2d(st + a_bytes, &map_x, kt * kHKT, t0, &full[s]);
+                        } else {
+                            mbar_arrive_expect_tx(&full[s], (uint32_t)a_bytes);
+                            tma_load_2d(st, &map_w, kt * kHKT, row0, &full[s]);
+                        }
+                    }
+                }
+                // nothing of this block's copies, and no arrival on its barriers, is in flight when it reaches the end
+                for (int j = 0; j < stages; ++j, ring.next())
+                    if (ring.wrapped && !mbar_wait<false>(ok ? &empty[ring.stage] : &full[ring.stage], ring.phase ^ 1u)) { ok = false; break; }
+            } else if (rank == 0) {
+                const uint32_t idesc = gemm_idesc_bf16(256, p.n_block);
+                const int own = warp >> 1;
+                const uint32_t dst = tmem_base + (uint32_t)own * 256u;
+                uint32_t uses = 0;
+                for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters) {
+#pragma unroll 1
+                    for (int kt = 0; kt < KT; ++kt, ring.next()) {
+                        if ((kt & 1) != own) continue;
+                        const int s = ring.stage;
+                        if (kt < 2 && uses > 0 && !mbar_wait<false>(&acc_empty[own], (uses - 1) & 1u)) { ok = false; break; }
+                        if (!mbar_wait<false>(&full[s], ring.phase) || !mbar_wait<false>(&peer_full[s], ring.phase)) { ok = false; break; }
+                        tcgen05_fence_after();
+                        const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
+                        const uint64_t da = gemm_smem_desc(st), db = gemm_smem_desc(st + a_bytes);
+#pragma unroll
+                        for (int ks = 0; ks < kHKT / 16; ++ks) pair_mma_f16(dst, da + 2 * ks, db + 2 * ks, idesc, (kt > 1 || ks > 0) ? 1u : 0u);
+                        pair_commit(&empty[s]);
+                        if (kt + 2 >= KT) {
+                            pair_commit(&acc_full[own]);
+                            ++uses;
+                        }
+                    }
+                }
+            } else if (warp == 1) {
+                for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters)
+#pragma unroll 1
+                    for (int kt = 0; kt < KT; ++kt, ring.next()) {
+                        if (!mbar_wait<false>(&full[ring.stage], ring.phase)) { ok = false; break; }
+                        mbar_arrive_leader(&peer_full[ring.stage]);
+                    }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        pdl_wait();
+        const int q = warp & 3, half = (warp - 4) >> 2, c_first = half * n_half;
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c_first;
+        uint32_t phase = 0u;
+        for (int unit = cluster; unit < p.tiles; unit += n_clusters, phase ^= 1u) {
+            const int rt = unit / p.x_tiles, row0 = rt * 256 + rank * 128 + q * 32, t0 = (unit - rt * p.x_tiles) * p.n_block + c_first;
+            unsigned long long acc[64];  // pairs of f32 sums
+#pragma unroll
+            for (int j = 0; j < 64; ++j) acc[j] = 0ull;
+#pragma unroll 1
+            for (int g = 0; g < min(KT, 2); ++g) {
+                ok = __all_sync(0xffffffffu, mbar_wait<false>(&acc_full[g], phase));
+                if (!ok) break;
+                tcgen05_fence_after();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c * 32 < n_half) {
+                        uint32_t d[32];
+                        tmem_load_x32(taddr + (uint32_t)g * 256u + (uint32_t)c * 32u, d);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) fma_pair(acc[c * 16 + j], 0x3f8000003f800000ull, d[2 * j], d[2 * j + 1]);
+                    }
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_leader(&acc_empty[g]);
+            }
+            if (!ok) break;
+#pragma unroll 1
+            for (int c = 0; c < n_half; c += 16) {  // (rolled: take_columns)
+                uint32_t d[16];
+                take_columns(acc, d);
+                store_bf16_columns(p, row0, lane, t0 + c, min(n_half - c, p.T - (t0 + c)), d);
+            }
+        }
+    }
+    // neither block may leave, or free tensor memory, while the other can still signal its barriers or read its operands
+    if (!ok) atomicCAS(&g_device_status, 0, 1);
+    __syncwarp();
+    tcgen05_fence_before();
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    tcgen05_fence_after();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+}
+
+// Up to 256 rows of x the one-block kernel keeps more multiprocessors busy (128-row tiles, K cut into pieces).
+static int bf16_gemm_pair(cudaStream_t stream, const Bf16Gemm& g, GemmBf16Params p) {
+    // rows of x per unit: a k-tile takes four MMAs of n / 2 + 15 cycles, a unit ~2500 more until both accumulators are drained
+    const int KT = (g.K + kHKT - 1) / kHKT, row_tiles = (g.rows + 255) / 256, xb_min = (g.T + kHMaxN - 1) / kHMaxN;
+    double best_cost = 1e30;
+    for (int xb = xb_min; xb <= 4 * xb_min; ++xb) {
+        const int n = (((g.T + xb - 1) / xb) + 15) & ~15;
+        if (xb > xb_min && n < 96) break;
+        const long long units = (long long)row_tiles * ((g.T + n - 1) / n);
+        const double cost = (double)((units + kPClusters - 1) / kPClusters) * (KT * (2.0 * n + 60.0) + 2500.0);
+        if (cost < best_cost * 0.995) {
+            best_cost = cost;
+            p.n_block = n;
+            p.x_tiles = (g.T + n - 1) / n;
+            p.tiles = (int)units;
+        }
+    }
+    p.row_tiles = row_tiles;
+    p.ksplit = 1;
+    const size_t stage = (size_t)kHRows * 128 + (size_t)p.n_block * 64;
+    p.stages = (int)((size_t)(227 * 1024 - 1024 - 512) / stage);
+    if (p.stages > 12) p.stages = 12;
+    const size_t smem = p.stages * stage + (3 * p.stages + 4) * 8 + 16 + 1024;
+    CUtensorMap map_w, map_x;
+    KMLL_TRY_RC(make_map_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.w, (uint64_t)g.K, (uint64_t)g.rows, (uint64_t)g.ldw * 2, kHKT, kHRows,
+                            CU_TENSOR_MAP_SWIZZLE_128B));
+    KMLL_TRY_RC(make_map_2d(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.x, (uint64_t)g.K, (uint64_t)g.T, (uint64_t)g.ldx * 2, kHKT,
+                            (uint32_t)p.n_block / 2, CU_TENSOR_MAP_SWIZZLE_128B));
+    cudaError_t e = allow_all_dynamic_smem(linear_gemm_bf16_pair_kernel);
+    const int clusters = p.tiles < kPClusters ? p.tiles : kPClusters;
+    if (e == cudaSuccess)
+        e = launch_cluster(linear_gemm_bf16_pair_kernel, dim3(2 * clusters), 2, dim3(kHPairThreads), smem, stream, true, p, map_w, map_x);
+    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "linear_gemm_bf16_pair: %s", cudaGetErrorString(e));
+    return KMLL_OK;
+}
+
 // ---- many rows of x, f32 on the CUDA cores -----------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) gemm_f32_kernel(const Bf16Gemm g) {
     constexpr int BT = 64, BR = 64, BK = 16;
@@ -615,6 +857,7 @@ int bf16_gemm(cudaStream_t stream, const Bf16Gemm& g) {
     p.x_tiles = (g.T + best - 1) / best;  // walked fastest: the blocks at work share their weight rows, and x stays in L2
     const long long tiles = (long long)p.row_tiles * p.x_tiles;
     if (tiles > 0x3fffffff) return fail(KMLL_ERR_UNSUPPORTED, "bf16_gemm: too many tiles");
+    if (g.T > kHMaxN) return bf16_gemm_pair(stream, g, p);
     p.tiles = (int)tiles;
     p.ksplit = 1;
     if (g.partial != nullptr && g.T <= kGemmSplitRows && p.tiles <= 74) {  // at least eight k-tiles per piece

@@ -494,3 +494,28 @@ def test_bf16_linear_operators(cuda):
         n = lo.rms_norm_plain(o, norm.double().cpu().numpy(), 1e-3) * lo.sigmoid(gate.double().cpu().numpy())
         got = ops.gated_linear_bf16(x[0].contiguous(), gate, w, 1e-3, norm_weight=norm, sigmoid=True)
         assert float((got.double() - w0 @ torch.from_numpy(n).cuda()).abs().max()) <= 4e-5 * cols ** 0.5
+
+
+# more than 256 rows of x: pairs of blocks.  One k-tile (one accumulator), a ragged last one, one row of weights, ragged tiles on both
+# sides, several units per pair
+@pytest.mark.parametrize("tokens,rows,cols", [(257, 130, 72), (300, 2, 64), (513, 520, 200), (640, 257, 1000), (1030, 6000, 136), (2500, 384, 4104)])
+def test_bf16_gemm_of_many_rows(cuda, tokens, rows, cols):
+    """Against 64-bit sums: f32 accumulation in steps of 16 columns (2^-23 of the partial sum each), bf16 results half an ulp more."""
+    import torch
+
+    from kmll_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, cols, generator=gen, device="cuda").bfloat16()
+    w = torch.randn(rows, cols, generator=gen, device="cuda").bfloat16()
+    res = torch.randn(tokens, rows, generator=gen, device="cuda")
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    bound = (cols / 16 + 8) * 2.0 ** -23 * (size + res.double().abs())
+    assert bool(((ops.linear_batched_bf16(x, w, residual=res).double() - want - res.double()).abs() <= bound).all())
+    assert bool(((ops.linear_batched_bf16(x, w, out_bf16=True).double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all())
+    if rows % 2 == 0:
+        gate, up = want[:, 0::2], want[:, 1::2]
+        got = ops.pair_linear_batched_bf16(x, w, 1).double()  # SiLU
+        pair = torch.nn.functional.silu(gate) * up
+        slack = bound[:, 0::2] * up.abs() * 1.1 + bound[:, 1::2] * gate.abs() + 2.0 ** -20 * pair.abs()
+        assert bool(((got - pair).abs() <= slack + 2.0 ** -8 * pair.abs()).all())
