@@ -263,6 +263,75 @@ __global__ void prepare_prefill_kernel(const float* __restrict__ q, const float*
     }
 }
 
+// The same for whole heads (no pass-through entries) in pieces of four aligned values.  A block serves one row, or one of `parts`
+// shares of its pieces: the row's sines and cosines are computed once into shared memory instead of once per rotated value, and
+// every load and store is 16 bytes.  Bound by HBM: 2048 rows of 32 + 2 x 8 heads of 128, 60 -> 20 us.
+__global__ void __launch_bounds__(256) prepare_prefill_quads_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                                    const float* __restrict__ freqs, int half, int q_len, int kv_len, int position0,
+                                                                    float* __restrict__ q_rot, float* __restrict__ k_cache, float* __restrict__ v_cache,
+                                                                    int kv_bf16) {
+    extern __shared__ float turns[];  // [half] cosines, [half] sines
+    pdl_wait();
+    const int row = blockIdx.x;
+    const float position = (float)(position0 + row);
+    for (int i = threadIdx.x; i < half; i += 256) {
+        const float angle = position * freqs[i];
+        turns[i] = cosf(angle);
+        turns[half + i] = sinf(angle);
+    }
+    __syncthreads();
+    // pieces: four pairs of a query head, four pairs of a key head, four values
+    const int per = half >> 2, nq = q_len >> 3, nk = kv_len >> 3, nv = kv_len >> 2;
+    const size_t q0 = (size_t)row * q_len, kv0 = (size_t)row * kv_len, cache0 = (size_t)(position0 + row) * kv_len;
+    auto put = [&](float* cache, size_t at, const float4& x) {
+        if (kv_bf16) {
+            const uint32_t lo = (uint32_t)f32_to_bf16_bits(x.x) | ((uint32_t)f32_to_bf16_bits(x.y) << 16);
+            const uint32_t hi = (uint32_t)f32_to_bf16_bits(x.z) | ((uint32_t)f32_to_bf16_bits(x.w) << 16);
+            *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(cache) + at) = make_uint2(lo, hi);
+        } else {
+            *reinterpret_cast<float4*>(cache + at) = x;
+        }
+    };
+    for (int i = (int)blockIdx.y * 256 + threadIdx.x; i < nq + nk + nv; i += 256 * (int)gridDim.y) {
+        if (i >= nq + nk) {
+            const int c = (i - nq - nk) * 4;
+            put(v_cache, cache0 + c, *reinterpret_cast<const float4*>(v + kv0 + c));
+            continue;
+        }
+        const bool is_q = i < nq;
+        const int j = is_q ? i : i - nq, head = j / per, c = (j - head * per) * 4, at = head * 2 * half + c;
+        const float* src = (is_q ? q + q0 : k + kv0) + at;
+        const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + half);
+        const float4 co = *reinterpret_cast<const float4*>(turns + c), si = *reinterpret_cast<const float4*>(turns + half + c);
+        // (rope_value's two products and one sum)
+        const float4 x = make_float4(a.x * co.x - b.x * si.x, a.y * co.y - b.y * si.y, a.z * co.z - b.z * si.z, a.w * co.w - b.w * si.w);
+        const float4 y = make_float4(b.x * co.x + a.x * si.x, b.y * co.y + a.y * si.y, b.z * co.z + a.z * si.z, b.w * co.w + a.w * si.w);
+        if (is_q) {
+            *reinterpret_cast<float4*>(q_rot + q0 + at) = x;
+            *reinterpret_cast<float4*>(q_rot + q0 + at + half) = y;
+        } else {
+            put(k_cache, cache0 + at, x);
+            put(k_cache, cache0 + at + half, y);
+        }
+    }
+}
+
+// Whole heads in aligned pieces of four, or one value per thread.  (The caches' alignment is that of their base: rows are multiples
+// of a head.)  Short prompts share a row between up to four blocks.
+static cudaError_t launch_prepare_prefill(cudaStream_t stream, const float* q, const float* k, const float* v, const float* freqs, int half, int rows, int q_len,
+                                          int kv_len, int head_dim, int position0, float* q_rot, float* k_cache, float* v_cache, int kv_bf16) {
+    uintptr_t bits = 0;
+    for (const void* p : {(const void*)q, (const void*)k, (const void*)v, (const void*)q_rot, (const void*)k_cache, (const void*)v_cache}) bits |= reinterpret_cast<uintptr_t>(p);
+    if (2 * half == head_dim && half % 4 == 0 && half <= 4096 && (bits & 15u) == 0) {
+        const int parts = rows >= 148 ? 1 : rows >= 74 ? 2 : 4;
+        return launch(prepare_prefill_quads_kernel, dim3(rows, parts), dim3(256), (size_t)half * 8, stream, true, q, k, v, freqs, half, q_len, kv_len, position0, q_rot,
+                      k_cache, v_cache, kv_bf16);
+    }
+    const size_t total = (size_t)rows * (q_len > kv_len ? q_len : kv_len);
+    return launch(prepare_prefill_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, true, q, k, v, freqs, half, rows, q_len, kv_len, head_dim,
+                  position0, q_rot, k_cache, v_cache, kv_bf16);
+}
+
 // ---- row softmax --------------------------------------------------------------------------------
 // max, sum of exp(x-max), exp(x-max)/sum (crates/inference/src/kernels/inference.rs:1343-1398).
 // The row is held in registers between the passes when it fits, so HBM sees one read + one write.
@@ -498,10 +567,7 @@ int qk_head_rmsnorm(cudaStream_t stream, float* q, float* k, const uint16_t* q_w
 int prepare_prefill_offset(cudaStream_t stream, const float* q, const float* k, const float* v, const float* freqs,
                            int n_freqs, int rows, int q_len, int kv_len, int head_dim, int position0, float* q_rot,
                            float* k_cache, float* v_cache, int kv_bf16) {
-    const int width = q_len > kv_len ? q_len : kv_len;
-    const size_t total = (size_t)rows * width;
-    cudaError_t e = launch(prepare_prefill_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, true, q, k, v,
-                           freqs, n_freqs, rows, q_len, kv_len, head_dim, position0, q_rot, k_cache, v_cache, kv_bf16);
+    cudaError_t e = launch_prepare_prefill(stream, q, k, v, freqs, n_freqs, rows, q_len, kv_len, head_dim, position0, q_rot, k_cache, v_cache, kv_bf16);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "prepare_prefill: %s", cudaGetErrorString(e));
     return KMLL_OK;
 }
@@ -756,9 +822,7 @@ int kmll_prepare_prefill_attention_batch(kmll_stream_t s, const float* q, const 
     if (rc) return rc;
     KMLL_REQUIRE(q_len > 0 && q_len % head_dim == 0, "prepare_prefill_attention_batch: query row shape mismatch");
     KMLL_REQUIRE(kv_len > 0 && kv_len % head_dim == 0, "prepare_prefill_attention_batch: KV row shape mismatch");
-    const int width = q_len > kv_len ? q_len : kv_len;
-    const size_t total = (size_t)prompt_len * width;
-    KMLL_LAUNCH_CHECK(launch(prepare_prefill_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, as_stream(s), true, q, k, v, freqs, n_freqs, prompt_len, q_len, kv_len, head_dim, 0, q_rot, k_cache, v_cache, 0), "prepare_prefill_attention_batch");
+    KMLL_LAUNCH_CHECK(launch_prepare_prefill(as_stream(s), q, k, v, freqs, n_freqs, prompt_len, q_len, kv_len, head_dim, 0, q_rot, k_cache, v_cache, 0), "prepare_prefill_attention_batch");
     return KMLL_OK;
 }
 

@@ -606,3 +606,22 @@ def test_prefill_attention_against_64_bits(cuda, n, h, g, d, shift):
         step = float((q64[head].abs() @ kh.abs().T).max()) * d ** -0.5
         bound = (2 * (d + 8) * 2.0 ** -24 * step + (n + 64) * 2.0 ** -23) * float(vh.abs().max())
         assert float((got[:, head] - w @ vh).abs().max()) <= bound
+
+
+# whole heads in aligned pieces (one, two or four blocks per row), part of a head rotated, unaligned rows: one value per thread
+@pytest.mark.parametrize("n,h,g,d,half,shift", [(1, 2, 2, 128, 64, 0), (5, 14, 2, 64, 32, 0), (80, 3, 1, 128, 64, 0), (150, 32, 8, 128, 64, 0), (7, 4, 2, 64, 16, 0),
+                                                (9, 4, 2, 64, 32, 1), (3, 2, 1, 12, 6, 0)])
+def test_prepare_prefill_against_64_bits(cuda, n, h, g, d, half, shift):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn(n * w * d + shift, generator=gen, device="cuda")[shift:] for w in (h, g, g))
+    freqs = (1e4 ** (-torch.arange(half, dtype=torch.float64) / half)).float().cuda()
+    q_rot, kc, vc = torch.zeros_like(q), torch.zeros(n * g * d, device="cuda"), torch.zeros(n * g * d, device="cuda")
+    ops.prepare_prefill_attention_batch(q, k, v, freqs, n, h * d, g * d, d, q_rot, kc, vc)
+    angle = (torch.arange(n, device="cuda", dtype=torch.float32)[:, None] * freqs[None, :]).double()[:, None, :]
+    for x, got in ((q, q_rot), (k, kc)):
+        x64 = x.view(n, -1, d).double()
+        a, b, rest = x64[..., :half], x64[..., half:2 * half], x64[..., 2 * half:]
+        want = torch.cat((a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin(), rest), -1)
+        size = torch.cat((a.abs() + b.abs(), a.abs() + b.abs(), torch.zeros_like(rest)), -1)
+        assert bool(((got.view(n, -1, d).double() - want).abs() <= 2.0 ** -21 * size).all())  # sine, cosine, two products, a sum
+    assert torch.equal(vc, v)
