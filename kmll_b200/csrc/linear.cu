@@ -1022,7 +1022,7 @@ static bool gemm_small_enabled() {
 
 // Small batches of W4-G128 (linear_gemm_small.cuh): byte digits of x, then ONE persistent launch over the row tiles of
 // all matrices.
-static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, int M, int K, int ldx, const uint16_t* norm_w, float eps, const void* const* w,
+static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, const float* up, int M, int K, int ldx, const uint16_t* norm_w, float eps, const void* const* w,
                           const void* const* scales, const int* rows, float* const* outs, const float* const* residuals, const int* ldos,
                           int nmat, void* workspace, const GemmPlan& big) {
     const bool w4 = fmt == FMT_W4;
@@ -1032,8 +1032,10 @@ static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, int M, i
     float* partial = reinterpret_cast<float*>(ws + big.off_partial);
     unsigned int* counters = reinterpret_cast<unsigned int*>(ws + big.off_counters);
     const int permute = w4 ? 1 : 0;
-    cudaError_t e = K <= 16384 ? launch(digit_rows_kernel<true>, dim3(M), dim3(512), 0, stream, true, x, ldx, K, M, norm_w, eps, digits, inv, counters, 16384, permute)
-                               : launch(digit_rows_kernel<false>, dim3(M), dim3(512), 0, stream, true, x, ldx, K, M, norm_w, eps, digits, inv, counters, 16384, permute);
+    int cluster = 1;  // blocks per row: one run of eight columns per thread
+    while (cluster < 8 && cluster * kDigitThreads * 8 < K) cluster *= 2;
+    cudaError_t e = launch_cluster(digit_rows_kernel, dim3(cluster, M), cluster, dim3(kDigitThreads), 0, stream, true, x, up, ldx, K, M, norm_w, eps, digits, inv, counters,
+                                   16384, permute);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "digit_rows: %s", cudaGetErrorString(e));
     const int nb = M <= 16 ? 16 : 32;
     const int gp = (w4 && nb == 16 && K >= 256) ? 2 : 1;  // groups per pipeline item (SmallShape)
@@ -1123,8 +1125,8 @@ static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, int M, i
     return KMLL_OK;
 }
 
-// y[m, :] (+= residual) = dequant(W_i) x[m, :] for every matrix i; x is split into f16 planes once for all of them.  With `up` (more
-// than 32 rows only) the input is SiLU(x) * up.
+// y[m, :] (+= residual) = dequant(W_i) x[m, :] for every matrix i; x is split into f16 planes once for all of them.  With `up`
+// the input is SiLU(x) * up.
 template <int FMT>
 static int run_gemm(cudaStream_t stream, const float* x, const float* up, int M, int K, int ldx, const uint16_t* norm_w, float eps, const void* const* w,
                     const void* const* scales, const int* rows, float* const* outs, const float* const* residuals, const int* ldos, int nmat,
@@ -1136,7 +1138,7 @@ static int run_gemm(cudaStream_t stream, const float* x, const float* up, int M,
     // 5 to 32 rows of x: the persistent kind::i8 kernels (RS-I8 needs at least two 128-column groups and K <= 131072 for its
     // s32 accumulators)
     if (M <= 32 && gemm_small_enabled() && (FMT == FMT_W4 || (K >= 256 && K <= 131072)))
-        return run_gemm_small(FMT, stream, x, M, K, ldx, norm_w, eps, w, scales, rows, outs, residuals, ldos, nmat, workspace, big);
+        return run_gemm_small(FMT, stream, x, up, M, K, ldx, norm_w, eps, w, scales, rows, outs, residuals, ldos, nmat, workspace, big);
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     __half* x_hi = reinterpret_cast<__half*>(ws);
     __half* x_lo = reinterpret_cast<__half*>(ws + big.off_lo);
@@ -1430,7 +1432,7 @@ static int batched_forms(int form, cudaStream_t stream, const float* x, int batc
         }
         case 5: {  // SiLU(gate) * up + projection + residual: the activation is formed where the tensor-core path splits its input
             GemmPlan pl;
-            if (batch > 32 && workspace != nullptr && gemm_enabled() && (cols & 3) == 0 && aligned16(gate_tmp) && aligned16(up_tmp) && aligned16(workspace) &&
+            if (workspace != nullptr && gemm_enabled() && (cols & 3) == 0 && aligned16(gate_tmp) && aligned16(up_tmp) && aligned16(workspace) &&
                 aligned16(w[0]) && gemm_plan(FMT, batch, cols, rows[0], &pl)) {
                 const int ldo = rows[0];
                 return run_gemm<FMT>(stream, gate_tmp, up_tmp, batch, cols, cols, nullptr, 0.f, w, scales, rows, outs, &residual, &ldo, 1, workspace);

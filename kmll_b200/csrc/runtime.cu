@@ -724,20 +724,20 @@ static int enqueue_batch_step(BatchDecoder* b, cudaStream_t s, int* launches) {
             float* outs[1] = {b->hidden_mid};
             KMLL_TRY(linear_batched_form(2, s, c.format, b->attn, B, nullptr, 0.f, w, sc, rows, q_len, outs, hidden, b->linear_ws));
         }
-        {
-            const void* w[2] = {L.w1.w, L.w3.w};
-            const void* sc[2] = {L.w1.scales, L.w3.scales};
-            const int rows[1] = {c.hidden_dim};
-            float* outs[1] = {b->act};
-            KMLL_TRY(linear_batched_form(1, s, c.format, b->hidden_mid, B, L.ffn_norm, c.norm_eps, w, sc, rows, c.dim, outs, nullptr, b->linear_ws, b->gate,
+        const void* w13[2] = {L.w1.w, L.w3.w};
+        const void* sc13[2] = {L.w1.scales, L.w3.scales};
+        const void* w2[1] = {L.w2.w};
+        const void* sc2[1] = {L.w2.scales};
+        const int hidden_rows[1] = {c.hidden_dim}, dim_rows[1] = {c.dim};
+        float *act_out[1] = {b->act}, *out[1] = {other};
+        if (b->linear_ws != nullptr) {  // SiLU * up is formed where the down projection reads its input
+            KMLL_TRY(linear_batched_form(4, s, c.format, b->hidden_mid, B, L.ffn_norm, c.norm_eps, w13, sc13, hidden_rows, c.dim, nullptr, nullptr, b->linear_ws,
+                                         b->gate, b->up));
+            KMLL_TRY(linear_batched_form(5, s, c.format, nullptr, B, nullptr, 0.f, w2, sc2, dim_rows, c.hidden_dim, out, b->hidden_mid, b->linear_ws, b->gate, b->up));
+        } else {
+            KMLL_TRY(linear_batched_form(1, s, c.format, b->hidden_mid, B, L.ffn_norm, c.norm_eps, w13, sc13, hidden_rows, c.dim, act_out, nullptr, b->linear_ws, b->gate,
                                          b->up));
-        }
-        {
-            const void* w[1] = {L.w2.w};
-            const void* sc[1] = {L.w2.scales};
-            const int rows[1] = {c.dim};
-            float* outs[1] = {other};
-            KMLL_TRY(linear_batched_form(2, s, c.format, b->act, B, nullptr, 0.f, w, sc, rows, c.hidden_dim, outs, b->hidden_mid, b->linear_ws));
+            KMLL_TRY(linear_batched_form(2, s, c.format, b->act, B, nullptr, 0.f, w2, sc2, dim_rows, c.hidden_dim, out, b->hidden_mid, b->linear_ws));
         }
         float* t = hidden;
         hidden = other;
