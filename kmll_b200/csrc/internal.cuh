@@ -190,7 +190,7 @@ int widen_bf16(cudaStream_t stream, const uint16_t* src, size_t n, float* dst);
 // linear.cu: lm_head arg-max whose token ids are offset (vocabulary shards of tensor parallelism)
 int linear_top1_offset(cudaStream_t stream, int fmt, const float* x, const uint16_t* norm_w, float eps, const void* w,
                        const void* scales, int rows, int cols, uint32_t token_offset, uint32_t* partial_tokens,
-                       float* partial_logits, uint64_t* packed_out, const TpExchange* xc = nullptr);
+                       float* partial_logits, uint64_t* packed_out, const TpExchange* xc = nullptr, DecodeState* state = nullptr);
 // Batched fused linear forms for rows of x that are independent sequences (batch <= 16 per pass):
 // form 0 = RMSNorm + QKV (3 matrices, rows[0..2]), 1 = RMSNorm + gate/up + SiLU*up (2 matrices of rows[0]),
 // 2 = projection + residual, 3 = (RMSNorm +) projection, 4 = RMSNorm + gate/up into gate_tmp and up_tmp, 5 = SiLU(gate_tmp) *

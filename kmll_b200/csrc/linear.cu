@@ -534,10 +534,11 @@ __global__ void __launch_bounds__(1024) linear_i8_rowwarp_top1_kernel(const floa
     }
 }
 
-// Second stage of the fused arg-max: one block reduces the per-block partials
+// Second stage of the fused arg-max: one block reduces the per-block partials; with `state` it also ends the decode step (a launch of
+// its own before: 2 us of each step)
 // (argmax_pairs_f32_packed_kernel, crates/inference/src/kernels/inference.rs:1812-1878).
 __global__ void top1_reduce_kernel(const uint32_t* __restrict__ tokens, const float* __restrict__ logits, int count,
-                                   uint32_t token_offset, uint64_t* __restrict__ packed_out, const TpExchange* xcp) {
+                                   uint32_t token_offset, uint64_t* __restrict__ packed_out, const TpExchange* xcp, DecodeState* state) {
     pdl_wait();
     __shared__ float s_logit[32];
     __shared__ uint32_t s_tok[32];
@@ -571,6 +572,11 @@ __global__ void top1_reduce_kernel(const uint32_t* __restrict__ tokens, const fl
         if (lane == 0) {
             const uint64_t packed = pack_top1(best, tok == 0xffffffffu ? tok : tok + token_offset);
             packed_out[0] = packed;
+            if (state != nullptr) {
+                state->next_top = packed;
+                state->position += 1;
+                state->step += 1;
+            }
             if (xcp != nullptr) {  // tensor parallel: hand this rank's result to every rank (two 8-byte words)
                 const TpExchange& xc = *xcp;
                 const unsigned int epoch = *xc.epoch * (unsigned int)xc.mult + (unsigned int)xc.top_index + 1u;
@@ -1354,7 +1360,7 @@ static int run_linear(const char* name, cudaStream_t stream, const float* x, int
 template <int FMT>
 static int run_top1(const char* name, cudaStream_t stream, const float* x, const uint16_t* norm_w, float eps,
                     const void* w, const void* scales, int rows, int cols, uint32_t* partial_tokens,
-                    float* partial_logits, uint64_t* packed_out, uint32_t token_offset = 0, const TpExchange* xc = nullptr) {
+                    float* partial_logits, uint64_t* packed_out, uint32_t token_offset = 0, const TpExchange* xc = nullptr, DecodeState* state = nullptr) {
     if (partial_tokens == nullptr || partial_logits == nullptr || packed_out == nullptr) {
         set_exchange_args(nullptr, -1, -1, nullptr);
         return fail(KMLL_ERR_NULL, "%s: null partial/packed buffer", name);
@@ -1364,7 +1370,7 @@ static int run_top1(const char* name, cudaStream_t stream, const float* x, const
     int rc = run_linear<FMT, EPI_TOP1>(name, stream, x, 1, cols, cols, norm_w, eps, &m, 1, 0, partial_tokens, partial_logits, &count);
     if (rc != KMLL_OK) return rc;
     cudaError_t e = launch(top1_reduce_kernel, dim3(1), dim3(256), 0, stream, true, (const uint32_t*)partial_tokens,
-                           (const float*)partial_logits, count, token_offset, packed_out, xc);
+                           (const float*)partial_logits, count, token_offset, packed_out, xc, state);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "%s: %s", name, cudaGetErrorString(e));
     return KMLL_OK;
 }
@@ -1386,12 +1392,12 @@ __global__ void merge_packed_kernel(const uint64_t* __restrict__ packed_all, int
 
 int linear_top1_offset(cudaStream_t stream, int fmt, const float* x, const uint16_t* norm_w, float eps, const void* w,
                        const void* scales, int rows, int cols, uint32_t token_offset, uint32_t* partial_tokens,
-                       float* partial_logits, uint64_t* packed_out, const TpExchange* xc) {
+                       float* partial_logits, uint64_t* packed_out, const TpExchange* xc, DecodeState* state) {
     if (fmt == FMT_W4)
         return run_top1<FMT_W4>("linear_top1", stream, x, norm_w, eps, w, scales, rows, cols, partial_tokens, partial_logits,
-                                packed_out, token_offset, xc);
+                                packed_out, token_offset, xc, state);
     return run_top1<FMT_I8>("linear_top1", stream, x, norm_w, eps, w, scales, rows, cols, partial_tokens, partial_logits,
-                            packed_out, token_offset, xc);
+                            packed_out, token_offset, xc, state);
 }
 
 int decode_end_gather(cudaStream_t stream, const TpExchange* xc, DecodeState* state, uint64_t* packed_final) {

@@ -142,7 +142,8 @@ static int row_parallel_residual(Decoder* d, cudaStream_t s, const float* x, con
 // lm_head arg-max of `hidden` into d->packed_final (and the decode state is NOT touched).
 // With gather_index >= 0 (peer-memory exchange) the hidden state is first summed from the ranks' partial vectors
 // (and written to `hidden_out`), and this rank's result is pushed to every rank for decode_end_gather.
-static int output_top1(Decoder* d, cudaStream_t s, const float* hidden, int gather_index = -1, float* hidden_out = nullptr) {
+// `end_step` (one GPU, fused): the step's end rides on the arg-max.
+static int output_top1(Decoder* d, cudaStream_t s, const float* hidden, int gather_index = -1, float* hidden_out = nullptr, bool end_step = false) {
     const kmll_decoder_config& c = d->cfg;
     const uint32_t offset = (uint32_t)(c.tp_rank * d->vocab_l);
     uint64_t* dst = c.tp_size == 1 ? d->packed_final : d->packed;
@@ -153,7 +154,7 @@ static int output_top1(Decoder* d, cudaStream_t s, const float* hidden, int gath
     }
     if (c.fused) {
         KMLL_TRY(linear_top1_offset(s, c.format, hidden, d->final_norm, c.norm_eps, d->output.w, d->output.scales, d->vocab_l, c.dim,
-                                    offset, d->part_tok, d->part_logit, dst));
+                                    offset, d->part_tok, d->part_logit, dst, nullptr, end_step ? d->state : nullptr));
     } else {
         KMLL_TRY(kmll_rmsnorm(s, hidden, d->final_norm, c.dim, c.norm_eps, d->normed));
         KMLL_TRY(linear_top1_offset(s, c.format, d->normed, nullptr, 0.0f, d->output.w, d->output.scales, d->vocab_l, c.dim, offset,
@@ -233,10 +234,13 @@ static int enqueue_step_fused(Decoder* d, cudaStream_t s, int* launches) {
         KMLL_TRY(decode_end_gather(s, d->xc, d->state, d->packed_final));
         n += 3;
     } else {
-        KMLL_TRY(output_top1(d, s, hidden));
+        const bool end = c.tp_size == 1 && c.fused;
+        KMLL_TRY(output_top1(d, s, hidden, -1, nullptr, end));
         n += 2 + (c.tp_size > 1 ? 2 : 0);
-        KMLL_TRY(decode_end(s, d->packed_final, d->state));
-        ++n;
+        if (!end) {
+            KMLL_TRY(decode_end(s, d->packed_final, d->state));
+            ++n;
+        }
     }
     // keep the final hidden state where kmll_decoder_last_hidden finds it
     if (hidden != d->hidden_a) {
