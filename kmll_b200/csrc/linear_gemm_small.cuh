@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kDigitThreads) digit_rows_kernel(const float* 
                                                                    const uint16_t* __restrict__ norm_w, float eps, int8_t* __restrict__ digits,
                                                                    float* __restrict__ inv_xscale, unsigned int* counters, int n_counters, int permute) {
     __shared__ float2 warp_part[kDigitThreads / 32], block_part[8];
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");  // this block runs: the others may write to its shared memory
     pdl_wait();
     pdl_launch_dependents();  // the kernel that follows starts bringing in its weights; it waits for this grid before it reads the digits
     const int m = blockIdx.y, rank = blockIdx.x, size = (int)gridDim.x, n8 = K >> 3, stride = size * kDigitThreads;
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__(kDigitThreads) digit_rows_kernel(const float* 
     mx = warp_max(mx);
     if (lane == 0) warp_part[warp] = make_float2(ss, mx);
     __syncthreads();
+    asm volatile("barrier.cluster.wait;" ::: "memory");  // every block of the cluster has started
     if (warp == 0) {
         const float2 t = lane < kDigitThreads / 32 ? warp_part[lane] : make_float2(0.0f, 0.0f);
         const float bs = warp_sum(t.x), bm = warp_max(t.y);
