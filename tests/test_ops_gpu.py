@@ -608,6 +608,24 @@ def test_prefill_attention_against_64_bits(cuda, n, h, g, d, shift):
         assert float((got[:, head] - w @ vh).abs().max()) <= bound
 
 
+# two, four and eight rows per thread; a position inside a 64-key tile, at its ends, on the diagonal of a row block
+@pytest.mark.parametrize("n,h,g,d", [(70, 2, 1, 128), (200, 32, 8, 64), (320, 64, 8, 64), (320, 64, 8, 128)])
+@pytest.mark.parametrize("at", [0, 15, 31, 40, 63, 64, 69])
+def test_prefill_attention_causal_for_non_finite_values(cuda, n, h, g, d, at):
+    """Rows before a token do not see it, whatever its key and value hold."""
+    gen = torch.Generator(device="cuda").manual_seed(at)
+    q, k, v = (torch.randn(n, w, d, generator=gen, device="cuda") for w in (h, g, g))
+    want = ops.prefill_causal_attention(q, k, v, n, n, h, g, d).view(n, h, d).clone()
+    for bad in (float("inf"), float("nan")):
+        v2, k2 = v.clone(), k.clone()
+        v2[at] = bad
+        k2[at] = float("nan")
+        for got in (ops.prefill_causal_attention(q, k, v2, n, n, h, g, d), ops.prefill_causal_attention(q, k2, v, n, n, h, g, d)):
+            got = got.view(n, h, d)
+            assert torch.equal(got[:at], want[:at])
+            assert not bool(torch.isfinite(got[at]).any())
+
+
 # whole heads in aligned pieces (one, two or four blocks per row), part of a head rotated, unaligned rows: one value per thread
 @pytest.mark.parametrize("n,h,g,d,half,shift", [(1, 2, 2, 128, 64, 0), (5, 14, 2, 64, 32, 0), (80, 3, 1, 128, 64, 0), (150, 32, 8, 128, 64, 0), (7, 4, 2, 64, 16, 0),
                                                 (9, 4, 2, 64, 32, 1), (3, 2, 1, 12, 6, 0)])

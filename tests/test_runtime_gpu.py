@@ -77,6 +77,29 @@ def test_sliding_window_other_step_forms_and_bf16(cuda):
         dec.close()
 
 
+@pytest.mark.parametrize("window", [1, 20, 70])
+def test_f32_prompt_attention_window_keeps_non_finite_values_out(cuda, window):
+    """fused = 0, one layer: the last row's hidden state does not change when a token before its window turns into NaN (the
+    tile of keys that holds the window's start holds that token too), and does when the window reaches it."""
+    cfg = tiny(rt.FORMAT_RS_I8, False, n_layers=1, max_seq_len=160, sliding_window=window)
+    dec = make(cfg)
+    table = dec.get_tensor(-1, rt.T_EMBEDDING).copy()
+    table[639] = 0x7FC0
+    dec.set_tensor(-1, rt.T_EMBEDDING, table)
+    prompt = np.random.default_rng(window).integers(0, 639, 139)
+    dec.prefill(prompt)
+    want = dec.last_hidden()
+    assert np.isfinite(want).all()
+    poisoned = prompt.copy()
+    poisoned[138 - window] = 639
+    dec.prefill(poisoned)
+    assert np.array_equal(dec.last_hidden(), want)
+    poisoned[139 - window] = 639
+    dec.prefill(poisoned)
+    assert not np.isfinite(dec.last_hidden()).any()
+    dec.close()
+
+
 @pytest.mark.parametrize("kv_bf16", [False, True])
 def test_long_context_fused_step_matches_oracle(cuda, kv_bf16):
     """A cache of 1300 positions x 8 KV heads: the fused batch-1 step plans slices of 128 positions (8 stages of 16, one
