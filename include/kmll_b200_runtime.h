@@ -175,11 +175,17 @@ int kmll_decoder_set_rope_freqs(kmll_decoder_t dec, const float* freqs_host, int
  * (crates/inference/src/model.rs:5319-5352).  One GPU only (a tensor-parallel rank holds a slice of the vocabulary). */
 int kmll_decoder_next_logits(kmll_decoder_t dec, kmll_stream_t stream, float* logits_device);
 /* Kernel launches per decode step; bytes of weights / KV cache resident on this rank; bytes of every device allocation of
- * the decoder (weights + KV cache + scratch: RuntimeMemoryStats, crates/inference/src/model.rs:803-808,5368-5391). */
+ * the decoder (weights + KV cache + scratch: RuntimeMemoryStats, crates/inference/src/model.rs:803-808,5368-5391).  The scratch of
+ * prompts is no decoder's and not in these figures: see kmll_release_scratch. */
 int kmll_decoder_launches_per_step(kmll_decoder_t dec);
 size_t kmll_decoder_weight_bytes(kmll_decoder_t dec);
 size_t kmll_decoder_kv_bytes(kmll_decoder_t dec);
 size_t kmll_decoder_resident_bytes(kmll_decoder_t dec);
+/* kmll_decoder_prefill keeps the scratch of its last call for the next one: at most one idle buffer of at most 2 GiB per GPU, shared
+ * by all decoders of the process, none on a GPU that has less than four times as much memory free.  It is given back by itself
+ * when an allocation of this library finds no memory and with the last decoder; this call gives it back at once, for other users
+ * of the GPU, and returns the bytes.  Safe from any thread, also while prompts run (their buffers are not touched). */
+size_t kmll_release_scratch(void);
 
 /* ---- layered decoders ----------------------------------------------------------------------------------------------
  * A decoder over a list of layer descriptions with bf16 weights: pre-norm layers (x += mixer(norm(x)), x += feed_forward(

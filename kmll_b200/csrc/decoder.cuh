@@ -45,7 +45,15 @@ struct Layer {
 
 enum ShardKind { SHARD_NONE, SHARD_ROWS, SHARD_COLS };
 
+// cudaMalloc; when the GPU is short of memory, the prompt scratch that is kept between calls (runtime.cu) is given back first.
+cudaError_t device_malloc(void** p, size_t bytes);
+void decoders_alive(int change);  // with the last decoder the kept prompt scratch goes, too
+
 struct Decoder {
+    Decoder() { decoders_alive(1); }
+    ~Decoder() { decoders_alive(-1); }
+    Decoder(const Decoder&) = delete;
+    Decoder& operator=(const Decoder&) = delete;
     kmll_decoder_config cfg;
     int device = 0;
     int n_heads_l = 0, n_kv_l = 0, hidden_l = 0, vocab_l = 0;  // per-rank sizes
@@ -91,15 +99,13 @@ struct Decoder {
     bool chain_words = false;      // one GPU, one launch per projection: still hand the vectors over as exchange words (KMLL_CHAIN=words)
     bool prepared_valid = false;   // the prepared buffers match the canonical tensors
     unsigned int* top1_counter = nullptr;
-    void* prompt_scratch = nullptr;  // scratch of the batched prompt path, as large as the longest prompt so far needed
-    size_t prompt_scratch_bytes = 0;
     Layered* lay = nullptr;  // a decoder over a list of layer descriptions (layered.cu); null = kmll's uniform layers
 };
 
 template <typename T>
 inline int dalloc(Decoder* d, T** out, size_t count) {
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T) + 16);
+    cudaError_t e = device_malloc(&p, count * sizeof(T) + 16);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "cudaMalloc(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));
     d->allocs.push_back(p);
     d->resident_bytes += count * sizeof(T);

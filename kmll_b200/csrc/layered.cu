@@ -462,7 +462,7 @@ int ensure_rows(Decoder* d, cudaStream_t s, int n) {
                 if (m.mixer == KMLL_MIXER_GATED_LINEAR) lin = std::max(lin, gated_chunk_scratch_floats(want, m.heads, m.dim, m.vdim, m.delta));
             }
     auto take = [&](void** p, size_t bytes) -> int {
-        cudaError_t er = cudaMalloc(p, bytes + 64);
+        cudaError_t er = device_malloc(p, bytes + 64);
         if (er != cudaSuccess) return fail(KMLL_ERR_CUDA, "prompt scratch (%zu bytes): %s", bytes, cudaGetErrorString(er));
         L->row_allocs.push_back(*p);
         total += bytes;
@@ -485,7 +485,7 @@ int ensure_expanded(Layered* L, cudaStream_t s, size_t bytes) {
     cudaFree(L->expanded);
     L->expanded = nullptr;
     L->expanded_bytes = 0;
-    cudaError_t e = cudaMalloc(&L->expanded, bytes + 64);
+    cudaError_t e = device_malloc(&L->expanded, bytes + 64);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "latent expansion (%zu bytes): %s", bytes, cudaGetErrorString(e));
     L->expanded_bytes = bytes;
     return KMLL_OK;
@@ -844,7 +844,7 @@ int layered_init_random(Decoder* d, uint64_t seed, float std, int tie_embeddings
     const kmll_layered_config& c = L->cfg;
     constexpr size_t kBatch = 1u << 24;
     float* tmp = nullptr;
-    KMLL_CUDA(cudaMalloc((void**)&tmp, kBatch * 4));
+    KMLL_CUDA(device_malloc((void**)&tmp, kBatch * 4));
     uint64_t at = seed * 0x9e3779b97f4a7c15ull;
     auto normal = [&](uint16_t* w, size_t n) -> int {  // (row padding included: the other operand is zero there)
         for (size_t i = 0; i < n; i += kBatch) {
@@ -957,7 +957,7 @@ int kmll_layered_set_rotation(kmll_decoder_t dec, int layer, const double* freqs
     LMixer& y = d->lay->layers[layer].mix[0];
     KMLL_REQUIRE(y.sp.rot_dim > 0 && count == y.sp.rot_dim / 2, "set_rotation: %d frequencies given, %d expected", count, y.sp.rot_dim / 2);
     double* dev = nullptr;
-    KMLL_CUDA(cudaMalloc((void**)&dev, sizeof(double) * count));
+    KMLL_CUDA(device_malloc((void**)&dev, sizeof(double) * count));
     cudaError_t e = cudaMemcpy(dev, freqs_host, sizeof(double) * count, cudaMemcpyHostToDevice);
     int rc = e == cudaSuccess ? rotation_table(nullptr, dev, count, d->cfg.max_seq_len, magnitude, y.table) : fail(KMLL_ERR_CUDA, "set_rotation: %s", cudaGetErrorString(e));
     e = cudaDeviceSynchronize();

@@ -6,6 +6,7 @@
 #include <dlfcn.h>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "decoder.cuh"
@@ -96,6 +97,91 @@ static int tp_allreduce(Decoder* d, cudaStream_t s, float* buf, size_t count) {
     ncclResult_t r = api->AllReduce(buf, buf, count, ncclFloat, ncclSum, d->comm, s);
     if (r != ncclSuccess) return fail(KMLL_ERR_CUDA, "ncclAllReduce: %s", api->GetErrorString ? api->GetErrorString(r) : "error");
     return KMLL_OK;
+}
+
+// ---- prompt scratch kept between calls --------------------------------------------------------------------
+// Allocating and freeing the scratch of a prompt in each call (14 buffers, with the synchronisations inside) took 10 ms of the 13.9 ms
+// of a 200-token prompt of an 8-layer 4096 / 14336 wide decoder (45 ms in some runs); with a buffer at hand it takes 2.6 ms in all.
+// The buffer belongs to no decoder: one idle buffer per GPU is kept, whoever used it last, so what is held does not grow with the
+// number of decoders.  A call has its buffer to itself (of two prompts at once the second allocates its own) and has synchronised its
+// stream before it gives the buffer back.  Not kept are buffers above 2 GiB (more than ~8000 positions at that width) and those of
+// a GPU that has less than four times as much memory free.  Kept memory goes back when an allocation of this library finds
+// no memory, with the last decoder, and by kmll_release_scratch.
+struct PromptScratch {
+    void* p = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+    bool keep = false;
+};
+static std::mutex g_scratch_mutex;
+static std::vector<PromptScratch> g_scratch;  // idle buffers, one per GPU
+static int g_decoders = 0;
+
+static size_t release_scratch() {
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    size_t bytes = 0;
+    for (const PromptScratch& s : g_scratch) {
+        bytes += s.bytes;
+        cudaFree(s.p);
+    }
+    g_scratch.clear();
+    return bytes;
+}
+void decoders_alive(int change) {
+    bool last = false;
+    {
+        std::lock_guard<std::mutex> lock(g_scratch_mutex);
+        g_decoders += change;
+        last = g_decoders == 0;
+    }
+    if (last) release_scratch();
+}
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && release_scratch() > 0) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+static int take_scratch(size_t bytes, PromptScratch* out) {
+    PromptScratch s;
+    KMLL_CUDA(cudaGetDevice(&s.device));
+    {
+        std::lock_guard<std::mutex> lock(g_scratch_mutex);
+        for (size_t i = 0; i < g_scratch.size(); ++i)
+            if (g_scratch[i].device == s.device) {
+                PromptScratch idle = g_scratch[i];
+                g_scratch.erase(g_scratch.begin() + i);
+                if (idle.bytes >= bytes) {
+                    *out = idle;
+                    return KMLL_OK;
+                }
+                cudaFree(idle.p);
+                break;
+            }
+    }
+    cudaError_t e = device_malloc(&s.p, bytes);
+    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "prefill scratch: %s", cudaGetErrorString(e));
+    s.bytes = bytes;
+    size_t left = 0, total = 0;
+    s.keep = bytes <= (size_t)2 << 30 && cudaMemGetInfo(&left, &total) == cudaSuccess && left / 4 >= bytes;
+    *out = s;
+    return KMLL_OK;
+}
+static void give_scratch(PromptScratch s) {
+    if (s.keep) {
+        std::lock_guard<std::mutex> lock(g_scratch_mutex);
+        PromptScratch* idle = nullptr;
+        for (PromptScratch& o : g_scratch)
+            if (o.device == s.device) idle = &o;
+        if (idle == nullptr) {
+            g_scratch.push_back(s);
+            return;
+        }
+        if (idle->bytes < s.bytes) std::swap(*idle, s);
+    }
+    cudaFree(s.p);
 }
 
 // ---- linear dispatch on the decoder's format ------------------------------------------------------
@@ -692,7 +778,7 @@ struct BatchDecoder {
 template <typename T>
 static int balloc(BatchDecoder* b, T** out, size_t count) {
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T) + 16);
+    cudaError_t e = device_malloc(&p, count * sizeof(T) + 16);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "cudaMalloc(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));
     b->allocs.push_back(p);
     *out = static_cast<T*>(p);
@@ -814,7 +900,7 @@ static int setup_exchange(Decoder* d) {
     const size_t off_ready = off_box + box_bytes;  // arrival hints: inbox exchanges, then the local vector (256 each)
     const size_t off_local = off_ready + 2 * 256 * sizeof(unsigned int);  // epoch
     const size_t total = off_local + 256;
-    KMLL_CUDA(cudaMalloc(&d->xc_local, total));
+    KMLL_CUDA(device_malloc(&d->xc_local, total));
     KMLL_CUDA(cudaMemset(d->xc_local, 0, total));
     std::vector<cudaIpcMemHandle_t> handles(tp);
     if (tp > 1) {
@@ -862,35 +948,6 @@ static int setup_exchange(Decoder* d) {
     KMLL_TRY(dalloc(d, &d->xc, 1));
     KMLL_CUDA(cudaMemcpy(d->xc, &h, sizeof(h), cudaMemcpyHostToDevice));
     d->xc_host = h;
-    return KMLL_OK;
-}
-
-// Scratch of a prompt, kept by the decoder: its calls are one after another, and each ends in a stream synchronisation.  Allocating
-// and freeing 14 buffers per call (with the synchronisations inside) took 10 ms of the 13.9 ms of a 200-token prompt of an 8-layer
-// 4096 / 14336 wide decoder (45 ms in some runs); now 2.6 ms in all.
-// Above 2 GiB (more than ~5500 positions at that width, whose prompt takes 20 ms and more) it is allocated for the call and given back.
-static int prefill_scratch(Decoder* d, size_t bytes, unsigned char** out, bool* kept) {
-    constexpr size_t kKeep = (size_t)2 << 30;
-    *kept = bytes <= kKeep;
-    if (*kept && bytes <= d->prompt_scratch_bytes) {
-        *out = static_cast<unsigned char*>(d->prompt_scratch);
-        return KMLL_OK;
-    }
-    if (d->prompt_scratch != nullptr) {
-        cudaFree(d->prompt_scratch);
-        d->resident_bytes -= d->prompt_scratch_bytes;
-        d->prompt_scratch = nullptr;
-        d->prompt_scratch_bytes = 0;
-    }
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "prefill scratch: %s", cudaGetErrorString(e));
-    if (*kept) {
-        d->prompt_scratch = p;
-        d->prompt_scratch_bytes = bytes;
-        d->resident_bytes += bytes;
-    }
-    *out = static_cast<unsigned char*>(p);
     return KMLL_OK;
 }
 
@@ -1006,7 +1063,6 @@ int kmll_decoder_destroy(kmll_decoder_t dec) {
         if (d->xc_peer_base[r]) cudaIpcCloseMemHandle(d->xc_peer_base[r]);
     if (d->xc_local) cudaFree(d->xc_local);
     for (void* p : d->allocs) cudaFree(p);
-    cudaFree(d->prompt_scratch);
     if (d->pinned) cudaFreeHost(d->pinned);
     layered_destroy(d);
     delete d;
@@ -1031,10 +1087,10 @@ int kmll_decoder_init_random(kmll_decoder_t dec, uint64_t seed, float std, int t
         cudaFree(tmp); cudaFree(tmp_bf16); cudaFree(full_w); cudaFree(full_s);
     };
     auto body = [&]() -> int {
-        KMLL_CUDA(cudaMalloc((void**)&tmp, max_elems * sizeof(float)));
-        KMLL_CUDA(cudaMalloc((void**)&tmp_bf16, max_elems * sizeof(uint16_t)));
-        KMLL_CUDA(cudaMalloc((void**)&full_w, max_elems));
-        KMLL_CUDA(cudaMalloc((void**)&full_s, max_elems / 16 + 16 + (size_t)c.vocab_size * 4));
+        KMLL_CUDA(device_malloc((void**)&tmp, max_elems * sizeof(float)));
+        KMLL_CUDA(device_malloc((void**)&tmp_bf16, max_elems * sizeof(uint16_t)));
+        KMLL_CUDA(device_malloc((void**)&full_w, max_elems));
+        KMLL_CUDA(device_malloc((void**)&full_s, max_elems / 16 + 16 + (size_t)c.vocab_size * 4));
         std::vector<uint16_t> ones(c.dim, 0x3f80);  // bf16 1.0
         auto fill_quant = [&](int layer, int tensor, const uint16_t* bf16_source) -> int {
             TensorRef t;
@@ -1109,8 +1165,8 @@ int kmll_decoder_set_tensor(kmll_decoder_t dec, int layer, int tensor, const voi
     size_t sb = 0;
     const size_t wb = qweight_bytes(d->cfg.format, t.full_rows, t.full_cols, &sb);
     uint8_t *fw = nullptr, *fs = nullptr;
-    KMLL_CUDA(cudaMalloc((void**)&fw, wb));
-    cudaError_t e = cudaMalloc((void**)&fs, sb);
+    KMLL_CUDA(device_malloc((void**)&fw, wb));
+    cudaError_t e = device_malloc((void**)&fs, sb);
     if (e != cudaSuccess) { cudaFree(fw); return fail(KMLL_ERR_CUDA, "cudaMalloc: %s", cudaGetErrorString(e)); }
     int rc = KMLL_OK;
     if (cudaMemcpy(fw, values, wb, cudaMemcpyHostToDevice) != cudaSuccess || cudaMemcpy(fs, scales, sb, cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1228,9 +1284,9 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
     const size_t o_x = part(row * c.dim), o_x2 = part(row * c.dim), o_q = part(row * q_len), o_qr = part(row * q_len), o_a = part(row * q_len);
     const size_t o_k = part(row * kv_len), o_v = part(row * kv_len), o_g = part(row * d->hidden_l), o_u = part(row * d->hidden_l), o_act = part(forms ? 0 : row * d->hidden_l);
     const size_t o_tok = part(row), o_ws = part(ws_bytes), o_n = part(forms ? 0 : row * c.dim), o_o = part(forms ? 0 : row * c.dim);
-    unsigned char* base = nullptr;
-    bool kept = false;
-    KMLL_TRY(prefill_scratch(d, scratch_bytes, &base, &kept));
+    PromptScratch scratch;
+    KMLL_TRY(take_scratch(scratch_bytes, &scratch));
+    unsigned char* base = static_cast<unsigned char*>(scratch.p);
     auto at = [&](size_t o) { return reinterpret_cast<float*>(base + o); };
     float *xb = at(o_x), *x2b = at(o_x2), *nb = at(o_n), *ob = at(o_o), *qb = at(o_q), *qrb = at(o_qr), *ab = at(o_a), *kb = at(o_k), *vb = at(o_v),
           *gb = at(o_g), *ub = at(o_u), *actb = at(o_act);
@@ -1306,7 +1362,7 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
     };
     const int rc = body();
     cudaStreamSynchronize(s);
-    if (!kept) cudaFree(base);
+    give_scratch(scratch);
     if (rc != KMLL_OK) return rc;
     d->host_position = n;
     d->have_next = true;
@@ -1542,6 +1598,7 @@ int kmll_decoder_set_rope_freqs(kmll_decoder_t dec, const float* freqs_host, int
     return KMLL_OK;
 }
 
+size_t kmll_release_scratch(void) { return release_scratch(); }
 size_t kmll_decoder_resident_bytes(kmll_decoder_t dec) { return dec ? static_cast<Decoder*>(dec)->resident_bytes : 0; }
 int kmll_decoder_launches_per_step(kmll_decoder_t dec) { return dec ? static_cast<Decoder*>(dec)->launches_per_step : 0; }
 size_t kmll_decoder_weight_bytes(kmll_decoder_t dec) { return dec ? static_cast<Decoder*>(dec)->weight_bytes : 0; }

@@ -89,6 +89,12 @@ def _tensor_shape(cfg: DecoderConfig, tensor: int, sharded: bool):
             T_OUTPUT: (cfg.vocab_size // tp, cfg.dim)}[tensor]
 
 
+def release_scratch() -> int:
+    """Gives back the prompt scratch that is kept between calls (at most one idle buffer of at most 2 GiB per GPU, shared by the
+    decoders of the process); returns its bytes."""
+    return int(load().kmll_release_scratch())
+
+
 class Decoder:
     def __init__(self, cfg: DecoderConfig):
         self.cfg = cfg

@@ -127,7 +127,8 @@ class Session:
 
     def memory_stats(self) -> dict:
         """RuntimeMemoryStats (model.rs:803-808).  Scratch is everything resident that is neither a weight in its
-        canonical layout nor KV cache: activations, workspaces, and the prepared-layout copy of W4-G128 weights."""
+        canonical layout nor KV cache: activations, workspaces, and the prepared-layout copy of W4-G128 weights.  The scratch
+        of prompts, which all decoders share, is not in it (runtime.release_scratch)."""
         w, kv, total = self.dec.weight_bytes, self.dec.kv_bytes, self.dec.resident_bytes
         return {"weights_bytes": w, "kv_cache_bytes": kv, "scratch_bytes": max(0, total - w - kv), "total_resident_bytes": total}
 

@@ -175,6 +175,98 @@ def test_batched_prefill_matches_oracle_and_token_loop(cuda, fmt):
     dec.close()
 
 
+def test_prompt_scratch_is_no_decoders_and_is_given_back(cuda):
+    """Growing and shorter prompts in shared scratch give what they give in a fresh decoder; byte counts stay, one buffer serves two
+    decoders, and nothing is held once it is released."""
+    cfg = tiny(rt.FORMAT_W4G128, hidden_dim=8192, max_seq_len=600)
+    rng = np.random.default_rng(8)
+    prompts = [rng.integers(0, cfg.vocab_size, n) for n in (40, 600, 7, 300, 1)]
+    want = []
+    for p in prompts:
+        dec = make(cfg)
+        rt.release_scratch()
+        dec.prefill(p)
+        want.append(dec.last_hidden())
+        dec.close()
+    rt.release_scratch()
+    decs = [make(cfg), make(cfg)]
+    resident = decs[0].resident_bytes
+    free = torch.cuda.mem_get_info()[0]
+    for dec in decs:
+        for p, w in zip(prompts, want):
+            dec.prefill(p)
+            assert np.array_equal(dec.last_hidden(), w)
+        assert dec.resident_bytes == resident
+    held = free - torch.cuda.mem_get_info()[0]
+    rows = 600 * 4 * (2 * 256 + 3 * 256 + 2 * 128 + 2 * 8192)  # of the longest prompt
+    assert rows <= held <= 1.5 * rows + (32 << 20)  # planes and partial tiles of the linears beside them; once, not twice
+    assert rt.release_scratch() >= rows and rt.release_scratch() == 0
+    assert torch.cuda.mem_get_info()[0] == free
+    decs[0].prefill(prompts[1])
+    assert np.array_equal(decs[0].last_hidden(), want[1])
+    for dec in decs:
+        dec.close()
+
+
+def test_prompt_scratch_above_its_bound_is_not_kept(cuda):
+    cfg = tiny(rt.FORMAT_RS_I8, n_layers=1, dim=64, n_heads=1, n_kv_heads=1, hidden_dim=16384, max_seq_len=14000)
+    dec = make(cfg)
+    prompt = np.random.default_rng(4).integers(0, cfg.vocab_size, 14000)  # 14000 x (2 x 16384 x 4 + 16384 x 4) bytes and more
+    dec.prefill(prompt)
+    rt.release_scratch()
+    free = torch.cuda.mem_get_info()[0]
+    dec.prefill(prompt)
+    assert torch.cuda.mem_get_info()[0] == free and rt.release_scratch() == 0
+    assert np.isfinite(dec.last_hidden()).all()
+    dec.close()
+
+
+def test_kept_prompt_scratch_makes_room_for_a_batch(cuda):
+    """A batch that fits the GPU only without the kept scratch can be created."""
+    cfg = tiny(rt.FORMAT_RS_I8, n_layers=1, dim=64, n_heads=1, n_kv_heads=1, hidden_dim=16384, max_seq_len=8000)
+    dec = make(cfg)
+    dec.prefill(np.arange(8000) % cfg.vocab_size)
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    kept = rt.release_scratch()
+    assert kept > 1 << 30
+    dec.prefill(np.arange(8000) % cfg.vocab_size)
+    hold = torch.empty(free - (kept >> 2), dtype=torch.uint8, device="cuda")
+    other = rt.DecoderConfig(**{**cfg.__dict__, "max_seq_len": kept // 2 // (2 * 64 * 4)})  # its caches: half of the kept scratch
+    try:
+        second = make(other)
+        assert rt.release_scratch() == 0
+        second.close()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    dec.close()
+
+
+def test_prompts_of_two_threads_have_scratch_of_their_own(cuda):
+    from concurrent.futures import ThreadPoolExecutor
+
+    cfg = tiny(rt.FORMAT_W4G128, hidden_dim=2048, max_seq_len=300)
+    rng = np.random.default_rng(12)
+    prompts = [rng.integers(0, cfg.vocab_size, n) for n in (300, 45, 120, 9) * 6]
+
+    def all_of(dec, order):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got = {}
+            for i in order:
+                dec.prefill(prompts[i])
+                got[i] = dec.last_hidden()
+            return got
+
+    decs = [make(cfg) for _ in range(3)]
+    want = all_of(decs[0], range(len(prompts)))
+    with ThreadPoolExecutor(3) as pool:
+        for got in pool.map(all_of, decs, [range(24), range(23, -1, -1), range(24)]):
+            assert all(np.array_equal(got[i], want[i]) for i in range(24))
+    for dec in decs:
+        dec.close()
+
+
 def test_fused_and_unfused_paths_agree(cuda):
     prompt = np.arange(1, 8)
     outs = []
