@@ -819,11 +819,12 @@ int w4_prepare(cudaStream_t stream, const uint8_t* pa, const uint16_t* sa, const
     const size_t words = w4_prepared_bytes(rows, cols, pair) / 4;
     if (words == 0) return fail(KMLL_ERR_SHAPE, "w4g128_prepare: rows=%d cols=%d (cols must be a positive multiple of 128)", rows, cols);
     if ((reinterpret_cast<uintptr_t>(out) & 15u) != 0) return fail(KMLL_ERR_UNSUPPORTED, "w4g128_prepare: the output must be 16-byte aligned");
-    const size_t records = words / (kCRecBytes / 4), blocks = (records + 7) / 8;
+    // a block per record as long as there are no more than eight for a multiprocessor, else eight warps to a block
+    const size_t records = words / (kCRecBytes / 4), warps = records <= 148 * 8 ? 1 : 8, blocks = (records + warps - 1) / warps;
     if (blocks > 0x7fffffffull) return fail(KMLL_ERR_CAPACITY, "w4g128_prepare: matrix too large");
     const bool aligned = aligned16(pa) && (pb == nullptr || aligned16(pb));
     auto kern = aligned ? w4_prepare_kernel<true> : w4_prepare_kernel<false>;
-    kern<<<(unsigned)blocks, 256, 0, stream>>>(pa, sa, pb, sb, rows, cols, pair, records, static_cast<uint8_t*>(out));
+    kern<<<(unsigned)blocks, (unsigned)(32 * warps), 0, stream>>>(pa, sa, pb, sb, rows, cols, pair, records, static_cast<uint8_t*>(out));
     return check_launch("w4g128_prepare");
 }
 

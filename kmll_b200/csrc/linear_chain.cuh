@@ -644,21 +644,30 @@ __global__ void __launch_bounds__(kSBlock, 1) linear_chain_kernel(const __grid_c
 // ---- canonical W4-G128 -> prepared records --------------------------------------------------------------------
 // pair != 0: the A rows of unit u are rows 16u.. of matrix a (gate) and the B rows the same rows of matrix b (up); else A rows =
 // 32u.., B rows = 32u + 16.. of matrix a.  Bound by HBM: one warp per record; lane (g, t) reads 16 bytes (32 columns) of the four rows
-// g, g + 8 of both halves and writes four 16-byte words, so a warp's stores are 512 contiguous bytes.  14336 x 4096: 49 us (one
-// thread per output word, eight byte loads each) -> 19 us = 3.2 TB/s.  ALIGNED: the packed rows start on 16 bytes.
+// g, g + 8 of both halves and writes four 16-byte words, so a warp's stores are 512 contiguous bytes.  14336 x 4096 in a row of calls, the
+// matrix in L2: 47 us (one thread per output word, eight byte loads each) -> 8.4 us.  Few records are bound by the latency of one, so all its
+// loads are issued together and its place is found in 32 bits: 896 x 896 2.7 -> 2.3 us.  ALIGNED: the packed rows start on 16 bytes.
 template <bool ALIGNED>
 __global__ void __launch_bounds__(256) w4_prepare_kernel(const uint8_t* __restrict__ pa, const uint16_t* __restrict__ sa, const uint8_t* __restrict__ pb,
                                                          const uint16_t* __restrict__ sb, int rows, int cols, int pair, size_t records,
                                                          uint8_t* __restrict__ out) {
-    const size_t rec = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const size_t rec = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (rec >= records) return;
     const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
     const int ngroups = cols >> 7;
-    const int unit = (int)(rec / ngroups), grp = (int)(rec - (size_t)unit * ngroups);
+    const int unit = (int)((uint32_t)rec / (uint32_t)ngroups), grp = (int)((uint32_t)rec - (uint32_t)unit * (uint32_t)ngroups);  // (2^32 records: 9 TB)
     const int rowA0 = pair ? unit * 16 : unit * 32, rowB0 = pair ? unit * 16 : unit * 32 + 16;
     const uint8_t* pB = pair ? pb : pa;
     const uint16_t* sB = pair ? sb : sa;
     const size_t rowbytes = (size_t)cols >> 1;
+    uint32_t row_scales = 0u;
+    if (lane < 16) {  // (g, which): g = lane / 2; which = 0: A rows g, g + 8; 1: B rows g, g + 8
+        const int r0 = ((lane & 1) ? rowB0 : rowA0) + (lane >> 1), r1 = r0 + 8;
+        const uint16_t* s = (lane & 1) ? sB : sa;
+        const uint32_t lo = r0 < rows ? s[(size_t)r0 * ngroups + grp] : 0u;
+        const uint32_t hi = r1 < rows ? s[(size_t)r1 * ngroups + grp] : 0u;
+        row_scales = lo | (hi << 16);
+    }
     uint32_t n[2][2][4];  // [A / B][row g / g + 8][word of 8 columns]; rows past the end: q = 0
 #pragma unroll
     for (int m = 0; m < 2; ++m)
@@ -692,13 +701,7 @@ __global__ void __launch_bounds__(256) w4_prepare_kernel(const uint8_t* __restri
         }
         reinterpret_cast<uint4*>(to)[i * 32 + lane] = make_uint4(o[0], o[1], o[2], o[3]);
     }
-    if (lane < 16) {  // (g, which): g = lane / 2; which = 0: A rows g, g + 8; 1: B rows g, g + 8
-        const int r0 = ((lane & 1) ? rowB0 : rowA0) + (lane >> 1), r1 = r0 + 8;
-        const uint16_t* s = (lane & 1) ? sB : sa;
-        const uint32_t lo = r0 < rows ? s[(size_t)r0 * ngroups + grp] : 0u;
-        const uint32_t hi = r1 < rows ? s[(size_t)r1 * ngroups + grp] : 0u;
-        reinterpret_cast<uint32_t*>(to)[512 + lane] = lo | (hi << 16);
-    }
+    if (lane < 16) reinterpret_cast<uint32_t*>(to)[512 + lane] = row_scales;
 }
 
 }  // namespace kmll

@@ -19,17 +19,18 @@ __device__ inline uint32_t round_quotient(float v, float scale, float inv, float
     return (uint32_t)(__float_as_int(fminf(fmaxf(m, kMagic - limit), kMagic + limit)) - __float_as_int(kMagic));
 }
 
-// One block per row.  VEC (rows of whole 8-column pieces, aligned): bound by HBM, 16-byte loads; the row stays in registers between
-// the maximum and the rounding (up to 32 columns per thread and 16384 per block, further ones are read again).  14336 x 4096: 68 ->
-// 51 us = 3.4 TB/s; what is left is the block reduction between the two halves of a row.
-template <bool VEC>
+// One block per row.  kHold > 0 (rows of whole 8-column pieces, aligned): bound by HBM, 16-byte loads; a thread keeps up to kHold pieces
+// between the maximum and the rounding (with 4: 16384 columns per block, further ones are read again).  14336 x 4096: 65 -> 49 us =
+// 3.6 TB/s; what is left is the block reduction between the two halves of a row.  Small matrices are bound by latency, which four
+// pieces one after another in a thread add to: 896 x 896 5.0 us with 4 pieces, 2.8 with one (value by value: 3.5).  kHold = 0: value
+// by value.
+template <int kHold>
 __global__ void __launch_bounds__(512, 2) quantize_rs_i8_kernel(const uint16_t* __restrict__ w, int cols,
                                                              int8_t* __restrict__ values, float* __restrict__ scales) {
     __shared__ float scratch[40];
     const size_t base = (size_t)blockIdx.x * cols;
     float mx = 0.0f;
-    if constexpr (VEC) {
-        constexpr int kHold = 4;
+    if constexpr (kHold > 0) {
         const uint4* src = reinterpret_cast<const uint4*>(w + base);
         const int n8 = cols >> 3;
         uint4 held[kHold];
@@ -45,7 +46,8 @@ __global__ void __launch_bounds__(512, 2) quantize_rs_i8_kernel(const uint16_t* 
         }
 #pragma unroll
         for (int h = 0; h < kHold; ++h) look(held[h]);
-        for (int c = threadIdx.x + kHold * blockDim.x; c < n8; c += blockDim.x) look(__ldg(src + c));
+        if (kHold > 1)
+            for (int c = threadIdx.x + kHold * blockDim.x; c < n8; c += blockDim.x) look(__ldg(src + c));
         mx = block_max(mx, scratch);
         const float scale = (mx == 0.0f) ? 1.0f : mx / 127.0f, inv = 1.0f / scale;
         if (threadIdx.x == 0) scales[blockIdx.x] = scale;
@@ -65,7 +67,8 @@ __global__ void __launch_bounds__(512, 2) quantize_rs_i8_kernel(const uint16_t* 
             const int c = threadIdx.x + h * blockDim.x;
             if (c < n8) put(held[h], c);
         }
-        for (int c = threadIdx.x + kHold * blockDim.x; c < n8; c += blockDim.x) put(__ldg(src + c), c);
+        if (kHold > 1)
+            for (int c = threadIdx.x + kHold * blockDim.x; c < n8; c += blockDim.x) put(__ldg(src + c), c);
     } else {
         for (int c = threadIdx.x; c < cols; c += 256) mx = fmaxf(mx, fabsf(bf16_bits_to_f32(w[base + c])));
         mx = block_max(mx, scratch);
@@ -78,17 +81,17 @@ __global__ void __launch_bounds__(512, 2) quantize_rs_i8_kernel(const uint16_t* 
     }
 }
 
-// Dequantizers: bound by the f32 stores; a thread turns four values into 16 bytes, kDequantSteps times, so that several loads are in
+// Dequantizers: bound by the f32 stores; a thread turns four values into 16 bytes, kSteps times, so that several loads are in
 // flight and a warp's stores are contiguous (14336 x 4096: RS-I8 167 -> 49 us = 6.0 TB/s, W4 166 -> 47 us = 5.6 TB/s; one value per thread
 // was bound by address arithmetic, a 64-bit division per value in the RS-I8 form).  RS-I8 rows that are not a multiple of four columns go one value per thread.
-constexpr int kDequantSteps = 4;
+template <int kSteps>
 __global__ void __launch_bounds__(256) dequant_rs_i8_quads_kernel(const uint32_t* __restrict__ values, const float* __restrict__ scales, uint32_t quads,
                                                                   uint32_t quads_per_row, float4* __restrict__ out) {
-    const uint32_t first = blockIdx.x * (256u * kDequantSteps) + threadIdx.x;
-    uint32_t v[kDequantSteps];
-    float s[kDequantSteps];
+    const uint32_t first = blockIdx.x * (256u * kSteps) + threadIdx.x;
+    uint32_t v[kSteps];
+    float s[kSteps];
 #pragma unroll
-    for (int j = 0; j < kDequantSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         const uint32_t i = first + 256u * j;
         if (i < quads) {
             v[j] = __ldg(values + i);
@@ -96,7 +99,7 @@ __global__ void __launch_bounds__(256) dequant_rs_i8_quads_kernel(const uint32_t
         }
     }
 #pragma unroll
-    for (int j = 0; j < kDequantSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         const uint32_t i = first + 256u * j;
         if (i < quads)
             out[i] = make_float4((float)(int8_t)v[j] * s[j], (float)(int8_t)(v[j] >> 8) * s[j], (float)(int8_t)(v[j] >> 16) * s[j], (float)(int8_t)(v[j] >> 24) * s[j]);
@@ -110,21 +113,24 @@ __global__ void dequant_rs_i8_kernel(const int8_t* __restrict__ values, const fl
     out[i] = (float)values[i] * scales[i / cols];
 }
 
-// Eight lanes per 128-column group, 16 consecutive columns (64 bytes in, 8 bytes out) per lane: four 16-byte loads in flight per lane
-// and three shuffles per group.  14336 x 4096: 76 us (one warp per group, one load per lane, IEEE divisions) -> 46 us = 5.7 TB/s.
+// kPer consecutive columns of a 128-column group per lane.  16 (eight lanes, 64 bytes in, 8 bytes out): four 16-byte loads in flight per
+// lane and three shuffles per group; 14336 x 4096: 74 us (one warp per group, one load per lane, IEEE divisions) -> 44 us = 6.0 TB/s.
+// 4 (a warp): a quarter of the work one after another, for matrices that do not fill the chip (896 x 896: 3.1 us with 16, 2.5 with 4).
+template <int kPer>
 __global__ void __launch_bounds__(256) quantize_w4_kernel(const float* __restrict__ w, size_t n_groups,
                                                           uint8_t* __restrict__ packed, uint16_t* __restrict__ gscales) {
-    const int part = threadIdx.x & 7;
-    const size_t grp = (size_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+    constexpr int kLanes = 128 / kPer;
+    const int part = threadIdx.x & (kLanes - 1);
+    const size_t grp = (size_t)blockIdx.x * (256 / kLanes) + threadIdx.x / kLanes;
     const bool live = grp < n_groups;
-    float4 v[4];
+    float4 v[kPer / 4];
     float mx = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = live ? reinterpret_cast<const float4*>(w + grp * 128 + part * 16)[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int j = 0; j < kPer / 4; ++j) v[j] = live ? reinterpret_cast<const float4*>(w + grp * 128 + part * kPer)[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+    for (int j = 0; j < kPer / 4; ++j) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
 #pragma unroll
-    for (int off = 1; off < 8; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    for (int off = 1; off < kLanes; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     if (!live) return;
     const float scale_f32 = (mx == 0.0f) ? 1.0f : mx / 7.0f;
     __half sh = __float2half_rn(scale_f32);
@@ -137,26 +143,29 @@ __global__ void __launch_bounds__(256) quantize_w4_kernel(const float* __restric
     const float scale = __half2float(sh), inv = 1.0f / scale;
     uint32_t o[2] = {0u, 0u};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < kPer / 4; ++j) {
         const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) o[j >> 1] |= (round_quotient(e[i], scale, inv, 7.0f) + 8u) << (16 * (j & 1) + 4 * i);
     }
+    uint8_t* to = packed + grp * 64 + part * (kPer / 2);
     if ((reinterpret_cast<uintptr_t>(packed) & 7u) == 0) {
-        reinterpret_cast<uint2*>(packed + grp * 64)[part] = make_uint2(o[0], o[1]);
+        if (kPer == 16) *reinterpret_cast<uint2*>(to) = make_uint2(o[0], o[1]);
+        else *reinterpret_cast<uint16_t*>(to) = (uint16_t)o[0];
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) packed[grp * 64 + part * 8 + i] = (uint8_t)(o[i >> 2] >> (8 * (i & 3)));
+        for (int i = 0; i < kPer / 2; ++i) to[i] = (uint8_t)(o[i >> 2] >> (8 * (i & 3)));
     }
 }
 
+template <int kSteps>
 __global__ void __launch_bounds__(256) dequant_w4_quads_kernel(const uint16_t* __restrict__ packed, const uint16_t* __restrict__ gscales, size_t quads,
                                                                float4* __restrict__ out) {
-    const size_t first = (size_t)blockIdx.x * (256 * kDequantSteps) + threadIdx.x;
-    uint32_t v[kDequantSteps];
-    float s[kDequantSteps];
+    const size_t first = (size_t)blockIdx.x * (256 * kSteps) + threadIdx.x;
+    uint32_t v[kSteps];
+    float s[kSteps];
 #pragma unroll
-    for (int j = 0; j < kDequantSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         const size_t i = first + 256 * j;
         if (i < quads) {
             v[j] = __ldg(packed + i);
@@ -164,7 +173,7 @@ __global__ void __launch_bounds__(256) dequant_w4_quads_kernel(const uint16_t* _
         }
     }
 #pragma unroll
-    for (int j = 0; j < kDequantSteps; ++j) {
+    for (int j = 0; j < kSteps; ++j) {
         const size_t i = first + 256 * j;
         if (i < quads)
             out[i] = make_float4((float)((int)(v[j] & 15u) - 8) * s[j], (float)((int)((v[j] >> 4) & 15u) - 8) * s[j], (float)((int)((v[j] >> 8) & 15u) - 8) * s[j],
@@ -218,15 +227,26 @@ int widen_bf16(cudaStream_t stream, const uint16_t* src, size_t n, float* dst) {
 
 using namespace kmll;
 
+// One step per thread while that leaves room on the multiprocessors (1024 threads each), else four (128 x 896: 2.0 us with four, 1.6 with one)
+template <typename K, typename... A>
+static void launch_quads(kmll_stream_t s, size_t quads, K one, K four, A... args) {
+    const int steps = quads <= 148 * 1024 ? 1 : 4;
+    (steps == 1 ? one : four)<<<(unsigned)((quads + 256 * steps - 1) / (256 * steps)), 256, 0, as_stream(s)>>>(args...);
+}
+
 extern "C" {
 
 int kmll_quantize_rs_i8(kmll_stream_t s, const uint16_t* w, int rows, int cols, int8_t* values, float* scales) {
     KMLL_REQUIRE_PTR(w); KMLL_REQUIRE_PTR(values); KMLL_REQUIRE_PTR(scales);
     KMLL_REQUIRE(rows > 0 && cols > 0, "quantize_rs_i8: shape [%d, %d] must be positive", rows, cols);
     const bool vec = cols % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (reinterpret_cast<uintptr_t>(values) & 7u) == 0;
-    const int wanted = (cols / 32 + 31) / 32 * 32, threads = wanted > 512 ? 512 : wanted < 32 ? 32 : wanted;  // four 16-byte pieces per thread
-    if (vec) quantize_rs_i8_kernel<true><<<rows, threads, 0, as_stream(s)>>>(w, cols, values, scales);
-    else quantize_rs_i8_kernel<false><<<rows, 256, 0, as_stream(s)>>>(w, cols, values, scales);
+    // One piece per thread while the rows' threads are no more than two rounds of the chip at 1024 per multiprocessor (2000 x 1024, 1.7
+    // rounds: 5.2 us with four pieces, 3.4 with one).
+    auto whole_warps = [](int n) { n = (n + 31) / 32 * 32; return n > 512 ? 512 : n; };
+    const int one = whole_warps((cols + 7) / 8), four = whole_warps((cols + 31) / 32);
+    if (!vec) quantize_rs_i8_kernel<0><<<rows, 256, 0, as_stream(s)>>>(w, cols, values, scales);
+    else if (one * 8 >= cols && (size_t)rows * one <= 2 * 148 * 1024) quantize_rs_i8_kernel<1><<<rows, one, 0, as_stream(s)>>>(w, cols, values, scales);
+    else quantize_rs_i8_kernel<4><<<rows, four, 0, as_stream(s)>>>(w, cols, values, scales);
     return check_launch("quantize_rs_i8");
 }
 int kmll_dequant_rs_i8(kmll_stream_t s, const int8_t* values, const float* scales, int rows, int cols, float* out) {
@@ -234,8 +254,8 @@ int kmll_dequant_rs_i8(kmll_stream_t s, const int8_t* values, const float* scale
     KMLL_REQUIRE(rows > 0 && cols > 0, "dequant_rs_i8: shape [%d, %d] must be positive", rows, cols);
     const size_t n = (size_t)rows * cols;
     if (cols % 4 == 0 && n / 4 < 0xfffffc00ull && (reinterpret_cast<uintptr_t>(values) & 3u) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0)
-        dequant_rs_i8_quads_kernel<<<(unsigned)((n / 4 + 256 * kDequantSteps - 1) / (256 * kDequantSteps)), 256, 0, as_stream(s)>>>(
-            reinterpret_cast<const uint32_t*>(values), scales, (uint32_t)(n / 4), (uint32_t)(cols / 4), reinterpret_cast<float4*>(out));
+        launch_quads(s, n / 4, dequant_rs_i8_quads_kernel<1>, dequant_rs_i8_quads_kernel<4>, reinterpret_cast<const uint32_t*>(values), scales, (uint32_t)(n / 4),
+                     (uint32_t)(cols / 4), reinterpret_cast<float4*>(out));
     else
         dequant_rs_i8_kernel<<<(unsigned)((n + 255) / 256), 256, 0, as_stream(s)>>>(values, scales, rows, cols, out);
     return check_launch("dequant_rs_i8");
@@ -245,7 +265,9 @@ int kmll_quantize_w4g128(kmll_stream_t s, const float* w, int rows, int cols, ui
     KMLL_REQUIRE(rows > 0 && cols > 0 && cols % 128 == 0, "quantize_w4g128: cols %d must be a positive multiple of 128", cols);
     KMLL_REQUIRE((reinterpret_cast<uintptr_t>(w) & 15u) == 0, "quantize_w4g128: source must be 16-byte aligned");
     const size_t n_groups = (size_t)rows * (cols / 128);
-    quantize_w4_kernel<<<(unsigned)((n_groups + 31) / 32), 256, 0, as_stream(s)>>>(w, n_groups, packed, gscales);
+    // a warp per group as long as all of them run at once (64 warps per multiprocessor; 16000 groups: 3.9 us either way)
+    if (n_groups <= 148 * 64) quantize_w4_kernel<4><<<(unsigned)((n_groups + 7) / 8), 256, 0, as_stream(s)>>>(w, n_groups, packed, gscales);
+    else quantize_w4_kernel<16><<<(unsigned)((n_groups + 31) / 32), 256, 0, as_stream(s)>>>(w, n_groups, packed, gscales);
     return check_launch("quantize_w4g128");
 }
 int kmll_dequant_w4g128(kmll_stream_t s, const uint8_t* packed, const uint16_t* gscales, int rows, int cols, float* out) {
@@ -253,8 +275,8 @@ int kmll_dequant_w4g128(kmll_stream_t s, const uint8_t* packed, const uint16_t* 
     KMLL_REQUIRE(rows > 0 && cols > 0 && cols % 128 == 0, "dequant_w4g128: cols %d must be a positive multiple of 128", cols);
     const size_t n = (size_t)rows * cols;
     if ((reinterpret_cast<uintptr_t>(packed) & 1u) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0)
-        dequant_w4_quads_kernel<<<(unsigned)((n / 4 + 256 * kDequantSteps - 1) / (256 * kDequantSteps)), 256, 0, as_stream(s)>>>(
-            reinterpret_cast<const uint16_t*>(packed), gscales, n / 4, reinterpret_cast<float4*>(out));
+        launch_quads(s, n / 4, dequant_w4_quads_kernel<1>, dequant_w4_quads_kernel<4>, reinterpret_cast<const uint16_t*>(packed), gscales, n / 4,
+                     reinterpret_cast<float4*>(out));
     else
         dequant_w4_kernel<<<(unsigned)((n + 255) / 256), 256, 0, as_stream(s)>>>(packed, gscales, n, out);
     return check_launch("dequant_w4g128");

@@ -10,7 +10,7 @@ import torch
 
 import oracle
 from kmll_b200 import ops
-from kmll_b200.lib import KmllError
+from kmll_b200.lib import KmllError, check, load
 
 pytestmark = pytest.mark.gpu
 F = np.float32
@@ -103,6 +103,44 @@ def test_quantize_rs_i8_ties_and_limits(cuda, rows, cols):
         assert np.array_equal(host(m.values), q)
         assert np.array_equal(host(m.scales).view(np.uint32), sc.view(np.uint32))
         assert np.array_equal(host(m.dequantize()).view(np.uint32), oracle.rs_i8_dequant(q, sc).view(np.uint32))
+
+
+# either side of the lines between a small matrix's form and a large one's: threads per row (RS-I8), lanes per group (W4), steps per thread
+# (dequantizers); a row of one piece more than a block's threads
+@pytest.mark.parametrize("rows,cols", [(9472, 256), (9473, 256), (2, 4096), (2, 4104), (2368, 256), (2369, 256)])
+def test_quantize_rs_i8_of_either_size(cuda, rows, cols):
+    rng = np.random.default_rng(rows + cols)
+    w = rng.integers(-254, 255, (rows, cols)).astype(F) * F(0.5)  # with a maximum of 127: ties
+    w[:, 3] = F(127.0)
+    w *= np.exp2(rng.integers(-20, 20, rows)).astype(F)[:, None]
+    wb = oracle.bf16_from_f32(w)
+    q, sc = oracle.rs_i8_quantize(wb)
+    m = ops.DeviceRowwiseScaledI8Matrix.from_bf16_rows_symmetric(torch.from_numpy(wb.view(np.int16)).view(torch.bfloat16).view(rows, cols).cuda())
+    assert np.array_equal(host(m.values), q)
+    assert np.array_equal(host(m.scales).view(np.uint32), sc.view(np.uint32))
+    assert np.array_equal(host(m.dequantize()).view(np.uint32), oracle.rs_i8_dequant(q, sc).view(np.uint32))
+
+
+@pytest.mark.parametrize("rows", [4736, 4737, 9472, 9473])
+def test_quantize_w4_of_either_size(cuda, rows):
+    rng = np.random.default_rng(rows)
+    w = rng.integers(-14, 15, (rows, 128)).astype(F) * F(0.5)  # with a maximum of 7: ties
+    w[:, 5] = F(7.0)
+    w *= np.exp2(np.linspace(-30, 12, rows)).astype(F)[:, None]
+    w[rows // 5:rows // 2] *= F(1.0007)
+    packed, gs = oracle.w4_quantize(w)
+    source = dev(w)
+    for shift in (0, 1):  # packed bytes that are not 8-byte aligned
+        m = ops.DeviceW4G128Matrix.from_f32_rows(source)
+        if shift:
+            room = torch.empty(rows * 64 + 1, dtype=torch.uint8, device="cuda")
+            check(load().kmll_quantize_w4g128(torch.cuda.current_stream().cuda_stream, source.data_ptr(), rows, 128, room.data_ptr() + 1, m.gscales.data_ptr()))
+            got = host(room[1:]).reshape(packed.shape)
+        else:
+            got = host(m.packed)
+            assert np.array_equal(host(m.dequantize()).view(np.uint32), oracle.w4_dequant(packed, gs).view(np.uint32))
+        assert np.array_equal(got, packed)
+        assert np.array_equal(host(m.gscales.view(torch.int16)).view(np.uint16), gs)
 
 
 def test_quantize_w4_ties_and_limits(cuda):

@@ -59,6 +59,15 @@ def prepare_ref(packed_a, gs_a, rows, cols, packed_b=None, gs_b=None):
     return out.reshape(-1)
 
 
+@pytest.mark.parametrize("rows,cols", [(37888, 128), (37889, 128), (6000, 896)])
+def test_prepare_on_either_side_of_a_block_per_record(cuda, rows, cols):
+    rng = np.random.default_rng(rows)
+    packed = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8)
+    gs = rng.integers(1, 0x7000, (rows, cols // 128), dtype=np.uint16)
+    w = ops.DeviceW4G128Matrix(dev(packed), dev(gs.view(np.int16)).view(torch.float16), rows, cols)
+    assert np.array_equal(host(ops.DeviceW4PMatrix.from_canonical(w).prepared), prepare_ref(packed, gs, rows, cols))
+
+
 @pytest.mark.parametrize("rows,cols", [(64, 256), (17, 128), (96, 384)])
 def test_prepare_matches_its_definition(cuda, rows, cols):
     rng = np.random.default_rng(rows + cols)
