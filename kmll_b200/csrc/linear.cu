@@ -1039,11 +1039,6 @@ static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, const fl
     float* partial = reinterpret_cast<float*>(ws + big.off_partial);
     unsigned int* counters = reinterpret_cast<unsigned int*>(ws + big.off_counters);
     const int permute = w4 ? 1 : 0;
-    int cluster = 1;  // blocks per row: one run of eight columns per thread
-    while (cluster < 8 && cluster * kDigitThreads * 8 < K) cluster *= 2;
-    cudaError_t e = launch_cluster(digit_rows_kernel, dim3(cluster, M), cluster, dim3(kDigitThreads), 0, stream, true, x, up, ldx, K, M, norm_w, eps, digits, inv, counters,
-                                   16384, permute);
-    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "digit_rows: %s", cudaGetErrorString(e));
     const int nb = M <= 16 ? 16 : 32;
     const int gp = (w4 && nb == 16 && K >= 256) ? 2 : 1;  // groups per pipeline item (SmallShape)
     const size_t smem = w4 ? (nb == 32 ? SmallShape<32, 1>::kSmemBytes : gp == 2 ? SmallShape<16, 2>::kSmemBytes : SmallShape<16, 1>::kSmemBytes)
@@ -1104,6 +1099,11 @@ static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, const fl
 #ifdef KMLL_ROLE_PROFILE
     { const char* pv = std::getenv("KMLL_ROLE_PROF"); sp.prof = pv ? reinterpret_cast<unsigned long long*>(strtoull(pv, nullptr, 0)) : nullptr; }
 #endif
+    int cluster = 1;  // blocks per row: one run of eight columns per thread
+    while (cluster < 8 && cluster * kDigitThreads * 8 < K) cluster *= 2;
+    cudaError_t e = launch_cluster(digit_rows_kernel, dim3(cluster, M), cluster, dim3(kDigitThreads), 0, stream, true, x, up, ldx, K, M, norm_w, eps, digits, inv, counters,
+                                   best > 1 ? tiles : 0, permute);
+    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "digit_rows: %s", cudaGetErrorString(e));
     const int grid = sp.units < 148 ? sp.units : 148;
     if (!w4) {
         if (nb == 16) {

@@ -73,7 +73,8 @@ struct SmallParams {
 // A cluster of 1 to 8 blocks per row of x: optional RMSNorm (kmll's order x * inv * w) or SiLU(x) * up, power-of-two scale, four
 // balanced byte digits.  digits = [4][M][K] signed bytes; with `permute` (W4-G128) position p of every run of eight columns holds column
 // {0,2,4,6,1,3,5,7}[p], the order in which the weight expansion lays out the nibbles of a 32-bit word; RS-I8 weights are
-// used as they lie, so their digits keep the natural order.  The first block also clears the split-K counters in use.
+// used as they lie, so their digits keep the natural order.  The first block also clears the split-K counters in use
+// (at most 296; clearing all 16384 of the workspace took a microsecond of every call, 14336 x 4096 at 8 rows 17.0 -> 16.0 us).
 // Bound by latency (load -> row statistics -> digits): one block per row put 16 rows' digits, and for the down projection their
 // exponentials, on 16 multiprocessors.  A thread now has one run of eight columns (up to 16384 columns; longer rows are read twice),
 // sum and maximum go through one block reduction and one exchange over distributed shared memory.  A lockstep

@@ -131,6 +131,26 @@ def test_gemm_without_workspace_still_works(cuda):
     assert float(np.max(np.abs(host(out) - ref))) <= 1e-4 * np.sqrt(k)
 
 
+# K cut into pieces and not; a call's own counters are clear whatever the workspace held
+@pytest.mark.parametrize("fmt", ["w4", "i8"])
+@pytest.mark.parametrize("m,n,k", [(5, 130, 4096), (16, 3000, 2048), (32, 128, 16512), (8, 40000, 256), (48, 300, 8192)])
+def test_workspace_contents_do_not_matter(cuda, fmt, m, n, k):
+    rng = np.random.default_rng(m + n)
+    w = (w4_weight if fmt == "w4" else i8_weight)(rng, n, k)[3]
+    x = dev(rng.normal(0, 1, (m, k)).astype(F))
+    ws = ops.linear_batched_workspace(m, k)
+    want = None
+    for fill in (0, 1, 0xff, 3):
+        ws.fill_(fill)
+        got = host(ops.linear_batched(x, w, m, k, n, workspace=ws))
+        want = got if want is None else want
+        assert np.array_equal(got, want)
+        again = host(ops.linear_batched(x, w, m, k, n, workspace=ws))  # (and what a call leaves there)
+        assert np.array_equal(again, want)
+    w64, x64 = host(w.dequantize()).astype(np.float64).reshape(n, k), host(x).astype(np.float64)
+    assert np.all(np.abs(want.reshape(m, n) - x64 @ w64.T) <= 1e-5 * (np.abs(x64) @ np.abs(w64).T))
+
+
 # 33 and more rows of x: pairs of blocks, 256 weight rows against up to 256 rows of x.  One row of weights, one k-tile, one group,
 # both sides of the one-MMA form (128 rows of x), ragged last tiles on either side, split K, several units per pair.
 PAIR = [("w4", 33, 1, 128), ("w4", 128, 257, 256), ("w4", 129, 300, 384), ("w4", 256, 256, 384), ("w4", 257, 255, 128), ("w4", 40, 600, 16384),
