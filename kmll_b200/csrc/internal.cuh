@@ -191,12 +191,11 @@ int widen_bf16(cudaStream_t stream, const uint16_t* src, size_t n, float* dst);
 int linear_top1_offset(cudaStream_t stream, int fmt, const float* x, const uint16_t* norm_w, float eps, const void* w,
                        const void* scales, int rows, int cols, uint32_t token_offset, uint32_t* partial_tokens,
                        float* partial_logits, uint64_t* packed_out, const TpExchange* xc = nullptr, DecodeState* state = nullptr);
-// Batched fused linear forms for rows of x that are independent sequences (batch <= 16 per pass):
-// form 0 = RMSNorm + QKV (3 matrices, rows[0..2]), 1 = RMSNorm + gate/up + SiLU*up (2 matrices of rows[0]),
+// Batched fused linear forms for rows of x (independent sequences, or the tokens of a prompt):
+// form 0 = RMSNorm + QKV (3 matrices, rows[0..2]), 1 = RMSNorm + gate/up + SiLU*up (2 matrices of rows[0]; without workspace),
 // 2 = projection + residual, 3 = (RMSNorm +) projection, 4 = RMSNorm + gate/up into gate_tmp and up_tmp, 5 = SiLU(gate_tmp) *
-// up_tmp + projection + residual (overwrites gate_tmp).  Outputs are [batch, rows] row-major.
-// `workspace` (linear_batched_workspace_bytes(batch, cols) bytes) enables the tensor-core path for 5 or more rows; form 1
-// then also needs two [batch, rows] scratch matrices for the gate and up projections.
+// up_tmp + projection + residual (overwrites gate_tmp where the tensor-core path is off).  Outputs are [batch, rows] row-major.
+// `workspace` (linear_batched_workspace_bytes(batch, cols) bytes) enables the tensor-core path for 5 or more rows.
 int linear_batched_form(int form, cudaStream_t stream, int fmt, const float* x, int batch, const uint16_t* norm_w, float eps,
                         const void* const* w, const void* const* scales, const int* rows, int cols, float* const* outs,
                         const float* residual, void* workspace = nullptr, float* gate_tmp = nullptr, float* up_tmp = nullptr);

@@ -1280,8 +1280,7 @@ static int run_linear(const char* name, cudaStream_t stream, const float* x, int
                         FMT == FMT_W4 ? 128 : 64);
         }
     }
-    // 5 or more rows of x and a caller-owned workspace: the tcgen05 kernel (linear_gemm.cuh), up to 256 rows of x per pass
-    // over the weights
+    // 5 or more rows of x and a caller-owned workspace: the tcgen05 kernels (linear_gemm_small.cuh up to 32 rows, linear_gemm_pair.cuh above)
     if constexpr (EPI == EPI_STORE || EPI == EPI_RESIDUAL) {
         GemmPlan pl;
         bool ok = workspace != nullptr && gemm_enabled() && ldw == 0 && (ldx & 3) == 0 && aligned16(x) && aligned16(workspace) &&
@@ -1419,16 +1418,7 @@ static int batched_forms(int form, cudaStream_t stream, const float* x, int batc
             return run_linear<FMT, EPI_STORE>("linear_qkv_batched_norm", stream, x, batch, cols, cols, norm_w, eps, m, 3, 0, nullptr, nullptr,
                                               nullptr, 0, 0, workspace);
         }
-        case 1: {  // RMSNorm + gate/up + SiLU*up
-            GemmPlan pl;
-            if (workspace != nullptr && gate_tmp != nullptr && up_tmp != nullptr && gemm_enabled() && gemm_plan(FMT, batch, cols, rows[0], &pl)) {
-                // tensor-core path: gate and up as two plain projections over the same f16 planes of x, then SiLU(gate) * up
-                MatArg m[2] = {{w[0], scales[0], rows[0], gate_tmp, nullptr}, {w[1], scales[1], rows[0], up_tmp, nullptr}};
-                const int rc = run_linear<FMT, EPI_STORE>("silu_gate_up_batched_norm", stream, x, batch, cols, cols, norm_w, eps, m, 2, 0, nullptr,
-                                                          nullptr, nullptr, 0, 0, workspace);
-                if (rc != KMLL_OK) return rc;
-                return kmll_silu_mul_prefix(stream, gate_tmp, up_tmp, (size_t)batch * rows[0], outs[0]);
-            }
+        case 1: {  // RMSNorm + gate/up + SiLU*up, a few rows
             MatArg m[2] = {{w[0], scales[0], rows[0], outs[0], nullptr}, {w[1], scales[1], rows[0], nullptr, nullptr}};
             return run_linear<FMT, EPI_SILU>("silu_gate_up_batched_norm", stream, x, batch, cols, cols, norm_w, eps, m, 2, 0, nullptr, nullptr);
         }

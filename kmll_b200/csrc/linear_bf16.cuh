@@ -746,6 +746,7 @@ static int bf16_gemm_pair(cudaStream_t stream, const Bf16Gemm& g, GemmBf16Params
         const int n = (((g.T + xb - 1) / xb) + 15) & ~15;
         if (xb > xb_min && n < 96) break;
         const long long units = (long long)row_tiles * ((g.T + n - 1) / n);
+        if (units > 0x3fffffff) break;
         const double cost = (double)((units + kPClusters - 1) / kPClusters) * (KT * (2.0 * n + 60.0) + 2500.0);
         if (cost < best_cost * 0.995) {
             best_cost = cost;
@@ -754,6 +755,7 @@ static int bf16_gemm_pair(cudaStream_t stream, const Bf16Gemm& g, GemmBf16Params
             p.tiles = (int)units;
         }
     }
+    if (p.tiles == 0) return fail(KMLL_ERR_UNSUPPORTED, "bf16_gemm: too many tiles");
     p.row_tiles = row_tiles;
     p.ksplit = 1;
     const size_t stage = (size_t)kHRows * 128 + (size_t)p.n_block * 64;
@@ -844,9 +846,10 @@ int bf16_gemm(cudaStream_t stream, const Bf16Gemm& g) {
     p.rows = g.rows; p.K = g.K; p.T = g.T;
     p.out = g.out; p.out_bf16 = g.out_bf16; p.ldo = g.ldo; p.residual = g.residual; p.silu_rows = g.silu_rows;
     p.pair_act = g.pair_act; p.out_scale = g.out_scale;
+    if (g.T > kHMaxN) return bf16_gemm_pair(stream, g, p);
     p.row_tiles = (g.rows + kHRows - 1) / kHRows;
     // rows of x per tile: the size whose rounds over 148 SMs cost least (measured with K = 4096: 24 us at 64 rows, 32 at 256)
-    const int nmax = g.T >= kHMaxN ? kHMaxN : (g.T + 15) / 16 * 16;
+    const int nmax = (g.T + 15) / 16 * 16;
     int best = nmax;
     long long best_cost = -1;
     for (int nb = nmax; nb >= 64 || nb == nmax; nb -= 16) {
@@ -857,7 +860,6 @@ int bf16_gemm(cudaStream_t stream, const Bf16Gemm& g) {
     p.x_tiles = (g.T + best - 1) / best;  // walked fastest: the blocks at work share their weight rows, and x stays in L2
     const long long tiles = (long long)p.row_tiles * p.x_tiles;
     if (tiles > 0x3fffffff) return fail(KMLL_ERR_UNSUPPORTED, "bf16_gemm: too many tiles");
-    if (g.T > kHMaxN) return bf16_gemm_pair(stream, g, p);
     p.tiles = (int)tiles;
     p.ksplit = 1;
     if (g.partial != nullptr && g.T <= kGemmSplitRows && p.tiles <= 74) {  // at least eight k-tiles per piece

@@ -1,5 +1,5 @@
 // W4-G128 linear for small batches (5 to 32 rows of activations: batches of sequences decoding in lockstep), included
-// by linear.cu after linear_gemm.cuh.  Serves the same kmll operator as linear_gemm.cuh (linear_batched_i8_scaled,
+// by linear.cu after linear_gemm.cuh.  Serves the same kmll operator as linear_gemm_pair.cuh (linear_batched_i8_scaled,
 // crates/inference/src/ops/matmul.rs:423-463, over W4-G128 weights) where the work is a stream of weights, not a
 // contraction: the point is to keep every multiprocessor's share of the HBM stream in flight.
 //

@@ -759,9 +759,10 @@ struct BatchDecoder {
     size_t cache_stride = 0;  // floats between two sequences' caches
     std::vector<float*> key_cache, value_cache;  // per layer: [batch][max_seq * kv_len]
     float *hidden_a = nullptr, *hidden_b = nullptr, *hidden_mid = nullptr, *q = nullptr, *k = nullptr, *v = nullptr;
-    float *attn = nullptr, *act = nullptr, *logits = nullptr, *attn_ws = nullptr;
-    float *gate = nullptr, *up = nullptr;  // [batch, hidden] scratch of the tensor-core gate/up path
-    void* linear_ws = nullptr;             // scratch of the batched linears (f16 planes of the activations)
+    float *attn = nullptr, *logits = nullptr, *attn_ws = nullptr;
+    void* linear_ws = nullptr;             // scratch of the batched linears (digits or planes of the activations); null below 5 sequences
+    float *gate = nullptr, *up = nullptr;  // [batch, hidden] of the feed-forward, with linear_ws
+    float* act = nullptr;                  // [batch, hidden] of the feed-forward, without
     BatchState* state = nullptr;
     uint64_t* history = nullptr;  // [batch][history_cap]
     int history_cap = 0;
@@ -825,9 +826,8 @@ static int enqueue_batch_step(BatchDecoder* b, cudaStream_t s, int* launches) {
                                          b->gate, b->up));
             KMLL_TRY(linear_batched_form(5, s, c.format, nullptr, B, nullptr, 0.f, w2, sc2, dim_rows, c.hidden_dim, out, b->hidden_mid, b->linear_ws, b->gate, b->up));
         } else {
-            KMLL_TRY(linear_batched_form(1, s, c.format, b->hidden_mid, B, L.ffn_norm, c.norm_eps, w13, sc13, hidden_rows, c.dim, act_out, nullptr, b->linear_ws, b->gate,
-                                         b->up));
-            KMLL_TRY(linear_batched_form(2, s, c.format, b->act, B, nullptr, 0.f, w2, sc2, dim_rows, c.hidden_dim, out, b->hidden_mid, b->linear_ws));
+            KMLL_TRY(linear_batched_form(1, s, c.format, b->hidden_mid, B, L.ffn_norm, c.norm_eps, w13, sc13, hidden_rows, c.dim, act_out, nullptr));
+            KMLL_TRY(linear_batched_form(2, s, c.format, b->act, B, nullptr, 0.f, w2, sc2, dim_rows, c.hidden_dim, out, b->hidden_mid));
         }
         float* t = hidden;
         hidden = other;
@@ -1647,9 +1647,6 @@ int kmll_batch_create(kmll_decoder_t dec, int batch, kmll_batch_t* out) {
         KMLL_TRY(balloc(b, &b->attn, (size_t)batch * q_len));
         KMLL_TRY(balloc(b, &b->k, (size_t)batch * kv_len));
         KMLL_TRY(balloc(b, &b->v, (size_t)batch * kv_len));
-        KMLL_TRY(balloc(b, &b->act, (size_t)batch * c.hidden_dim));
-        KMLL_TRY(balloc(b, &b->gate, (size_t)batch * c.hidden_dim));
-        KMLL_TRY(balloc(b, &b->up, (size_t)batch * c.hidden_dim));
         {
             const int widest = c.hidden_dim > c.dim ? (c.hidden_dim > q_len ? c.hidden_dim : q_len) : (c.dim > q_len ? c.dim : q_len);
             const size_t ws_bytes = linear_batched_workspace_bytes(batch, widest);
@@ -1657,6 +1654,10 @@ int kmll_batch_create(kmll_decoder_t dec, int batch, kmll_batch_t* out) {
                 unsigned char* p = nullptr;
                 KMLL_TRY(balloc(b, &p, ws_bytes));
                 b->linear_ws = p;
+                KMLL_TRY(balloc(b, &b->gate, (size_t)batch * c.hidden_dim));
+                KMLL_TRY(balloc(b, &b->up, (size_t)batch * c.hidden_dim));
+            } else {
+                KMLL_TRY(balloc(b, &b->act, (size_t)batch * c.hidden_dim));
             }
         }
         KMLL_TRY(balloc(b, &b->logits, (size_t)batch * c.vocab_size));
