@@ -173,6 +173,12 @@ def test_pair_gemm_error_bound(cuda, fmt, m, n, k):
     got = host(ops.linear_batched(dev(x), w, m, k, n, workspace=ops.linear_batched_workspace(m, k))).reshape(m, n)
     bound = (2.0 ** -22 + (k / 16 + 16) * 2.0 ** -23) * (np.abs(x64) @ np.abs(w64).T) + 1e-30
     assert np.all(np.abs(got - x64 @ w64.T) <= bound)
+    # That bound lets a lost plane of x pass at long K.  As a whole, rows of x of equal weight: half a bit of the planes (2^-22) and of each
+    # step of the sums, W4 eight to a group and one per group, RS-I8 one per 16 columns, half of them in either accumulator.  Without the low plane: 1.4e-4.
+    steps = 8 + k / 128 if fmt == "w4" else k / 32
+    length = np.linalg.norm(x64, axis=1)[:, None]
+    off = np.linalg.norm((got - x64 @ w64.T) / length) / np.linalg.norm(x64 @ w64.T / length)
+    assert off <= 2.0 ** -22 + steps * 2.0 ** -23
     again = host(ops.linear_batched(dev(x), w, m, k, n, workspace=ops.linear_batched_workspace(m, k))).reshape(m, n)
     assert np.array_equal(got, again)
 

@@ -77,6 +77,78 @@ def test_sliding_window_other_step_forms_and_bf16(cuda):
         dec.close()
 
 
+# fused = 0 keeps the f32 prompt attention: two, four and eight query rows per thread (by heads x rows), both head sizes and cache types; windows
+# that leave out whole 64-key tiles, begin inside one, hold one position, and none
+@pytest.mark.parametrize("n,heads,kv,hd", [(150, 4, 2, 64), (150, 4, 1, 128), (190, 32, 8, 64), (160, 32, 4, 128), (640, 32, 8, 64), (590, 32, 8, 128)])
+@pytest.mark.parametrize("window,kv_bf16", [(0, True), (1, False), (20, True), (70, False)])
+def test_f32_prompt_attention_matches_oracle(cuda, n, heads, kv, hd, window, kv_bf16):
+    """The last row of prompts that end at several places of a row block and of a tile, against the oracle's pass over the longest."""
+    cfg = tiny(rt.FORMAT_RS_I8, False, n_layers=1, n_heads=heads, n_kv_heads=kv, head_dim=hd, max_seq_len=n + 8, sliding_window=window, kv_bf16=kv_bf16)
+    dec = make(cfg)
+    ora = OracleDecoder(cfg, dec)
+    prompt = np.random.default_rng(n + window).integers(0, cfg.vocab_size, n)
+    ends = {n, n - 1, n - 9, n - 30, n // 64 * 64, n // 64 * 64 + 1}
+    for at, token in enumerate(prompt, 1):
+        ora.forward(int(token))
+        if at in ends:
+            dec.prefill(prompt[:at])
+            got = dec.last_hidden()
+            scale = max(float(np.max(np.abs(ora.hidden))), 1.0)
+            assert np.max(np.abs(got - ora.hidden)) <= (BF16_KV_BOUND["hid_tol"] if kv_bf16 else 2e-4) * scale, at
+    dec.close()
+
+
+WIDE_FEED_FORWARD = """
+import json, sys
+import numpy as np
+from kmll_b200 import runtime as rt
+out = {}
+for fmt in (rt.FORMAT_RS_I8, rt.FORMAT_W4G128):
+    dec = rt.Decoder(rt.DecoderConfig(n_layers=2, dim=128, n_heads=2, n_kv_heads=1, head_dim=64, hidden_dim=16512, vocab_size=640, norm_eps=1e-6, max_seq_len=96, format=fmt))
+    dec.init_random(3, 0.05)
+    for n in (7, 33, 70):
+        dec.prefill(np.arange(n) * 7 % 640)
+        out[f"{fmt} {n}"] = dec.last_hidden().tolist()
+    batch = rt.BatchDecoder(dec, 6)
+    for slot in range(6):
+        dec.prefill(np.arange(9) + slot)
+        batch.adopt(slot)
+    tokens, logits = batch.generate_greedy(3)
+    out[f"{fmt} batch"] = logits.tolist()
+    batch.close()
+    dec.close()
+print("RESULT " + json.dumps(out))
+"""
+
+
+def test_feed_forward_wider_than_a_block_holds(cuda):
+    """A down projection of 16512 columns: more than the kernels that form SiLU(gate) * up in front of it keep in registers, so they
+    read part of a row twice.  Prompts on either side of 32 rows against the oracle, and everything against the same
+    without the tensor-core linears (KMLL_GEMM=0: gate, up, SiLU * up and the projection one after another)."""
+    import json
+    import os
+    import subprocess
+    import sys
+
+    runs = []
+    for env in ({}, {"KMLL_GEMM": "0"}):
+        r = subprocess.run([sys.executable, "-c", WIDE_FEED_FORWARD], env=dict(os.environ, **env), capture_output=True, text=True, timeout=300,
+                           cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+        assert r.returncode == 0, r.stderr[-2000:]
+        runs.append(json.loads(next(line for line in r.stdout.splitlines() if line.startswith("RESULT "))[7:]))
+    for key, want in runs[1].items():
+        want, got = np.asarray(want), np.asarray(runs[0][key])
+        assert np.max(np.abs(got - want)) <= 2e-4 * max(float(np.max(np.abs(want))), 1.0), key
+    for fmt in (rt.FORMAT_RS_I8, rt.FORMAT_W4G128):
+        cfg = rt.DecoderConfig(n_layers=2, dim=128, n_heads=2, n_kv_heads=1, head_dim=64, hidden_dim=16512, vocab_size=640, norm_eps=1e-6, max_seq_len=96, format=fmt)
+        dec = make(cfg, seed=3)
+        for n in (7, 33):
+            ora = OracleDecoder(cfg, dec)
+            ora.prefill(np.arange(n) * 7 % 640)
+            assert np.max(np.abs(np.asarray(runs[0][f"{fmt} {n}"]) - ora.hidden)) <= 2e-4 * max(float(np.max(np.abs(ora.hidden))), 1.0), (fmt, n)
+        dec.close()
+
+
 @pytest.mark.parametrize("window", [1, 20, 70])
 def test_f32_prompt_attention_window_keeps_non_finite_values_out(cuda, window):
     """fused = 0, one layer: the last row's hidden state does not change when a token before its window turns into NaN (the
