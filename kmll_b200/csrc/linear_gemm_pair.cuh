@@ -15,9 +15,9 @@
 // Why pairs: with one block per tile both planes of 256 rows of x cross L2 -> SM for every 128 weight rows (64 bytes per cycle
 // at the MMA rate of two planes, the whole port); a pair brings each row of x into one of the two blocks only.
 //
-// Measured, split of x included (one block per 128 x 256 tile with three / two MMAs per k-step before): W4 2048 x 14336 x 4096
-// 612 -> 367 us (656 TFLOP/s useful, 1310 of MMA work), RS-I8 587 -> 329, W4 300 x 18944 x 3584 131 -> 81, 64 x 14336 x 4096 53 -> 32,
-// RS-I8 333 x 4096 x 4096 74 -> 38, W4 33 x 3584 x 3584 28 -> 22.  Error against 64 bits 8.4e-6 -> 2.6e-7 (W4: no second weight plane).
+// Measured in a graph of ten calls, split of x included (one block per 128 x 256 tile with three / two MMAs per k-step before): W4 2048 x 14336 x
+// 4096 612 -> 355 us (677 TFLOP/s useful, 1353 of MMA work), RS-I8 587 -> 328, W4 300 x 18944 x 3584 131 -> 73, 64 x 14336 x 4096 53 -> 29,
+// RS-I8 333 x 4096 x 4096 74 -> 31, W4 33 x 3584 x 3584 28 -> 17.  Error against 64 bits 8.4e-6 -> 2.6e-7 (W4: no second weight plane).
 //
 // Roles of a block (512 threads, one block per SM, persistent over units = (weight row tile, x block, k-split)):
 //   warp 0      TMA of x: both planes of n_block / 2 rows, one 3-D box per 64-column k-tile
