@@ -50,6 +50,35 @@ def test_batch_matches_single_sequence(cuda, fmt, batch):
     dec.close()
 
 
+@pytest.mark.parametrize("fmt", [rt.FORMAT_RS_I8, rt.FORMAT_W4G128])
+@pytest.mark.parametrize("vocab,batch", [(641, 7), (4100, 9), (16388, 2)])
+def test_batch_arg_max_over_ragged_rows(cuda, fmt, vocab, batch):
+    """Logits rows that are and are not whole 16-byte pieces (fewer pieces than threads, more, a last round of one): the step's
+    token is the arg-max that the single-sequence decoder finds for the same prompt, and so is its logit."""
+    cfg = _cfg(fmt, vocab_size=vocab)
+    dec = rt.Decoder(cfg)
+    dec.init_random(11, 0.05, False)
+    rng = np.random.default_rng(vocab)
+    prompts = [rng.integers(0, vocab, 9) for _ in range(batch)]
+    singles = []
+    for p in prompts:
+        dec.prefill(p)
+        singles.append([v.copy() for v in dec.generate_greedy(3)])
+    bd = rt.BatchDecoder(dec, batch)
+    for slot, p in enumerate(prompts):
+        dec.prefill(p)
+        bd.adopt(slot)
+    tokens, logits = bd.generate_greedy(3)
+    for slot, (ref_t, ref_l) in enumerate(singles):
+        for i in range(3):
+            tol = 2e-3 * max(1.0, abs(float(ref_l[i])))  # two kernels of f32 sums over 256 and 512 columns, as above
+            assert abs(float(logits[slot, i]) - float(ref_l[i])) <= tol, (slot, i)
+            if int(tokens[slot, i]) != int(ref_t[i]):  # a near-tie: the sequences part
+                break
+    bd.close()
+    dec.close()
+
+
 @pytest.mark.parametrize("kv_bf16", [False, True])
 def test_batch_gqa_head_dim_128(cuda, kv_bf16):
     cfg = _cfg(rt.FORMAT_W4G128, n_heads=8, n_kv_heads=2, head_dim=128, dim=256, max_seq_len=96, kv_bf16=kv_bf16)
