@@ -1375,9 +1375,14 @@ int decode_attention_launch(cudaStream_t stream, const float* q, const float* k_
 }
 
 int prefill_attention_launch(cudaStream_t stream, const float* q_batch, const float* k_cache, const float* v_cache, int prompt_len,
-                             int n_heads, int n_kv_heads, int head_dim, float* out, int kv_bf16, int window, int tensor_cores) {
+                             int n_heads, int n_kv_heads, int head_dim, float* out, int kv_bf16, int window, int tensor_cores,
+                             const uint16_t* k_planes, const uint16_t* v_planes) {
     cudaError_t e;
     static const bool mma_allowed = [] { const char* v = getenv("KMLL_PREFILL_MMA"); return !(v != nullptr && v[0] == '0'); }();
+    const void* k_rows = kv_bf16 ? static_cast<const void*>(k_cache) : k_planes;
+    const void* v_rows = kv_bf16 ? static_cast<const void*>(v_cache) : v_planes;
+    if (tensor_cores && mma_allowed && k_rows != nullptr && prompt_attention_serves(q_batch, k_rows, v_rows, out, prompt_len, n_heads, head_dim))
+        return prompt_attention_launch(stream, q_batch, k_rows, v_rows, prompt_len, n_heads, n_kv_heads, head_dim, out, kv_bf16, window);
     if (tensor_cores && mma_allowed && (head_dim == 64 || head_dim == 128)) {
         const dim3 grid_mma(n_heads, (prompt_len + 63) / 64);
         const size_t smem = (size_t)(kv_bf16 ? 2 : 4) * 64 * (head_dim + 8) * 2;

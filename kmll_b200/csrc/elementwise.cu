@@ -2,6 +2,7 @@
 // KV-cache writes, row softmax, embedding lookup, arg-max / top-k.  Each makes one pass over
 // HBM with 128-bit accesses where alignment allows; all arithmetic is f32 in kmll's order.
 #include "internal.cuh"
+#include "mma_bf16.cuh"
 
 namespace kmll {
 
@@ -269,7 +270,7 @@ __global__ void prepare_prefill_kernel(const float* __restrict__ q, const float*
 __global__ void __launch_bounds__(256) prepare_prefill_quads_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                                                     const float* __restrict__ freqs, int half, int q_len, int kv_len, int position0,
                                                                     float* __restrict__ q_rot, float* __restrict__ k_cache, float* __restrict__ v_cache,
-                                                                    int kv_bf16) {
+                                                                    int kv_bf16, uint16_t* __restrict__ k_planes, uint16_t* __restrict__ v_planes) {
     extern __shared__ float turns[];  // [half] cosines, [half] sines
     pdl_wait();
     const int row = blockIdx.x;
@@ -292,10 +293,20 @@ __global__ void __launch_bounds__(256) prepare_prefill_quads_kernel(const float*
             *reinterpret_cast<float4*>(cache + at) = x;
         }
     };
+    auto put_planes = [&](uint16_t* planes, int c, const float4& x) {  // for the tensor-core attention: (row, head), (row, remainder)
+        if (planes == nullptr) return;
+        uint2 hi, lo;
+        split_bf16x2(x.x, x.y, hi.x, lo.x);
+        split_bf16x2(x.z, x.w, hi.y, lo.y);
+        *reinterpret_cast<uint2*>(planes + 2 * kv0 + c) = hi;
+        *reinterpret_cast<uint2*>(planes + 2 * kv0 + kv_len + c) = lo;
+    };
     for (int i = (int)blockIdx.y * 256 + threadIdx.x; i < nq + nk + nv; i += 256 * (int)gridDim.y) {
         if (i >= nq + nk) {
             const int c = (i - nq - nk) * 4;
-            put(v_cache, cache0 + c, *reinterpret_cast<const float4*>(v + kv0 + c));
+            const float4 x = *reinterpret_cast<const float4*>(v + kv0 + c);
+            put(v_cache, cache0 + c, x);
+            put_planes(v_planes, c, x);
             continue;
         }
         const bool is_q = i < nq;
@@ -312,20 +323,26 @@ __global__ void __launch_bounds__(256) prepare_prefill_quads_kernel(const float*
         } else {
             put(k_cache, cache0 + at, x);
             put(k_cache, cache0 + at + half, y);
+            put_planes(k_planes, at, x);
+            put_planes(k_planes, at + half, y);
         }
     }
 }
 
 // Whole heads in aligned pieces of four, or one value per thread.  (The caches' alignment is that of their base: rows are multiples
-// of a head.)  Short prompts share a row between up to four blocks.
+// of a head.)  Short prompts share a row between up to four blocks.  The aligned form also writes the bf16 planes of the rows,
+// [row][2][kv_len], where they are asked for; `planes_written` says whether it did.
 static cudaError_t launch_prepare_prefill(cudaStream_t stream, const float* q, const float* k, const float* v, const float* freqs, int half, int rows, int q_len,
-                                          int kv_len, int head_dim, int position0, float* q_rot, float* k_cache, float* v_cache, int kv_bf16) {
+                                          int kv_len, int head_dim, int position0, float* q_rot, float* k_cache, float* v_cache, int kv_bf16,
+                                          uint16_t* k_planes = nullptr, uint16_t* v_planes = nullptr, bool* planes_written = nullptr) {
+    if (planes_written != nullptr) *planes_written = false;
     uintptr_t bits = 0;
     for (const void* p : {(const void*)q, (const void*)k, (const void*)v, (const void*)q_rot, (const void*)k_cache, (const void*)v_cache}) bits |= reinterpret_cast<uintptr_t>(p);
     if (2 * half == head_dim && half % 4 == 0 && half <= 4096 && (bits & 15u) == 0) {
         const int parts = rows >= 148 ? 1 : rows >= 74 ? 2 : 4;
+        if (planes_written != nullptr) *planes_written = k_planes != nullptr;
         return launch(prepare_prefill_quads_kernel, dim3(rows, parts), dim3(256), (size_t)half * 8, stream, true, q, k, v, freqs, half, q_len, kv_len, position0, q_rot,
-                      k_cache, v_cache, kv_bf16);
+                      k_cache, v_cache, kv_bf16, k_planes, v_planes);
     }
     const size_t total = (size_t)rows * (q_len > kv_len ? q_len : kv_len);
     return launch(prepare_prefill_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, true, q, k, v, freqs, half, rows, q_len, kv_len, head_dim,
@@ -566,8 +583,9 @@ int qk_head_rmsnorm(cudaStream_t stream, float* q, float* k, const uint16_t* q_w
 
 int prepare_prefill_offset(cudaStream_t stream, const float* q, const float* k, const float* v, const float* freqs,
                            int n_freqs, int rows, int q_len, int kv_len, int head_dim, int position0, float* q_rot,
-                           float* k_cache, float* v_cache, int kv_bf16) {
-    cudaError_t e = launch_prepare_prefill(stream, q, k, v, freqs, n_freqs, rows, q_len, kv_len, head_dim, position0, q_rot, k_cache, v_cache, kv_bf16);
+                           float* k_cache, float* v_cache, int kv_bf16, uint16_t* k_planes, uint16_t* v_planes, bool* planes_written) {
+    cudaError_t e = launch_prepare_prefill(stream, q, k, v, freqs, n_freqs, rows, q_len, kv_len, head_dim, position0, q_rot, k_cache, v_cache, kv_bf16, k_planes, v_planes,
+                                           planes_written);
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "prepare_prefill: %s", cudaGetErrorString(e));
     return KMLL_OK;
 }

@@ -6,6 +6,8 @@
 #include "../../include/kmll_b200_runtime.h"
 #include "common.cuh"
 
+struct CUtensorMap_st;
+
 namespace kmll {
 
 // Device-resident state of a decode loop.
@@ -160,11 +162,21 @@ int qk_head_rmsnorm(cudaStream_t stream, float* q, float* k, const uint16_t* q_w
                     int head_dim, float eps, size_t q_stride, size_t k_stride);
 int prepare_prefill_offset(cudaStream_t stream, const float* q, const float* k, const float* v, const float* freqs,
                            int n_freqs, int rows, int q_len, int kv_len, int head_dim, int position0, float* q_rot,
-                           float* k_cache, float* v_cache, int kv_bf16 = 0);
+                           float* k_cache, float* v_cache, int kv_bf16 = 0, uint16_t* k_planes = nullptr, uint16_t* v_planes = nullptr,
+                           bool* planes_written = nullptr);
 // one row of the KV cache at `position` (f32, or rounded to bf16 when the decoder keeps its cache in bf16)
 int write_kv_row(cudaStream_t stream, const float* x, int position, int token_len, int head_dim, float* cache, int kv_bf16);
+// Prompt attention on the tensor cores (prompt_attention.cu): rows of q in f32, 16-byte aligned operands.  `k`, `v`: rows of bf16,
+// [position][n_kv_heads * head_dim] (kv_bf16: the caches) or [position][2][n_kv_heads * head_dim], the two planes of an f32 row.
+bool prompt_attention_serves(const void* q, const void* k, const void* v, const void* out, int prompt_len, int n_heads, int head_dim);
+int prompt_attention_launch(cudaStream_t stream, const float* q_batch, const void* k, const void* v, int prompt_len, int n_heads, int n_kv_heads,
+                            int head_dim, float* out, int kv_bf16, int window);
+// tensor map of a row-major bf16 matrix [rows, inner] with boxes of box_rows rows of 64 entries in the 128-byte swizzle
+int make_map_bf16_rows(CUtensorMap_st* map, const void* base, uint64_t inner, uint64_t rows, uint64_t pitch_bytes, uint32_t box_rows);
+int prompt_attention_status(int* status_out);  // 1 after a wait inside a kernel of that file ran out, 0 otherwise
 int prefill_attention_launch(cudaStream_t stream, const float* q_batch, const float* k_cache, const float* v_cache, int prompt_len,
-                             int n_heads, int n_kv_heads, int head_dim, float* out, int kv_bf16, int window, int tensor_cores);
+                             int n_heads, int n_kv_heads, int head_dim, float* out, int kv_bf16, int window, int tensor_cores,
+                             const uint16_t* k_planes = nullptr, const uint16_t* v_planes = nullptr);
 // hidden = embedding[state->next_top.token]; also records next_top into history[state->step] and
 // sets seq_len = position + 1.
 int decode_begin(cudaStream_t stream, const uint16_t* table, int vocab, int dim, DecodeState* state, uint64_t* history,

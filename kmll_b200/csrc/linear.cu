@@ -29,6 +29,7 @@
 #include <mutex>
 
 #include "internal.cuh"
+#include "tcgen05.cuh"
 
 namespace kmll {
 // 0 = ok; first failure wins: 1 = a wait inside the linear kernel timed out, 2 = a tensor-parallel peer did not
@@ -1005,6 +1006,10 @@ static int make_map_2d(CUtensorMap* map, CUtensorMapDataType type, int elem, con
     return KMLL_OK;
 }
 
+int make_map_bf16_rows(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t pitch_bytes, uint32_t box_rows) {
+    return make_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, inner, rows, pitch_bytes, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+}
+
 }  // namespace kmll
 
 #include "linear_bf16.cuh"
@@ -1497,7 +1502,7 @@ int kmll_device_status(int* status_out) {
     KMLL_REQUIRE_PTR(status_out);
     cudaError_t e = cudaMemcpyFromSymbol(status_out, g_device_status, sizeof(int));
     if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "device_status: %s", cudaGetErrorString(e));
-    return KMLL_OK;
+    return *status_out != 0 ? KMLL_OK : prompt_attention_status(status_out);
 }
 
 int kmll_linear_i8(kmll_stream_t s, const float* x, const int8_t* w, const float* scales, int rows, int cols, float* y) {

@@ -366,10 +366,6 @@ struct GemmBf16Params {
     unsigned int* counters;  // [tiles], zero between launches
 };
 
-__host__ __device__ constexpr uint32_t gemm_idesc_bf16(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
 __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const GemmBf16Params p, const __grid_constant__ CUtensorMap map_w,
                                                                        const __grid_constant__ CUtensorMap map_x) {
     extern __shared__ unsigned char hsmem_raw[];

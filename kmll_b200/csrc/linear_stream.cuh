@@ -28,7 +28,6 @@ namespace kmll {
 
 constexpr int kSWarps = 16;
 constexpr int kSThreads = kSWarps * 32;
-constexpr unsigned long long kWaitLimitTicks = 4000000000ull;  // every mbarrier wait gives up after this many cycles (2 to 4 s)
 
 
 struct StreamParams {
@@ -53,42 +52,10 @@ struct StreamParams {
     float* x_out;      // gather: block 0 also writes the summed vector here (the residual stream)
 };
 
-__device__ inline uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ inline void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ inline void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ inline bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 __device__ inline unsigned long long global_timer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
-}
-// Bounded wait; false = timed out (the caller raises the status word and unwinds).  There is no
-// blocking hardware barrier anywhere in the kernel, so a time-out in one warp can never leave
-// another warp waiting forever.
-template <bool BACKOFF = true>
-__device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();  // (not %globaltimer: reading that register costs a good fraction of a microsecond)
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 32; ++i) {
-            if (mbar_try_wait(bar, parity)) return true;
-            if (BACKOFF) __nanosleep(64);  // leave the issue slots to the warps that share the scheduler
-        }
-        if ((unsigned long long)(clock64() - t0) > kWaitLimitTicks) return false;
-    }
 }
 // 16-byte asynchronous global->shared copy that bypasses L1 (weights are read once).
 __device__ inline void cp_async_stream16(void* smem_dst, const void* gmem_src) {

@@ -1317,10 +1317,14 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
                                                     q_len, kv_len, ws, qb, kb, vb));
             }
             KMLL_TRY(apply_qk_norm(d, s, L, qb, kb, n));
+            // An f32 cache's rows as bf16 planes for the attention: in the buffers of gate and up, which are written behind it
+            uint16_t* kp = c.fused && !c.kv_bf16 && d->hidden_l >= kv_len ? reinterpret_cast<uint16_t*>(gb) : nullptr;
+            uint16_t* vp = kp != nullptr ? reinterpret_cast<uint16_t*>(ub) : nullptr;
+            bool planes = false;
             KMLL_TRY(prepare_prefill_offset(s, qb, kb, vb, d->freqs, c.rotary_dim / 2, n, q_len, kv_len, c.head_dim, 0, qrb, L.key_cache,
-                                            L.value_cache, c.kv_bf16));
+                                            L.value_cache, c.kv_bf16, kp, vp, &planes));
             KMLL_TRY(prefill_attention_launch(s, qrb, L.key_cache, L.value_cache, n, d->n_heads_l, d->n_kv_l, c.head_dim, ab, c.kv_bf16,
-                                              c.sliding_window, c.fused ? 1 : 0));  // fused = 0: kmll's f32 operator arithmetic throughout
+                                              c.sliding_window, c.fused ? 1 : 0, planes ? kp : nullptr, planes ? vp : nullptr));  // fused = 0: kmll's f32 operator arithmetic throughout
             if (forms) {
                 {
                     const void* w[1] = {L.wo.w};

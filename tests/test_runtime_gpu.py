@@ -98,6 +98,27 @@ def test_f32_prompt_attention_matches_oracle(cuda, n, heads, kv, hd, window, kv_
     dec.close()
 
 
+@pytest.mark.parametrize("heads,kv,hd", [(4, 2, 64), (4, 1, 128), (8, 8, 128)])
+@pytest.mark.parametrize("window,kv_bf16", [(0, False), (0, True), (1, False), (100, True), (130, False), (300, False)])
+def test_prompt_attention_tiles_match_oracle(cuda, heads, kv, hd, window, kv_bf16):
+    """Attention on tensor memory: prompts that end around the 128 rows of a block and the 128 keys of a tile, one to four tiles (one and
+    two streams of tiles), windows that start inside a tile; (8, 8, 128) has keys wider than the feed-forward, so an f32 cache has
+    no room for planes and keeps the other kernel.  Bounds as in the tests above."""
+    n = 390
+    cfg = tiny(rt.FORMAT_RS_I8, True, n_layers=1, n_heads=heads, n_kv_heads=kv, head_dim=hd, max_seq_len=n + 8, sliding_window=window, kv_bf16=kv_bf16)
+    dec = make(cfg)
+    ora = OracleDecoder(cfg, dec)
+    prompt = np.random.default_rng(heads + hd + window).integers(0, cfg.vocab_size, n)
+    for at, token in enumerate(prompt, 1):
+        ora.forward(int(token))
+        if at in (1, 2, 64, 127, 128, 129, 255, 256, 257, 383, 384, 385, 390):
+            dec.prefill(prompt[:at])
+            got = dec.last_hidden()
+            scale = max(float(np.max(np.abs(ora.hidden))), 1.0)
+            assert np.max(np.abs(got - ora.hidden)) <= (BF16_KV_BOUND["hid_tol"] if kv_bf16 else 2e-4) * scale, at
+    dec.close()
+
+
 WIDE_FEED_FORWARD = """
 import json, sys
 import numpy as np
