@@ -12,18 +12,20 @@
 // per group.  No second weight plane and no cross terms are needed.
 //
 // Pipeline.  One persistent block per multiprocessor walks its (row tile, k-split) units group by group; up to three
-// matrices that share x (q / k / v, gate / up) are one launch, their row tiles numbered through.  Measured on B200: every
-// mbarrier, TMA or tcgen05 instruction costs the thread that issues it 100 to 250 cycles, so ONE pass of any role over a
-// group takes 1100 to 1300 cycles however little it computes - several times the HBM share of a group (8 KB at 44 GB/s
-// per multiprocessor = 360 cycles).  Two things follow.  Each buffer has a ring of its own, sized by how long its contents
-// live; and the roles that do work per group exist twice and take the groups alternately:
+// matrices that share x (q / k / v, gate / up) are one launch, their row tiles numbered through.  A pass of any role over a group
+// costs several hundred cycles however little it computes (waits, fences, arrivals), more than the HBM share of a group (8 KB at 44
+// GB/s per multiprocessor = 360 cycles).  So each buffer has a ring of its own, sized by how long its contents
+// live; the roles that do work per group exist twice and take the groups alternately; and the issuing roles run as whole
+// warps with one elected lane (tcgen05.cuh): as single threads, at 100 to 250 cycles per mbarrier, TMA or tcgen05 instruction, 16
+// rows of x took 30.2 us for 28672 x 4096 where they take 28.4 now, 13.0 / 11.7 for 4096 x 4096, 21.3 / 19.5 for 4096 x 14336, RS-I8
+// 4096 x 14336 18.8 / 17.5, 32 rows and 4096 x 4096 19.6 / 15.3.
 //   * raw weight tiles (128 rows x 64 bytes of nibbles, TMA by warp 8): 12 slots (7 with 32 rows of x) - they wait out the HBM latency;
 //   * digit planes of the same 128 columns (one 3-D TMA box, 128-byte swizzle, warp 4): 5 or 6 slots - L2 latency;
 //   * signed-byte weight tiles in the swizzled K-major layout the MMA reads: 4 slots, written by two sets of four
 //     expanding warps (seven integer instructions per word; the even and odd columns of a word come out as two runs, the
 //     digit planes are stored in that column order);
 //   * accumulators in tensor memory: 8 (16 rows of x) or 4 (32 rows) buffers of 4 n_block columns.
-//   One thread of each of warps 0 and 11 waits for a group's `a_ready` barrier, its digit planes and its accumulator
+//   The elected lane of each of warps 0 and 11 waits for a group's `a_ready` barrier, its digit planes and its accumulator
 //   buffer, issues the four MMAs (M = 128 weight rows, N = 4 n_block digit columns, K = 32 bytes each) and one commit on a
 //   ring of 16 `done` barriers; the producers, the expanding warps and the draining warps all derive what they wait for
 //   from that ring (the slot they want to refill was last used by the group `ring size` back).  Two sets of four warps
@@ -199,13 +201,6 @@ __global__ void __launch_bounds__(kDigitThreads) digit_rows_kernel(const float* 
 __host__ __device__ constexpr uint32_t gemm_idesc_s8s8(int m, int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-__device__ inline void gemm_mma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
 // four unsigned nibble bytes (0..15 each) -> four signed bytes nibble - 8, without a carry between the bytes
 __device__ inline uint32_t nibble_bytes_to_s8(uint32_t w, uint32_t shift) {
     const uint32_t t = lop3_and_or(w >> shift, 0x0f0f0f0fu, 0x80808080u);
@@ -342,7 +337,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xchg_free + 1);
     uint32_t* last_flag = tmem_slot + 1;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp_index();
     const int G = p.K >> 7;  // 128-column groups
 
     if (tid == 0) {
@@ -368,6 +363,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
     bool ok = true;
     // the `done` barrier and parity that report the completion of item number n of this block
     auto done_wait = [&](int n) { return mbar_wait<false>(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
+    auto done_warp_wait = [&](int n) { return warp_wait(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
     static_assert(kBtDoneRing == 16, "done_wait shifts by 4");
     const bool expander = warp < 11 && (warp & 3) != 0;  // warps 1 2 3 5 6 7 9 10
     UnitCursor cur;
@@ -376,48 +372,51 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
         // ---- TMA of the raw weight tiles.  The weights never change, so these copies start at once, whatever the previous
         // kernel is still doing.  With two groups per item the box is 128 bytes wide (128-byte swizzle, which the expanding
         // warps undo when they read); a box that reaches past the unit or past K brings bytes nobody uses, or zeros.
-        if (lane == 0 && cur.start(p, blockIdx.x, G)) {
+        if (cur.start(p, blockIdx.x, G)) {
+            const uint32_t lead = elect_lead();
             RingPos<S::kRawSlots> rp;
             PROF_DECL;
             do {
                 PROF_W0;
-                if (rp.wrapped && !mbar_wait<false>(&raw_free[rp.idx], rp.phase ^ 1u)) { ok = false; break; }
+                if (rp.wrapped && !warp_wait(&raw_free[rp.idx], rp.phase ^ 1u)) { ok = false; break; }
                 PROF_W1;
                 const int mi = (p.nmat > 2 && cur.tile >= p.mat[2].tile_start) ? 2 : (p.nmat > 1 && cur.tile >= p.mat[1].tile_start) ? 1 : 0;
                 const CUtensorMap* map = mi == 0 ? &map_w0 : mi == 1 ? &map_w1 : &map_w2;
-                mbar_arrive_expect_tx(&raw_full[rp.idx], (uint32_t)S::kRawBytes);
-                tma_load_2d(smem_base + (uint32_t)rp.idx * S::kRawBytes, map, cur.g * 64, (cur.tile - p.mat[mi].tile_start) * 128, &raw_full[rp.idx]);
+                lead_expect_tx(lead, &raw_full[rp.idx], (uint32_t)S::kRawBytes);
+                lead_tma_2d(lead, smem_base + (uint32_t)rp.idx * S::kRawBytes, map, cur.g * 64, (cur.tile - p.mat[mi].tile_start) * 128, &raw_full[rp.idx]);
                 rp.next();
             } while (cur.advance(p, G, GP));
-            PROF_END(0);
+            if (lane == 0) PROF_END(0);
         }
     } else if (warp == 4) {
         // ---- TMA of the digit planes: they come from the previous kernel; a slot is free when the item that used it
         // last (kXSlots back) has been multiplied
         pdl_wait();
-        if (lane == 0 && cur.start(p, blockIdx.x, G)) {
+        if (cur.start(p, blockIdx.x, G)) {
+            const uint32_t lead = elect_lead();
             RingPos<S::kXSlots> xp;
             int it = 0;
             PROF_DECL;
             do {
                 PROF_W0;
-                if (it >= S::kXSlots && !done_wait(it - S::kXSlots)) { ok = false; break; }
+                if (it >= S::kXSlots && !done_warp_wait(it - S::kXSlots)) { ok = false; break; }
                 PROF_W1;
-                mbar_arrive_expect_tx(&x_full[xp.idx], (uint32_t)S::kBBytes);
+                lead_expect_tx(lead, &x_full[xp.idx], (uint32_t)S::kBBytes);
 #pragma unroll
                 for (int j = 0; j < GP; ++j)
-                    tma_load_3d(smem_base + S::kOffX + (uint32_t)xp.idx * S::kBBytes + j * kGroupB, &map_x, (cur.g + j) * 128, 0, 0, &x_full[xp.idx]);
+                    lead_tma_3d(lead, smem_base + S::kOffX + (uint32_t)xp.idx * S::kBBytes + j * kGroupB, &map_x, (cur.g + j) * 128, 0, 0, &x_full[xp.idx]);
                 xp.next();
                 ++it;
             } while (cur.advance(p, G, GP));
-            PROF_END(1);
+            if (lane == 0) PROF_END(1);
         }
     } else if (warp == 0 || warp == 11) {
         // ---- MMA issuers: one thread of each of two warps, alternate items (their accumulators are different buffers, so
         // no order is needed between them).  Per item: the tiles are expanded, the digit planes have landed, the accumulator
         // buffer has been read out; four MMAs per group; one commit.
         const int set = warp == 0 ? 0 : 1;
-        if (lane == 0 && cur.start(p, blockIdx.x, G)) {
+        if (cur.start(p, blockIdx.x, G)) {
+            const uint32_t lead = elect_lead();
             constexpr uint32_t idesc = gemm_idesc_s8s8(128, kN);
             const uint64_t desc_a0 = gemm_smem_desc(smem_base + S::kOffA), desc_b0 = gemm_smem_desc(smem_base + S::kOffX);
             RingPos<S::kASlots> ap;
@@ -428,8 +427,13 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
             do {
                 if ((it & 1) == set) {
                     PROF_W0;
-                    if (!mbar_wait<false>(&a_ready[ap.idx], ap.phase) || !mbar_wait<false>(&x_full[xp.idx], xp.phase) ||
-                        (bp.wrapped && !mbar_wait<false>(&tmem_free[bp.idx], bp.phase ^ 1u))) {
+                    // Rings of an odd size: the slot's use before this one was the other warp's.  Until that has come and gone the
+                    // barrier's parity still is that of the use before it, and the waits below would fall through.
+                    constexpr int kBack = S::kASlots % 2 != 0 ? S::kASlots : S::kXSlots % 2 != 0 ? S::kXSlots : 0;
+                    static_assert(S::kASlots % 2 == 0 || S::kXSlots % 2 == 0 || S::kASlots == S::kXSlots, "one look back covers both rings");
+                    if (kBack > 0 && it >= kBack && !done_warp_wait(it - kBack)) { ok = false; break; }
+                    if (!warp_wait(&a_ready[ap.idx], ap.phase) || !warp_wait(&x_full[xp.idx], xp.phase) ||
+                        (bp.wrapped && !warp_wait(&tmem_free[bp.idx], bp.phase ^ 1u))) {
                         ok = false;
                         break;
                     }
@@ -441,17 +445,17 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                         if (j < ng) {
                             const uint64_t da = desc_a0 + (uint64_t)((uint32_t)ap.idx * (S::kABytes >> 4) + j * (kBtABytes >> 4));
                             const uint64_t db = desc_b0 + (uint64_t)((uint32_t)xp.idx * (S::kBBytes >> 4) + j * (kGroupB >> 4));
-                            const uint32_t d = tmem_base + (uint32_t)(bp.idx * GP * kN + j * kN);
+                            const uint32_t d = (uint32_t)(bp.idx * GP * kN + j * kN);  // (all 512 columns are this block's: they start at 0)
 #pragma unroll
-                            for (int ks = 0; ks < 4; ++ks) gemm_mma_i8(d, da + 2 * ks, db + 2 * ks, idesc, ks > 0 ? 1u : 0u);
+                            for (int ks = 0; ks < 4; ++ks) lead_mma_i8(lead, d, da + 2 * ks, db + 2 * ks, idesc, ks > 0 ? 1u : 0u);
                         }
                     }
-                    umma_commit(&done[it & (kBtDoneRing - 1)]);
+                    lead_commit(lead, &done[it & (kBtDoneRing - 1)]);
                 }
                 ap.next(); xp.next(); bp.next();
                 ++it;
             } while (cur.advance(p, G, GP));
-            PROF_END(2 + set);
+            if (lane == 0) PROF_END(2 + set);
         }
     } else if (expander) {
         // ---- weight expansion, two sets of four warps that take the items alternately.  A thread turns four 16-byte pieces
@@ -472,6 +476,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                 if ((it & 1) == set) {
                     // the raw tile has landed; the expanded slot is free (its last user, kASlots items back, has been multiplied)
                     PROF_W0;
+                    if (S::kRawSlots % 2 != 0 && it >= S::kRawSlots && !done_wait(it - S::kRawSlots)) { ok = false; break; }  // (as in the issuing warps)
                     if (!mbar_wait<false>(&raw_full[rp.idx], rp.phase) || (it >= S::kASlots && !done_wait(it - S::kASlots))) { ok = false; break; }
                     PROF_W1;
                     const unsigned char* raw = ssmem + (size_t)rp.idx * S::kRawBytes;
@@ -694,7 +699,7 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
                                                                        const __grid_constant__ CUtensorMap map_x) {
     using S = SmallShapeI8<NB>;
     constexpr int kN = 4 * NB;
-    constexpr uint32_t kTmemCols = 4 * kN;  // [unit parity][MMA thread]: 256 or 512 columns
+    constexpr uint32_t kTmemCols = 512;  // [unit parity][MMA warp] of kN columns each; all of them, so that they start at column 0
     extern __shared__ unsigned char ssmem_raw[];
     unsigned char* ssmem = ssmem_raw + ((1024u - (smem_u32(ssmem_raw) & 1023u)) & 1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(ssmem + S::kOffBars);  // [kStages] weights and digit planes have landed (two arrivals)
@@ -705,7 +710,7 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
     uint32_t* last_flag = tmem_slot + 1;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp_index();
     const int G = (p.K + 127) >> 7;  // 128-column groups (the last may be partial: TMA fills with zeros)
     if (tid == 0) {
         for (int s = 0; s < S::kStages; ++s) mbar_init(&full[s], 2);
@@ -728,6 +733,7 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
     const uint32_t smem_base = smem_u32(ssmem);
     bool ok = true;
     auto done_wait = [&](int n) { return mbar_wait<false>(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
+    auto done_warp_wait = [&](int n) { return warp_wait(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
     UnitCursor cur;
 
     if (warp == 4 || warp == 8) {
@@ -736,20 +742,21 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
         // failure whose cause was not found by reading; the single-thread form below is the one that has run every shape.)
         const bool digits = warp == 4;
         if (digits) pdl_wait();  // the digit planes come from the previous kernel; the weights never change
-        if (lane == 0 && cur.start(p, blockIdx.x, G)) {
+        if (cur.start(p, blockIdx.x, G)) {
+            const uint32_t lead = elect_lead();
             RingPos<S::kStages> sp;
             int it = 0;
             do {
-                if (it >= S::kStages && !done_wait(it - S::kStages)) { ok = false; break; }
+                if (it >= S::kStages && !done_warp_wait(it - S::kStages)) { ok = false; break; }
                 const uint32_t st = smem_base + (uint32_t)sp.idx * S::kStageBytes;
                 if (digits) {
-                    mbar_arrive_expect_tx(&full[sp.idx], (uint32_t)S::kBBytes);
-                    tma_load_3d(st + S::kWBytes, &map_x, cur.g * 128, 0, 0, &full[sp.idx]);
+                    lead_expect_tx(lead, &full[sp.idx], (uint32_t)S::kBBytes);
+                    lead_tma_3d(lead, st + S::kWBytes, &map_x, cur.g * 128, 0, 0, &full[sp.idx]);
                 } else {
                     const int mi = (p.nmat > 2 && cur.tile >= p.mat[2].tile_start) ? 2 : (p.nmat > 1 && cur.tile >= p.mat[1].tile_start) ? 1 : 0;
                     const CUtensorMap* map = mi == 0 ? &map_w0 : mi == 1 ? &map_w1 : &map_w2;
-                    mbar_arrive_expect_tx(&full[sp.idx], (uint32_t)S::kWBytes);
-                    tma_load_2d(st, map, cur.g * 128, (cur.tile - p.mat[mi].tile_start) * 128, &full[sp.idx]);
+                    lead_expect_tx(lead, &full[sp.idx], (uint32_t)S::kWBytes);
+                    lead_tma_2d(lead, st, map, cur.g * 128, (cur.tile - p.mat[mi].tile_start) * 128, &full[sp.idx]);
                 }
                 sp.next();
                 ++it;
@@ -757,28 +764,31 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
         }
     } else if (warp == 0 || warp == 11) {
         const int set = warp == 0 ? 0 : 1;
-        if (lane == 0 && cur.start(p, blockIdx.x, G)) {
+        if (cur.start(p, blockIdx.x, G)) {
+            const uint32_t lead = elect_lead();
             constexpr uint32_t idesc = gemm_idesc_s8s8(128, kN);
             const uint64_t desc_a0 = gemm_smem_desc(smem_base), desc_b0 = gemm_smem_desc(smem_base + S::kWBytes);
             RingPos<S::kStages> sp;
             int it = 0, unit_no = 0;
             bool more = true;
             while (more && ok) {
-                // accumulators of this unit: parity of the unit, then this thread's half
+                // accumulators of this unit: parity of the unit, then this warp's half
                 const int par = unit_no & 1;
-                if (unit_no >= 2 && !mbar_wait<false>(&tmem_free[par], (uint32_t)((unit_no >> 1) - 1) & 1u)) { ok = false; break; }
+                if (unit_no >= 2 && !warp_wait(&tmem_free[par], (uint32_t)((unit_no >> 1) - 1) & 1u)) { ok = false; break; }
                 tcgen05_fence_after();
-                const uint32_t d = tmem_base + (uint32_t)((par * 2 + set) * kN);
+                const uint32_t d = (uint32_t)((par * 2 + set) * kN);
                 bool first = true, same_unit = true;
                 while (same_unit) {
                     if ((it & 1) == set) {
-                        if (!mbar_wait<false>(&full[sp.idx], sp.phase)) { ok = false; break; }
+                        // (a ring of an odd size: the slot's use before this one was the other warp's, see the W4 kernel)
+                        if (S::kStages % 2 != 0 && it >= S::kStages && !done_warp_wait(it - S::kStages)) { ok = false; break; }
+                        if (!warp_wait(&full[sp.idx], sp.phase)) { ok = false; break; }
                         tcgen05_fence_after();
                         const uint64_t soff = (uint64_t)((uint32_t)sp.idx * (S::kStageBytes >> 4));
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) gemm_mma_i8(d, desc_a0 + soff + 2 * ks, desc_b0 + soff + 2 * ks, idesc, (first && ks == 0) ? 0u : 1u);
+                        for (int ks = 0; ks < 4; ++ks) lead_mma_i8(lead, d, desc_a0 + soff + 2 * ks, desc_b0 + soff + 2 * ks, idesc, (first && ks == 0) ? 0u : 1u);
                         first = false;
-                        umma_commit(&done[it & (kBtDoneRing - 1)]);
+                        lead_commit(lead, &done[it & (kBtDoneRing - 1)]);
                     }
                     sp.next();
                     ++it;
@@ -787,7 +797,7 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
                     same_unit = more && cur.u == u_before;
                 }
                 if (!ok) break;
-                umma_commit(&unit_done[par]);  // everything this thread issued for the unit (a unit has at least two groups)
+                lead_commit(lead, &unit_done[par]);  // everything this warp issued for the unit (a unit has at least two groups)
                 ++unit_no;
             }
         }
