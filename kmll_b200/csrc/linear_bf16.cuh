@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
     uint64_t* acc_free = acc_full + 2;    // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
     __shared__ unsigned int s_last;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp_index();
     const int KT = (p.K + kHKT - 1) / kHKT, kt_per = (KT + p.ksplit - 1) / p.ksplit, items = p.tiles * p.ksplit;
 
     if (tid == 0) {
@@ -400,44 +400,42 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
     pdl_wait();
     bool ok = true;
     if (warp == 0) {
-        if (lane == 0) {
-            PairRing ring(stages);
-            for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
-                const int tile = item / p.ksplit, kt0 = (item % p.ksplit) * kt_per, kt1 = min(kt0 + kt_per, KT);
-                const int row0 = (tile / p.x_tiles) * kHRows, t0 = (tile % p.x_tiles) * p.n_block;
+        const uint32_t lead = elect_lead();
+        PairRing ring(stages);
+        for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+            const int tile = item / p.ksplit, kt0 = (item % p.ksplit) * kt_per, kt1 = min(kt0 + kt_per, KT);
+            const int row0 = (tile / p.x_tiles) * kHRows, t0 = (tile % p.x_tiles) * p.n_block;
 #pragma unroll 1
-                for (int kt = kt0; kt < kt1; ++kt, ring.next()) {
-                    const int s = ring.stage;
-                    if (ring.wrapped && !mbar_wait<false>(&empty[s], ring.phase ^ 1u)) { ok = false; break; }
-                    const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
-                    mbar_arrive_expect_tx(&full[s], (uint32_t)stage_bytes);
-                    tma_load_2d(st, &map_w, kt * kHKT, row0, &full[s]);
-                    tma_load_2d(st + a_bytes, &map_x, kt * kHKT, t0, &full[s]);
-                }
+            for (int kt = kt0; kt < kt1; ++kt, ring.next()) {
+                const int s = ring.stage;
+                if (ring.wrapped && !warp_wait(&empty[s], ring.phase ^ 1u)) { ok = false; break; }
+                const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
+                lead_expect_tx(lead, &full[s], (uint32_t)stage_bytes);
+                lead_tma_2d(lead, st, &map_w, kt * kHKT, row0, &full[s]);
+                lead_tma_2d(lead, st + a_bytes, &map_x, kt * kHKT, t0, &full[s]);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            PairRing ring(stages);
-            int n = 0;
-            for (int item = blockIdx.x; ok && item < items; item += gridDim.x, ++n) {
-                const int buf = n & 1, kt0 = (item % p.ksplit) * kt_per, kt1 = min(kt0 + kt_per, KT);
-                if (n >= 2 && !mbar_wait<false>(&acc_free[buf], (uint32_t)((n >> 1) - 1) & 1u)) { ok = false; break; }
-                tcgen05_fence_after();
-                const uint32_t acc = tmem_base + (uint32_t)buf * 256u;
+        const uint32_t lead = elect_lead();
+        PairRing ring(stages);
+        int n = 0;
+        for (int item = blockIdx.x; ok && item < items; item += gridDim.x, ++n) {
+            const int buf = n & 1, kt0 = (item % p.ksplit) * kt_per, kt1 = min(kt0 + kt_per, KT);
+            if (n >= 2 && !warp_wait(&acc_free[buf], (uint32_t)((n >> 1) - 1) & 1u)) { ok = false; break; }
+            tcgen05_fence_after();
+            const uint32_t acc = (uint32_t)buf * 256u;  // (all 512 columns are this block's: they start at 0)
 #pragma unroll 1
-                for (int kt = kt0; kt < kt1; ++kt, ring.next()) {
-                    const int s = ring.stage;
-                    if (!mbar_wait<false>(&full[s], ring.phase)) { ok = false; break; }
-                    tcgen05_fence_after();
-                    const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
+            for (int kt = kt0; kt < kt1; ++kt, ring.next()) {
+                const int s = ring.stage;
+                if (!warp_wait(&full[s], ring.phase)) { ok = false; break; }
+                tcgen05_fence_after();
+                const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
+                const uint64_t da = gemm_smem_desc(st), db = gemm_smem_desc(st + a_bytes);
 #pragma unroll
-                    for (int ks = 0; ks < kHKT / 16; ++ks)
-                        gemm_mma_f16(acc, gemm_smem_desc(st + ks * 32), gemm_smem_desc(st + a_bytes + ks * 32), idesc, (kt > kt0 || ks > 0) ? 1u : 0u);
-                    umma_commit(&empty[s]);
-                }
-                if (ok) umma_commit(&acc_full[buf]);
+                for (int ks = 0; ks < kHKT / 16; ++ks) lead_mma_f16(lead, acc, da + 2 * ks, db + 2 * ks, idesc, (kt > kt0 || ks > 0) ? 1u : 0u);
+                lead_commit(lead, &empty[s]);
             }
+            if (ok) lead_commit(lead, &acc_full[buf]);
         }
     } else {
         const int q = warp & 3, half = (warp - 2) >> 2;  // lane quarter this warp may read; which half of the columns
@@ -531,9 +529,8 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
 // ---- more than 256 rows of x: pairs of multiprocessors ------------------------------------------------------------------------
 // The same contraction as linear_gemm_bf16_kernel on tcgen05.mma.cta_group::2: 256 weight rows (128 per block of a cluster of two)
 // against up to 256 rows of x, half of them in each block's shared memory - 32 KB per 64-column k-tile and block instead of 48.
-// Bound by the tensor cores.  What kept the one-block kernel at 0.43 of their rate on a prompt was its issuing thread: a commit holds it
-// for ~500 cycles, as long as the four MMAs of a k-tile take.  So two threads issue, even and odd k-tiles into an accumulator each;
-// the drain warps add the two in registers, give both back and store while the next unit's MMAs run (linear_gemm_pair.cuh has the
+// Bound by the tensor cores.  Two warps issue, even and odd k-tiles into an accumulator each, so that one's waits and commits run behind
+// the other's MMAs; the drain warps add the two in registers, give both back and store while the next unit's MMAs run (linear_gemm_pair.cuh has the
 // same structure and the reasons for its barriers).  Roles of a block: warp 0 TMA of x, warp 2 TMA of the weights,
 // warps 1 and 3 the issuers in the leader block; in the other block warp 1 tells the leader that a stage has landed;
 // warps 4-11 drain and store.  Registers: 56 + 2 x 224 = 3 x 168 per thread of a warpgroup.
@@ -607,7 +604,7 @@ __global__ void __launch_bounds__(kHPairThreads, 1) linear_gemm_bf16_pair_kernel
     uint64_t* acc_full = empty + stages;    // [2], in each block
     uint64_t* acc_empty = acc_full + 2;     // [2], in the leader: drained by both blocks' eight warps
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp_index();
     const int rank = (int)(blockIdx.x & 1u), cluster = (int)(blockIdx.x >> 1), n_clusters = (int)(gridDim.x >> 1);
     const int KT = (p.K + kHKT - 1) / kHKT;
 
@@ -631,60 +628,63 @@ __global__ void __launch_bounds__(kHPairThreads, 1) linear_gemm_bf16_pair_kernel
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         pdl_wait();
-        if (lane == 0) {
-            PairRing ring(stages);
-            if (warp == 0 || warp == 2) {
-                for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters) {
-                    const int rt = unit / p.x_tiles, row0 = rt * 256 + rank * 128, t0 = (unit - rt * p.x_tiles) * p.n_block + rank * n_half;
+        const uint32_t lead = elect_lead();
+        PairRing ring(stages);
+        if (warp == 0 || warp == 2) {
+            for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters) {
+                const int rt = unit / p.x_tiles, row0 = rt * 256 + rank * 128, t0 = (unit - rt * p.x_tiles) * p.n_block + rank * n_half;
 #pragma unroll 1
-                    for (int kt = 0; kt < KT; ++kt, ring.next()) {
-                        const int s = ring.stage;
-                        if (ring.wrapped && !mbar_wait<false>(&empty[s], ring.phase ^ 1u)) { ok = false; break; }
-                        const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
-                        if (warp == 0) {
-                            mbar_arrive_expect_tx(&full[s], (uint32_t)b_bytes);
-                            tma_load_2d(st + a_bytes, &map_x, kt * kHKT, t0, &full[s]);
-                        } else {
-                            mbar_arrive_expect_tx(&full[s], (uint32_t)a_bytes);
-                            tma_load_2d(st, &map_w, kt * kHKT, row0, &full[s]);
-                        }
+                for (int kt = 0; kt < KT; ++kt, ring.next()) {
+                    const int s = ring.stage;
+                    if (ring.wrapped && !warp_wait(&empty[s], ring.phase ^ 1u)) { ok = false; break; }
+                    const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
+                    if (warp == 0) {
+                        lead_expect_tx(lead, &full[s], (uint32_t)b_bytes);
+                        lead_tma_2d(lead, st + a_bytes, &map_x, kt * kHKT, t0, &full[s]);
+                    } else {
+                        lead_expect_tx(lead, &full[s], (uint32_t)a_bytes);
+                        lead_tma_2d(lead, st, &map_w, kt * kHKT, row0, &full[s]);
                     }
                 }
-                // nothing of this block's copies, and no arrival on its barriers, is in flight when it reaches the end
-                for (int j = 0; j < stages; ++j, ring.next())
-                    if (ring.wrapped && !mbar_wait<false>(ok ? &empty[ring.stage] : &full[ring.stage], ring.phase ^ 1u)) { ok = false; break; }
-            } else if (rank == 0) {
-                const uint32_t idesc = gemm_idesc_bf16(256, p.n_block);
-                const int own = warp >> 1;
-                const uint32_t dst = tmem_base + (uint32_t)own * 256u;
-                uint32_t uses = 0;
-                for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters) {
+            }
+            // nothing of this block's copies, and no arrival on its barriers, is in flight when it reaches the end
+            for (int j = 0; j < stages; ++j, ring.next())
+                if (ring.wrapped && !warp_wait(ok ? &empty[ring.stage] : &full[ring.stage], ring.phase ^ 1u)) { ok = false; break; }
+        } else if (rank == 0) {
+            const uint32_t idesc = gemm_idesc_bf16(256, p.n_block);
+            const int own = warp >> 1;
+            const uint32_t dst = (uint32_t)own * 256u;  // (all 512 columns are this pair's: they start at 0)
+            uint32_t uses = 0;
+            for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters) {
 #pragma unroll 1
-                    for (int kt = 0; kt < KT; ++kt, ring.next()) {
-                        if ((kt & 1) != own) continue;
-                        const int s = ring.stage;
-                        if (kt < 2 && uses > 0 && !mbar_wait<false>(&acc_empty[own], (uses - 1) & 1u)) { ok = false; break; }
-                        if (!mbar_wait<false>(&full[s], ring.phase) || !mbar_wait<false>(&peer_full[s], ring.phase)) { ok = false; break; }
-                        tcgen05_fence_after();
-                        const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
-                        const uint64_t da = gemm_smem_desc(st), db = gemm_smem_desc(st + a_bytes);
+                for (int kt = 0; kt < KT; ++kt, ring.next()) {
+                    if ((kt & 1) != own) continue;
+                    const int s = ring.stage;
+                    if (kt < 2 && uses > 0 && !warp_wait(&acc_empty[own], (uses - 1) & 1u)) { ok = false; break; }
+                    // (the stage's use before this one may have been the other warp's: linear_gemm_pair.cuh)
+                    if (ring.wrapped && !warp_wait(&empty[s], ring.phase ^ 1u)) { ok = false; break; }
+                    if (!warp_wait(&full[s], ring.phase) || !warp_wait(&peer_full[s], ring.phase)) { ok = false; break; }
+                    tcgen05_fence_after();
+                    const uint32_t st = smem_base + (uint32_t)s * stage_bytes;
+                    const uint64_t da = gemm_smem_desc(st), db = gemm_smem_desc(st + a_bytes);
 #pragma unroll
-                        for (int ks = 0; ks < kHKT / 16; ++ks) pair_mma_f16(dst, da + 2 * ks, db + 2 * ks, idesc, (kt > 1 || ks > 0) ? 1u : 0u);
-                        pair_commit(&empty[s]);
-                        if (kt + 2 >= KT) {
-                            pair_commit(&acc_full[own]);
-                            ++uses;
-                        }
+                    for (int ks = 0; ks < kHKT / 16; ++ks) pair_mma_f16(lead, dst, da + 2 * ks, db + 2 * ks, idesc, (kt > 1 || ks > 0) ? 1u : 0u);
+                    pair_commit(lead, &empty[s]);
+                    if (kt + 2 >= KT) {
+                        pair_commit(lead, &acc_full[own]);
+                        ++uses;
                     }
                 }
-            } else if (warp == 1) {
+            }
+        } else if (warp == 1) {
+            if (lane == 0)
                 for (int unit = cluster; unit < p.tiles && ok; unit += n_clusters)
 #pragma unroll 1
                     for (int kt = 0; kt < KT; ++kt, ring.next()) {
                         if (!mbar_wait<false>(&full[ring.stage], ring.phase)) { ok = false; break; }
                         mbar_arrive_leader(&peer_full[ring.stage]);
                     }
-            }
+            __syncwarp();
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");

@@ -138,22 +138,4 @@ __global__ void __launch_bounds__(512, 2) split_rows_kernel(const float* __restr
     if (threadIdx.x == 0) inv_xscale[m] = inv_scale;
 }
 
-// ---- TMA helpers ----------------------------------------------------------------------------------------------------
-__device__ inline void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// 2-D tiled TMA load into this block's shared memory (no multicast), completion on an mbarrier
-__device__ inline void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// 3-D tiled TMA load (inner, row, plane)
-__device__ inline void tma_load_3d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 }  // namespace kmll

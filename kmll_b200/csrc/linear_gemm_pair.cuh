@@ -17,13 +17,13 @@
 //
 // Measured in a graph of ten calls, split of x included (one block per 128 x 256 tile with three / two MMAs per k-step before): W4 2048 x 14336 x
 // 4096 612 -> 355 us (677 TFLOP/s useful, 1353 of MMA work), RS-I8 587 -> 328, W4 300 x 18944 x 3584 131 -> 73, 64 x 14336 x 4096 53 -> 29,
-// RS-I8 333 x 4096 x 4096 74 -> 31, W4 33 x 3584 x 3584 28 -> 17.  Error against 64 bits 8.4e-6 -> 2.6e-7 (W4: no second weight plane).
+// RS-I8 333 x 4096 x 4096 74 -> 31, W4 33 x 3584 x 3584 28 -> 17.  Issued by whole warps (tcgen05.cuh) instead of single threads: W4 2048 x 14336 x
+// 4096 362 -> 334, 300 x 18944 x 3584 72 -> 62, 200 x 28672 x 4096 97 -> 90, 200 x 4096 x 14336 56 -> 50, RS-I8 333 x 4096 x 14336 82 -> 76.  Error against 64 bits 8.4e-6 -> 2.6e-7 (W4: no second weight plane).
 //
 // Roles of a block (512 threads, one block per SM, persistent over units = (weight row tile, x block, k-split)):
 //   warp 0      TMA of x: both planes of n_block / 2 rows, one 3-D box per 64-column k-tile
-//   warp 1, 3   tensor memory (warp 1); in the leader block (rank 0) one thread of each issues the MMAs of one accumulator.  A
-//               commit holds its thread for ~500 cycles, longer than the tensor cores' queue: with one issuer a k-tile of 256
-//               rows took 1540 cycles, with two 1070 (1080 at the nominal MMA rate)
+//   warp 1, 3   tensor memory (warp 1); in the leader block (rank 0) each issues the MMAs of one accumulator, so that one's waits and
+//               commits run behind the other's MMAs
 //   warp 2      TMA of the raw weight tile (ahead of the grid dependency: weights are constants)
 //   warps 4-7   expand raw weights to swizzled binary16 rows of the MMA operand
 //   warps 8-15  drain accumulators, epilogue
@@ -65,17 +65,19 @@ __device__ inline void mbar_arrive_leader(uint64_t* bar) {
         "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}"
         ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ inline void pair_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// (issued by the elected lane of a converged warp, see tcgen05.cuh)
+__device__ inline void pair_mma_f16(uint32_t lead, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
 // completion of all earlier MMAs of this thread, signalled on the same barrier of both blocks
-__device__ inline void pair_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+__device__ inline void pair_commit(uint32_t lead, uint64_t* bar) {
+    asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+                 "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3), "r"(lead) : "memory");
 }
 // two f32 sums: acc += s * (lo, hi)
 __device__ inline void fma_pair(unsigned long long& acc, unsigned long long s2, uint32_t lo, uint32_t hi) {
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp_index();
     const int rank = (int)(blockIdx.x & 1u), cluster = (int)(blockIdx.x >> 1), n_clusters = (int)(gridDim.x >> 1);
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 2); mbar_init(&a_ready[s], 8); mbar_init(&empty[s], 1); }
@@ -200,69 +202,68 @@ __global__ void __launch_bounds__(kPThreads, 1) linear_gemm_pair_kernel(const Pa
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (warp != 2) pdl_wait();  // the planes of x come from the previous kernel
+        const uint32_t lead = elect_lead();
+        PairRing ring(stages);
         if (warp == 0 || warp == 2) {
-            if (lane == 0) {
-                PairRing ring(stages);
-                for (int unit = cluster; unit < p.units && ok; unit += n_clusters) {
-                    const PairUnit u = pair_unit<W4>(p, unit, rank);
-                    const CUtensorMap* mw = u.mat == 0 ? &map_w0 : u.mat == 1 ? &map_w1 : &map_w2;
+            for (int unit = cluster; unit < p.units && ok; unit += n_clusters) {
+                const PairUnit u = pair_unit<W4>(p, unit, rank);
+                const CUtensorMap* mw = u.mat == 0 ? &map_w0 : u.mat == 1 ? &map_w1 : &map_w2;
 #pragma unroll 1
-                    for (int kt = 0; kt < u.KT; ++kt, ring.next()) {
-                        const int stage = ring.stage;
-                        if (ring.wrapped && !mbar_wait<false>(&empty[stage], ring.phase ^ 1u)) { ok = false; break; }
-                        const uint32_t st = smem_base + (uint32_t)stage * stage_bytes;
-                        const int k = (u.kt0 + kt) * kGKT;
-                        if (warp == 0) {
-                            mbar_arrive_expect_tx(&full[stage], (uint32_t)(2 * b_bytes));
-                            tma_load_3d(st + kABytes, &map_x, k, u.m0 + rank * n_half, 0, &full[stage]);
-                        } else {
-                            mbar_arrive_expect_tx(&full[stage], (uint32_t)kRawBytes);
-                            tma_load_2d(st + kABytes + 2 * b_bytes, mw, W4 ? k / 2 : k, u.row0, &full[stage]);
-                        }
+                for (int kt = 0; kt < u.KT; ++kt, ring.next()) {
+                    const int stage = ring.stage;
+                    if (ring.wrapped && !warp_wait(&empty[stage], ring.phase ^ 1u)) { ok = false; break; }
+                    const uint32_t st = smem_base + (uint32_t)stage * stage_bytes;
+                    const int k = (u.kt0 + kt) * kGKT;
+                    if (warp == 0) {
+                        lead_expect_tx(lead, &full[stage], (uint32_t)(2 * b_bytes));
+                        lead_tma_3d(lead, st + kABytes, &map_x, k, u.m0 + rank * n_half, 0, &full[stage]);
+                    } else {
+                        lead_expect_tx(lead, &full[stage], (uint32_t)kRawBytes);
+                        lead_tma_2d(lead, st + kABytes + 2 * b_bytes, mw, W4 ? k / 2 : k, u.row0, &full[stage]);
                     }
                 }
-                // nothing of this block's copies, and no arrival on its barriers, is in flight when it reaches the end
-                for (int j = 0; j < stages; ++j, ring.next())
-                    if (ring.wrapped && !mbar_wait<false>(ok ? &empty[ring.stage] : &full[ring.stage], ring.phase ^ 1u)) { ok = false; break; }
             }
+            // nothing of this block's copies, and no arrival on its barriers, is in flight when it reaches the end
+            for (int j = 0; j < stages; ++j, ring.next())
+                if (ring.wrapped && !warp_wait(ok ? &empty[ring.stage] : &full[ring.stage], ring.phase ^ 1u)) { ok = false; break; }
         } else if (rank == 0) {
-            // ---- two MMA issuers, one per accumulator: warp 1 the even spans, warp 3 the odd ones (a span: W4 the two k-tiles of
+            // ---- two issuing warps, one per accumulator: warp 1 the even spans, warp 3 the odd ones (a span: W4 the two k-tiles of
             // a group, RS-I8 every other k-tile of a unit)
-            if (lane == 0) {
-                const uint32_t idesc = gemm_idesc_f16(256, WIDE ? 2 * p.n_block : p.n_block);
-                const int own = warp >> 1;
-                const uint32_t dst = tmem_base + (uint32_t)own * 256u;
-                PairRing ring(stages);
-                int span0 = 0;
-                uint32_t uses = 0, acc = 0u;
-                for (int unit = cluster; unit < p.units && ok; unit += n_clusters) {
-                    const int KT = pair_unit<W4>(p, unit, 0).KT;
+            const uint32_t idesc = gemm_idesc_f16(256, WIDE ? 2 * p.n_block : p.n_block);
+            const int own = warp >> 1;
+            const uint32_t dst = (uint32_t)own * 256u;  // (all 512 columns are this pair's: they start at 0)
+            int span0 = 0;
+            uint32_t uses = 0, acc = 0u;
+            for (int unit = cluster; unit < p.units && ok; unit += n_clusters) {
+                const int KT = pair_unit<W4>(p, unit, 0).KT;
 #pragma unroll 1
-                    for (int kt = 0; kt < KT; ++kt, ring.next()) {
-                        if (((W4 ? span0 + (kt >> 1) : kt) & 1) != own) continue;
-                        const int stage = ring.stage;
-                        if (W4 ? (kt & 1) == 0 : kt < 2) {  // first k-tile of a span
-                            if (uses > 0 && !mbar_wait<false>(&acc_empty[own], (uses - 1) & 1u)) { ok = false; break; }
-                            acc = 0u;
-                        }
-                        if (!mbar_wait<false>(&a_ready[stage], ring.phase)) { ok = false; break; }
-                        tcgen05_fence_after();
-                        const uint32_t st = smem_base + (uint32_t)stage * stage_bytes;
-                        const uint64_t da = gemm_smem_desc(st), dh = gemm_smem_desc(st + kABytes), dl = gemm_smem_desc(st + kABytes + b_bytes);
-#pragma unroll
-                        for (int ks = 0; ks < kGKT / 16; ++ks) {  // 32 bytes = 2 descriptor units per k-step
-                            pair_mma_f16(dst, da + 2 * ks, dh + 2 * ks, idesc, acc);
-                            if (!WIDE) pair_mma_f16(dst, da + 2 * ks, dl + 2 * ks, idesc, 1u);
-                            acc = 1u;
-                        }
-                        pair_commit(&empty[stage]);
-                        if (W4 ? (kt & 1) == 1 : kt + 2 >= KT) {  // last one
-                            pair_commit(&acc_full[own]);
-                            ++uses;
-                        }
+                for (int kt = 0; kt < KT; ++kt, ring.next()) {
+                    if (((W4 ? span0 + (kt >> 1) : kt) & 1) != own) continue;
+                    const int stage = ring.stage;
+                    if (W4 ? (kt & 1) == 0 : kt < 2) {  // first k-tile of a span
+                        if (uses > 0 && !warp_wait(&acc_empty[own], (uses - 1) & 1u)) { ok = false; break; }
+                        acc = 0u;
                     }
-                    span0 += KT >> 1;
+                    // an odd ring: the stage's use before this one was the other warp's; before it has come, the parity below is that
+                    // of the use before it
+                    if ((stages & 1) != 0 && ring.wrapped && !warp_wait(&empty[stage], ring.phase ^ 1u)) { ok = false; break; }
+                    if (!warp_wait(&a_ready[stage], ring.phase)) { ok = false; break; }
+                    tcgen05_fence_after();
+                    const uint32_t st = smem_base + (uint32_t)stage * stage_bytes;
+                    const uint64_t da = gemm_smem_desc(st), dh = gemm_smem_desc(st + kABytes), dl = gemm_smem_desc(st + kABytes + b_bytes);
+#pragma unroll
+                    for (int ks = 0; ks < kGKT / 16; ++ks) {  // 32 bytes = 2 descriptor units per k-step
+                        pair_mma_f16(lead, dst, da + 2 * ks, dh + 2 * ks, idesc, acc);
+                        if (!WIDE) pair_mma_f16(lead, dst, da + 2 * ks, dl + 2 * ks, idesc, 1u);
+                        acc = 1u;
+                    }
+                    pair_commit(lead, &empty[stage]);
+                    if (W4 ? (kt & 1) == 1 : kt + 2 >= KT) {  // last one
+                        pair_commit(lead, &acc_full[own]);
+                        ++uses;
+                    }
                 }
+                span0 += KT >> 1;
             }
         }
     } else if (warp < 8) {

@@ -38,9 +38,6 @@ __device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if ((unsigned long long)(clock64() - t0) > kWaitLimitTicks) return false;
     }
 }
-__device__ inline void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ inline void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ inline void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ inline void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -56,13 +53,6 @@ __host__ __device__ constexpr uint32_t gemm_idesc_f16(int m, int n) {
 // the same with A = B = bf16
 __host__ __device__ constexpr uint32_t gemm_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-__device__ inline void gemm_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
 }
 // ---- issue by a converged warp -------------------------------------------------------------------------------------------
 // A role that issues MMAs, commits or copies walks its loops as a whole warp, and one elected lane's predicate does the issuing.  The
