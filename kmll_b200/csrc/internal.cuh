@@ -356,6 +356,8 @@ size_t latent_decode_work_floats(int heads, int rank, int rot, int span);
 bool latent_decode_ok(const LatentArgs& a);
 int latent_attention_decode(cudaStream_t stream, const LatentArgs& a);  // T = 1, bf16 cache; writes the cache row itself
 bool latent_prefill_ok(const LatentArgs& a);
+bool latent_prompt_serves(const LatentArgs& a);  // the form of prompt_attention.cu
+int latent_prompt_launch(cudaStream_t stream, const LatentArgs& a);
 int latent_attention_prefill(cudaStream_t stream, const LatentArgs& a); // after latent_write_cache and the expansion
 
 // ---- grouped softmax attention (grouped_attention.cu) --------------------------------------------------------------------

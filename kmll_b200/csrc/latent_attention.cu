@@ -700,6 +700,7 @@ int latent_attention_decode(cudaStream_t stream, const LatentArgs& a) {
 bool latent_prefill_ok(const LatentArgs& a) { return !a.in_f32 && !a.cache_f32 && round_up(a.dim, 8) + a.rot <= 256 && a.vdim <= 128; }
 int latent_attention_prefill(cudaStream_t stream, const LatentArgs& a) {
     if (!latent_prefill_ok(a)) return fail(KMLL_ERR_UNSUPPORTED, "latent attention: no prompt form for head sizes %d + %d, %d", a.dim, a.rot, a.vdim);
+    if (latent_prompt_serves(a)) return latent_prompt_launch(stream, a);
     const int dq = round_up(a.dim, 8) + a.rot;
     if (a.vdim <= 64) return dq <= 64 ? run_prefill<64, 64>(stream, a) : dq <= 128 ? run_prefill<128, 64>(stream, a) : dq <= 192 ? run_prefill<192, 64>(stream, a) : run_prefill<256, 64>(stream, a);
     return dq <= 64 ? run_prefill<64, 128>(stream, a) : dq <= 128 ? run_prefill<128, 128>(stream, a) : dq <= 192 ? run_prefill<192, 128>(stream, a) : run_prefill<256, 128>(stream, a);

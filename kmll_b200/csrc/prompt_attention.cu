@@ -355,7 +355,84 @@ __global__ void __launch_bounds__(kPaThreads, 1) prompt_attention_kernel(const f
     prompt_attention_block(src, rg, out + (size_t)r0 * src.q_len + (size_t)head * HD, src.q_len);
 }
 
+// ---- latent attention: heads of 128 + 64 rotated entries, values of 128; keys and values from the expanded latents, the rotated key part
+// (one for all heads) from the cache --------------------------------------------------------------------------------------------
+struct LatentSource {
+    static constexpr int kDQ = 192, kDV = 128, kNQ = 1, kNK = 1;
+    const uint16_t* q;    // first query row of the block, this head: 128 entries, then 64 unrotated ones
+    size_t ld;
+    const float2* turns;  // of the first row's position, [position][32]
+    const CUtensorMap *map_ex, *map_cache;
+    int kcol, vcol, kr_off, first;
+    __device__ void q_planes(int r, int c8, uint4 (&pl)[1]) const {
+        const uint16_t* row = q + (size_t)r * ld;
+        if (c8 < 16) {
+            pl[0] = *reinterpret_cast<const uint4*>(row + c8 * 8);
+            return;
+        }
+        const bool second = c8 >= 20;  // entry j of the first half turns with entry j + 32
+        const int j0 = (c8 - (second ? 20 : 16)) * 8;
+        const uint4 ua = *reinterpret_cast<const uint4*>(row + 128 + j0), va = *reinterpret_cast<const uint4*>(row + 160 + j0);
+        const uint32_t uu[4] = {ua.x, ua.y, ua.z, ua.w}, vv[4] = {va.x, va.y, va.z, va.w};
+        const float2* cs = turns + (size_t)r * 32 + j0;
+        uint32_t y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float u = bf16_bits_to_f32((uint16_t)(uu[i >> 1] >> (16 * (i & 1)))), v = bf16_bits_to_f32((uint16_t)(vv[i >> 1] >> (16 * (i & 1))));
+            const float2 f = cs[i];
+            y[i] = f32_to_bf16_bits(second ? v * f.x + u * f.y : u * f.x - v * f.y);
+        }
+        pl[0] = make_uint4(y[0] | (y[1] << 16), y[2] | (y[3] << 16), y[4] | (y[5] << 16), y[6] | (y[7] << 16));
+    }
+    // (positions in front of the first expanded one are rows before the map's: zeros)
+    __device__ void load_k(uint32_t lead, int box, int pos, uint32_t dst, uint64_t* bar) const {
+        if (box < 2) lead_tma_2d(lead, dst, map_ex, kcol + box * 64, pos - first, bar);
+        else lead_tma_2d(lead, dst, map_cache, kr_off, pos, bar);
+    }
+    __device__ void load_v(uint32_t lead, int box, int pos, uint32_t dst, uint64_t* bar) const { lead_tma_2d(lead, dst, map_ex, vcol + box * 64, pos - first, bar); }
+};
+
+__global__ void __launch_bounds__(kPaThreads, 1) latent_prompt_kernel(const LatentArgs a, const __grid_constant__ CUtensorMap map_ex, const __grid_constant__ CUtensorMap map_cache) {
+    const int head = blockIdx.x, r0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kPaRows;
+    LatentSource src;
+    src.ld = (size_t)a.ld;
+    src.q = static_cast<const uint16_t*>(a.in) + (size_t)r0 * a.ld + a.q_off + (size_t)head * 192;
+    src.turns = a.table + (size_t)(a.pos0 + r0) * 32;
+    src.map_ex = &map_ex;
+    src.map_cache = &map_cache;
+    src.kcol = head * 128;
+    src.vcol = a.heads * 128 + head * 128;
+    src.kr_off = a.kr_off;
+    src.first = a.first;
+    PaRange rg;
+    rg.pos0 = a.pos0 + r0;
+    rg.live_rows = min(kPaRows, a.T - r0);
+    rg.first = a.window > 0 ? max(0, rg.pos0 - a.window + 1) : 0;
+    rg.last = rg.pos0 + rg.live_rows - 1;
+    rg.window = a.window;
+    rg.scale2 = 1.4426950408889634f * a.scale;
+    prompt_attention_block(src, rg, a.out + (size_t)r0 * a.ldo + (size_t)head * 128, (size_t)a.ldo);
+}
+
 }  // namespace
+
+// Whole heads of 128 + 64 / 128 in aligned bf16 rows; a positive scale (the row maximum is taken before it is applied).
+bool latent_prompt_serves(const LatentArgs& a) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.cache) | reinterpret_cast<uintptr_t>(a.expanded) | reinterpret_cast<uintptr_t>(a.out);
+    return !a.in_f32 && !a.cache_f32 && a.dim == 128 && a.rot == 64 && a.vdim == 128 && a.scale > 0.0f && (bits & 15u) == 0 &&
+           ((a.ld | a.q_off | a.lde | a.pitch | a.kr_off) & 7) == 0 && (a.ldo & 3) == 0 && a.lde >= a.heads * 256;
+}
+
+int latent_prompt_launch(cudaStream_t stream, const LatentArgs& a) {
+    CUtensorMap map_ex, map_cache;
+    KMLL_TRY_RC(make_map_bf16_rows(&map_ex, a.expanded, (uint64_t)a.heads * 256, (uint64_t)(a.pos0 + a.T - a.first), (uint64_t)a.lde * 2, kPaKeys));
+    KMLL_TRY_RC(make_map_bf16_rows(&map_cache, a.cache, (uint64_t)a.pitch, (uint64_t)(a.pos0 + a.T), (uint64_t)a.pitch * 2, kPaKeys));
+    cudaError_t e = allow_all_dynamic_smem(latent_prompt_kernel);
+    if (e == cudaSuccess)
+        e = launch(latent_prompt_kernel, dim3(a.heads, (a.T + kPaRows - 1) / kPaRows), dim3(kPaThreads), PaShape<192, 128, 1, 1>::kSmemBytes, stream, true, a, map_ex, map_cache);
+    if (e != cudaSuccess) return fail(KMLL_ERR_CUDA, "latent attention (prompt): %s", cudaGetErrorString(e));
+    return KMLL_OK;
+}
 
 bool prompt_attention_serves(const void* q, const void* k, const void* v, const void* out, int prompt_len, int n_heads, int head_dim) {
     (void)prompt_len;

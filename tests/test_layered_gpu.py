@@ -226,6 +226,21 @@ def test_other_sizes(cuda, name, dtype):
     m.close()
 
 
+@pytest.mark.parametrize("window", [1, 100, 128, 300, 512])
+def test_latent_prompt_over_tiles(cuda, window):
+    """Latent heads of 128 + 64 and 128 (attention on tensor memory): every position of a prompt of several 128-row blocks and 128-key
+    tiles, in one portion and in portions that start and end inside both, windows that start inside a tile and that see all."""
+    n = 390
+    cfg = config([latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=64, window=window, scale=192 ** -0.5)], width=128, positions=512)
+    m = Model(cfg, "bfloat16", seed=window)
+    tokens = m.tokens(n)
+    want = m.oracle(tokens)
+    check(m.run(tokens), want, "bfloat16", 1.5)
+    check(m.run(tokens, [127, 2, 129, 132]), want, "bfloat16", 1.5)
+    check(m.run(tokens, [5, 256, 129]), want, "bfloat16", 1.5)
+    m.close()
+
+
 # ---- one key that stands out ---------------------------------------------------------------------------------------------------
 MARK, ASK = 1, 2  # token MARK leaves a key that token ASK looks for
 
