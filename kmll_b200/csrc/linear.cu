@@ -1067,9 +1067,9 @@ static int run_gemm_small(int fmt, cudaStream_t stream, const float* x, const fl
     int tiles = 0;
     for (int i = 0; i < kBtMaxMats; ++i) {
         const int src = i < nmat ? i : 0;  // unused tensor-map slots repeat the first matrix
-        if (w4)  // nibbles of one group per row and box, or of two groups in the 128-byte swizzle
+        if (w4)  // nibbles of one group per row and box, or of two groups, in the swizzle of that width
             KMLL_TRY_RC(make_map_2d(&map_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w[src], (uint64_t)K / 2, (uint64_t)rows[src], (uint64_t)K / 2, 64 * gp, 128,
-                                    gp == 2 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE));
+                                    gp == 2 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B));
         else  // int8 rows as they lie: 128 rows x 128 bytes, 128-byte swizzle - the MMA reads the tile TMA wrote
             KMLL_TRY_RC(make_map_2d(&map_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w[src], (uint64_t)K, (uint64_t)rows[src], (uint64_t)K, 128, 128,
                                     CU_TENSOR_MAP_SWIZZLE_128B));

@@ -21,11 +21,12 @@
 // 4096 x 14336 18.8 / 17.5, 32 rows and 4096 x 4096 19.6 / 15.3.
 //   * raw weight tiles (128 rows x 64 bytes of nibbles, TMA by warp 8): 12 slots (7 with 32 rows of x) - they wait out the HBM latency;
 //   * digit planes of the same 128 columns (one 3-D TMA box, 128-byte swizzle, warp 4): 5 or 6 slots - L2 latency;
-//   * signed-byte weight tiles in the swizzled K-major layout the MMA reads: 4 slots, written by two sets of four
+//   * signed-byte weight tiles in tensor memory (lane = weight row, a column = four bytes of K): 4 slots, written by two sets of four
 //     expanding warps (seven integer instructions per word; the even and odd columns of a word come out as two runs, the
-//     digit planes are stored in that column order);
-//   * accumulators in tensor memory: 8 (16 rows of x) or 4 (32 rows) buffers of 4 n_block columns.
-//   The elected lane of each of warps 0 and 11 waits for a group's `a_ready` barrier, its digit planes and its accumulator
+//     digit planes are stored in that column order).  In shared memory they were written and read through the port that the
+//     raw tiles and the digit planes also cross: 128 KB per two groups and 16 rows of x, 1000 of the 1450 cycles those took;
+//   * accumulators in tensor memory: a buffer of 4 n_block columns per group for each draining set.
+//   The elected lane of each issuing warp waits for a group's `a_ready` barrier, its digit planes and its accumulator
 //   buffer, issues the four MMAs (M = 128 weight rows, N = 4 n_block digit columns, K = 32 bytes each) and one commit on a
 //   ring of 16 `done` barriers; the producers, the expanding warps and the draining warps all derive what they wait for
 //   from that ring (the slot they want to refill was last used by the group `ring size` back).  Two sets of four warps
@@ -44,9 +45,9 @@ namespace kmll {
 
 constexpr int kBtSetWarps = 4;     // warps per expanding set and per draining set; two sets of each take the groups alternately
 constexpr int kBtThreads = 20 * 32;  // roles by warp: see linear_gemm_small_kernel
-constexpr int kBtABytes = 128 * 128;  // expanded weight tile: 128 rows x 128 signed bytes
+constexpr int kBtACols = 32;       // tensor-memory columns of an expanded weight tile: 128 rows x 128 signed bytes
 constexpr int kBtRawBytes = 128 * 64;
-constexpr int kBtASlots = 4;   // expanded-tile slots with one group per item
+constexpr int kBtASlots = 4;   // expanded-tile slots (even: a slot always belongs to the same set of warps)
 constexpr int kBtDoneRing = 16;    // `done` barriers; a power of two above every ring size
 constexpr int kBtMaxUnits = 592;   // split-K partial tiles the workspace holds (four per multiprocessor)
 constexpr int kBtMaxMats = 3;
@@ -224,28 +225,31 @@ struct RingPos {
     }
 };
 
-// Ring sizes and the shared-memory plan: [raw slots | digit slots | expanded slots | hand-over | barriers].  An *item* - what
+// Ring sizes, the shared-memory plan [raw slots | digit slots | hand-over | barriers] and the tensor-memory plan [accumulator buffers |
+// expanded slots].  An *item* - what
 // moves through the rings and what every role handles per pass - is GP consecutive 128-column groups: 2 with 16 rows of x
 // (every role's pass costs about the same however much it carries, so two groups per pass halve the cost per byte), 1 with
-// 32 rows (tensor memory holds 512 columns: four buffers of 4 x 32).
+// 32 rows.  All rings that two sets of warps use alternately are even, so that a slot has one user: with an odd ring a set would
+// see every second use of a slot only, and a wait by parity could take the use before last for the last one.
 template <int NB, int GP>
 struct SmallShape {
     static constexpr int kBBytes = GP * 4 * NB * 128;      // the four digit planes of the item's groups
-    static constexpr int kABytes = GP * kBtABytes;         // expanded tiles of the item
     static constexpr int kRawBytes = GP * kBtRawBytes;     // 128 rows x 64 GP bytes of nibbles
-    static constexpr int kASlots = GP == 2 ? 3 : kBtASlots;
-    static constexpr int kXSlots = GP == 2 ? 3 : (NB == 16 ? 6 : 5);
-    static constexpr int kBufs = 512 / (GP * 4 * NB);      // accumulator buffers of GP x 4 NB columns
+    static constexpr int kASlots = kBtASlots, kACols = GP * kBtACols;
+    static constexpr int kXSlots = 4;
+    static constexpr int kBufs = 2;                        // accumulator buffers of GP x 4 NB columns
+    static constexpr int kTmemA = kBufs * GP * 4 * NB;     // first column of the expanded slots
     static constexpr int kXchgBytes = NB * 128 * 4;        // partial rows handed from the second drain set to the first
-    static constexpr int kRawSlots = (224 * 1024 - 2048 - kASlots * kABytes - kXSlots * kBBytes - kXchgBytes) / kRawBytes;
+    static constexpr int kRawFit = (224 * 1024 - 2048 - kXSlots * kBBytes - kXchgBytes) / kRawBytes;
+    static constexpr int kRawSlots = (kRawFit < 14 ? kRawFit : 14) & ~1;
     static constexpr int kOffX = kRawSlots * kRawBytes;
-    static constexpr int kOffA = kOffX + kXSlots * kBBytes;
-    static constexpr int kOffXchg = kOffA + kASlots * kABytes;
+    static constexpr int kOffXchg = kOffX + kXSlots * kBBytes;
     static constexpr int kOffBars = kOffXchg + kXchgBytes;
     static constexpr int kNumBars = 2 * kRawSlots + kXSlots + kASlots + kBtDoneRing + kBufs + 3;
     static constexpr int kSmemBytes = kOffBars + kNumBars * 8 + 16 + 1024;  // + slack for the 1024-byte alignment
-    static_assert(kRawSlots >= 4 && kRawSlots < kBtDoneRing && kXSlots < kBtDoneRing && kBufs < kBtDoneRing && kBufs >= 2, "ring sizes");
-    static_assert(kOffX % 1024 == 0 && kOffA % 1024 == 0 && kSmemBytes <= 227 * 1024, "swizzled tiles start on 1024-byte boundaries");
+    static_assert(kRawSlots >= 4 && kRawSlots < kBtDoneRing && kXSlots < kBtDoneRing && kASlots % 2 == 0, "ring sizes");
+    static_assert(kTmemA + kASlots * kACols <= 512, "tensor memory");
+    static_assert(kOffX % 1024 == 0 && kSmemBytes <= 227 * 1024, "swizzled tiles start on 1024-byte boundaries");
 };
 
 // The unit sequence of one block: units u = blockIdx.x, + gridDim.x, ...; unit = (row tile over all matrices, split);
@@ -310,10 +314,9 @@ __device__ inline void small_store(const SmallParams& p, const SmallMat& mt, int
 #define PROF_END(role)
 #endif
 // NB = rows of x per block (16 or 32): N = 4 NB digit columns per MMA; GP = groups per item (SmallShape).
-// Warp roles are placed by scheduler (warp % 4): an MMA warp shares its scheduler with the two TMA warps, which sleep on
-// barriers most of the time, and drain warps; the expanding warps, which spin and compute, sit on the other three.
-//   warps 0, 11: MMA     warp 4: TMA digits     warp 8: TMA weights     warps 1 2 3 5 | 6 7 9 10: the two expanding sets
-//   warps 12..15 | 16..19: the two draining sets (tensor-memory lanes 32 (w % 4) ..)
+// Expanding and draining warps work on the tensor-memory lanes 32 (w % 4) .. they may reach:
+//   warps 0..3 | 4..7: the two expanding sets     warps 8..11 | 12..15: the two draining sets
+//   warps 16, 17: MMA     warp 18: TMA weights     warp 19: TMA digits
 template <int NB, int GP>
 __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const SmallParams p, const __grid_constant__ CUtensorMap map_w0,
                                                                         const __grid_constant__ CUtensorMap map_w1,
@@ -365,10 +368,9 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
     auto done_wait = [&](int n) { return mbar_wait<false>(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
     auto done_warp_wait = [&](int n) { return warp_wait(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
     static_assert(kBtDoneRing == 16, "done_wait shifts by 4");
-    const bool expander = warp < 11 && (warp & 3) != 0;  // warps 1 2 3 5 6 7 9 10
     UnitCursor cur;
 
-    if (warp == 8) {
+    if (warp == 18) {
         // ---- TMA of the raw weight tiles.  The weights never change, so these copies start at once, whatever the previous
         // kernel is still doing.  With two groups per item the box is 128 bytes wide (128-byte swizzle, which the expanding
         // warps undo when they read); a box that reaches past the unit or past K brings bytes nobody uses, or zeros.
@@ -388,7 +390,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
             } while (cur.advance(p, G, GP));
             if (lane == 0) PROF_END(0);
         }
-    } else if (warp == 4) {
+    } else if (warp == 19) {
         // ---- TMA of the digit planes: they come from the previous kernel; a slot is free when the item that used it
         // last (kXSlots back) has been multiplied
         pdl_wait();
@@ -410,15 +412,15 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
             } while (cur.advance(p, G, GP));
             if (lane == 0) PROF_END(1);
         }
-    } else if (warp == 0 || warp == 11) {
+    } else if (warp >= 16) {
         // ---- MMA issuers: one thread of each of two warps, alternate items (their accumulators are different buffers, so
         // no order is needed between them).  Per item: the tiles are expanded, the digit planes have landed, the accumulator
         // buffer has been read out; four MMAs per group; one commit.
-        const int set = warp == 0 ? 0 : 1;
+        const int set = warp - 16;
         if (cur.start(p, blockIdx.x, G)) {
             const uint32_t lead = elect_lead();
             constexpr uint32_t idesc = gemm_idesc_s8s8(128, kN);
-            const uint64_t desc_a0 = gemm_smem_desc(smem_base + S::kOffA), desc_b0 = gemm_smem_desc(smem_base + S::kOffX);
+            const uint64_t desc_b0 = gemm_smem_desc(smem_base + S::kOffX);
             RingPos<S::kASlots> ap;
             RingPos<S::kXSlots> xp;
             RingPos<S::kBufs> bp;
@@ -427,11 +429,6 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
             do {
                 if ((it & 1) == set) {
                     PROF_W0;
-                    // Rings of an odd size: the slot's use before this one was the other warp's.  Until that has come and gone the
-                    // barrier's parity still is that of the use before it, and the waits below would fall through.
-                    constexpr int kBack = S::kASlots % 2 != 0 ? S::kASlots : S::kXSlots % 2 != 0 ? S::kXSlots : 0;
-                    static_assert(S::kASlots % 2 == 0 || S::kXSlots % 2 == 0 || S::kASlots == S::kXSlots, "one look back covers both rings");
-                    if (kBack > 0 && it >= kBack && !done_warp_wait(it - kBack)) { ok = false; break; }
                     if (!warp_wait(&a_ready[ap.idx], ap.phase) || !warp_wait(&x_full[xp.idx], xp.phase) ||
                         (bp.wrapped && !warp_wait(&tmem_free[bp.idx], bp.phase ^ 1u))) {
                         ok = false;
@@ -443,11 +440,11 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
 #pragma unroll
                     for (int j = 0; j < GP; ++j) {
                         if (j < ng) {
-                            const uint64_t da = desc_a0 + (uint64_t)((uint32_t)ap.idx * (S::kABytes >> 4) + j * (kBtABytes >> 4));
+                            const uint32_t ta = (uint32_t)(S::kTmemA + ap.idx * S::kACols + j * kBtACols);
                             const uint64_t db = desc_b0 + (uint64_t)((uint32_t)xp.idx * (S::kBBytes >> 4) + j * (kGroupB >> 4));
                             const uint32_t d = (uint32_t)(bp.idx * GP * kN + j * kN);  // (all 512 columns are this block's: they start at 0)
 #pragma unroll
-                            for (int ks = 0; ks < 4; ++ks) lead_mma_i8(lead, d, da + 2 * ks, db + 2 * ks, idesc, ks > 0 ? 1u : 0u);
+                            for (int ks = 0; ks < 4; ++ks) lead_mma_i8_ts(lead, d, ta + 8 * ks, db + 2 * ks, idesc, ks > 0 ? 1u : 0u);
                         }
                     }
                     lead_commit(lead, &done[it & (kBtDoneRing - 1)]);
@@ -457,16 +454,13 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
             } while (cur.advance(p, G, GP));
             if (lane == 0) PROF_END(2 + set);
         }
-    } else if (expander) {
-        // ---- weight expansion, two sets of four warps that take the items alternately.  A thread turns four 16-byte pieces
-        // of raw nibbles per group (32 columns each) into signed bytes.  One group per item: piece id = 128 i + (thread of
-        // the set) is (row id / 4, quarter id % 4) of the 64-byte rows - a warp reads 512 contiguous bytes.  Two groups per
-        // item: the raw rows are 128 bytes in the 128-byte swizzle, and the eight lanes of a quarter warp take eight
-        // consecutive rows at the same quarter, so that their reads and their writes fall on distinct banks.
-        const int e = warp - 1 - (warp > 4 ? 1 : 0) - (warp > 8 ? 1 : 0);  // 0..7
-        const int set = e >> 2;
-        const int wv = e & 3;
-        const int dt = wv * 32 + lane;  // thread of the set, 0..127
+    } else if (warp < 8) {
+        // ---- weight expansion, two sets of four warps that take the items alternately.  A thread has a weight row of the tile: per group it
+        // turns 64 bytes of nibbles into 128 signed bytes, the 32 columns of its tensor-memory lane.  Raw rows of two groups are
+        // 128 bytes in the 128-byte swizzle, those of one 64 bytes in the 64-byte swizzle: eight lanes read distinct banks.
+        const int set = warp >> 2;
+        const int r = (warp & 3) * 32 + lane;
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
         if (cur.start(p, blockIdx.x, G)) {
             RingPos<S::kRawSlots> rp;
             RingPos<S::kASlots> ap;
@@ -476,43 +470,30 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                 if ((it & 1) == set) {
                     // the raw tile has landed; the expanded slot is free (its last user, kASlots items back, has been multiplied)
                     PROF_W0;
-                    if (S::kRawSlots % 2 != 0 && it >= S::kRawSlots && !done_wait(it - S::kRawSlots)) { ok = false; break; }  // (as in the issuing warps)
-                    if (!mbar_wait<false>(&raw_full[rp.idx], rp.phase) || (it >= S::kASlots && !done_wait(it - S::kASlots))) { ok = false; break; }
+                    if (!warp_wait(&raw_full[rp.idx], rp.phase) || (it >= S::kASlots && !done_warp_wait(it - S::kASlots))) { ok = false; break; }
                     PROF_W1;
+                    tcgen05_fence_after();
                     const unsigned char* raw = ssmem + (size_t)rp.idx * S::kRawBytes;
                     const int ng = min(GP, cur.g1 - cur.g);
 #pragma unroll
                     for (int j = 0; j < GP; ++j) {
                         if (j < ng) {
-                            unsigned char* a = ssmem + S::kOffA + (size_t)ap.idx * S::kABytes + (size_t)j * kBtABytes;
-                            uint4 w[4];
-                            int row[4], qt[4];
+                            uint32_t d[32];
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                if (GP == 1) {
-                                    const int id = i * 128 + dt;
-                                    row[i] = id >> 2;
-                                    qt[i] = id & 3;
-                                    w[i] = *reinterpret_cast<const uint4*>(raw + (size_t)id * 16);
-                                } else {
-                                    row[i] = i * 32 + wv * 8 + (lane & 7);
-                                    qt[i] = lane >> 3;
-                                    w[i] = *reinterpret_cast<const uint4*>(raw + row[i] * 128 + (((4 * j + qt[i]) ^ (row[i] & 7)) << 4));
+                            for (int c = 0; c < 4; ++c) {
+                                const uint4 w = *reinterpret_cast<const uint4*>(GP == 1 ? raw + r * 64 + ((c ^ ((r >> 1) & 3)) << 4) : raw + r * 128 + (((4 * j + c) ^ (r & 7)) << 4));
+                                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    d[c * 8 + 2 * i] = nibble_bytes_to_s8(ww[i], 0);
+                                    d[c * 8 + 2 * i + 1] = nibble_bytes_to_s8(ww[i], 4);
                                 }
                             }
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int r = row[i];
-                                const uint4 lo = make_uint4(nibble_bytes_to_s8(w[i].x, 0), nibble_bytes_to_s8(w[i].x, 4), nibble_bytes_to_s8(w[i].y, 0),
-                                                            nibble_bytes_to_s8(w[i].y, 4));
-                                const uint4 hi = make_uint4(nibble_bytes_to_s8(w[i].z, 0), nibble_bytes_to_s8(w[i].z, 4), nibble_bytes_to_s8(w[i].w, 0),
-                                                            nibble_bytes_to_s8(w[i].w, 4));
-                                *reinterpret_cast<uint4*>(a + r * 128 + (((2 * qt[i]) ^ (r & 7)) << 4)) = lo;
-                                *reinterpret_cast<uint4*>(a + r * 128 + (((2 * qt[i] + 1) ^ (r & 7)) << 4)) = hi;
-                            }
+                            tmem_store_x32(lanes + (uint32_t)(S::kTmemA + ap.idx * S::kACols + j * kBtACols), d);
                         }
                     }
-                    fence_proxy_async_smem();  // the tensor core reads the tiles through the async proxy
+                    tmem_store_wait();
+                    tcgen05_fence_before();
                     __syncwarp();
                     if (lane == 0) {
                         mbar_arrive(&raw_free[rp.idx]);
@@ -522,15 +503,15 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                 rp.next(); ap.next();
                 ++it;
             } while (cur.advance(p, G, GP));
-            if (dt == 0) PROF_END(4 + set);
+            if (r == 0) PROF_END(4 + set);
         }
-    } else if (warp >= 12) {
+    } else {
         // ---- drain, two sets of four warps that take the items alternately: warp w may read tensor-memory lanes
         // 32 (w % 4) ..; lane = weight row inside the tile; each thread accumulates its row for all rows of x.  At the end of
         // a unit the second set hands its sums to the first through shared memory; the first set finishes the rows.
         const int q = warp & 3;
         const int rl = q * 32 + lane;
-        const int set = warp >= 16 ? 1 : 0;
+        const int set = warp >= 12 ? 1 : 0;
         float* xchg = reinterpret_cast<float*>(ssmem + S::kOffXchg);  // [NB][128]
         uint32_t drain_phase = 0, xchg_phase = 0;
         pdl_wait();  // inv_xscale, the residual and the cleared counters come from earlier kernels
@@ -565,7 +546,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                             s_next[j] = cur.g + 2 * GP + j < cur.g1 ? __ldg(srow + cur.g + 2 * GP + j) : 0u;
                         }
                         PROF_W0;
-                        if (!done_wait(it)) { ok = false; break; }
+                        if (!done_warp_wait(it)) { ok = false; break; }  // (the loads below want the whole warp)
                         PROF_W1;
                         tcgen05_fence_after();
                         const int ng = min(GP, cur.g1 - cur.g);
@@ -635,7 +616,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                     if (lane == 0) mbar_arrive(drain_bar);
                     if (!mbar_wait<false>(drain_bar, drain_phase & 1u)) { ok = false; break; }
                     ++drain_phase;
-                    if (warp == 12 && lane == 0) {
+                    if (warp == 8 && lane == 0) {
                         const unsigned int prev = atomicAdd(&p.counters[tile], 1u);
                         *last_flag = prev == (unsigned int)p.ksplit - 1u ? 1u : 0u;
                     }
@@ -658,7 +639,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                             for (int m = 0; m < NB; ++m) acc[m] += t[m];
                         }
                         small_store<NB, NB <= 16 ? 4 : 1>(p, mt, row, 1.0f, acc);
-                        if (warp == 12 && lane == 0) p.counters[tile] = 0u;
+                        if (warp == 8 && lane == 0) p.counters[tile] = 0u;
                     }
                 }
             }
@@ -820,7 +801,7 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
                 it += n_items;
                 for (int k = 0; k < n_items && more; ++k) more = cur.advance(p, G);
                 const int par = unit_no & 1;
-                if (!mbar_wait<false>(&unit_done[par], (uint32_t)(unit_no >> 1) & 1u)) { ok = false; break; }
+                if (!warp_wait(&unit_done[par], (uint32_t)(unit_no >> 1) & 1u)) { ok = false; break; }
                 tcgen05_fence_after();
                 // which thread took the first group of the unit decides nothing here: both accumulators are simply added
                 const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((par * 2 + 0) * kN);

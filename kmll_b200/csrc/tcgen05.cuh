@@ -83,6 +83,11 @@ __device__ inline void lead_mma_i8(uint32_t lead, uint32_t d, uint64_t a, uint64
         "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t@e tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
+__device__ inline void lead_mma_i8_ts(uint32_t lead, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t@e tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
 __device__ inline void lead_commit(uint32_t lead, uint64_t* bar) {
     asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
                  ::"r"(smem_u32(bar)), "r"(lead) : "memory");

@@ -226,6 +226,24 @@ def test_other_sizes(cuda, name, dtype):
     m.close()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_wanted_rows_with_and_without_the_last(cuda, dtype):
+    """The last row's logits come from the projection that finds the next token; asked for alone, among others and not at all, in
+    one portion and in portions of one row, every row is the oracle's."""
+    m = Model(config([with_mlp(lightning(), 100), latent(heads=2, window=70)]), dtype, seed=4)
+    tokens = m.tokens(9)
+    want = m.oracle(tokens)
+    session = Session(m.dec)
+    for rows in ([8], [0, 8], [7], [2, 7], list(range(9))):
+        session.reset_sequence()
+        check(session.extend([int(t) for t in tokens], rows), want[rows], dtype, 1.5)
+        check(np.asarray(session.next_logits_to_host(), dtype=np.float64).reshape(1, -1), want[8:9], dtype, 1.5)
+    m.dec.reset()
+    for i in range(9):
+        check(m.dec.extend(tokens[i:i + 1], [0]), want[i:i + 1], dtype, 1.5)
+    m.close()
+
+
 @pytest.mark.parametrize("window", [1, 100, 128, 300, 512])
 def test_latent_prompt_over_tiles(cuda, window):
     """Latent heads of 128 + 64 and 128 (attention on tensor memory): every position of a prompt of several 128-row blocks and 128-key
