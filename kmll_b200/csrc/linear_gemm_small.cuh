@@ -18,7 +18,9 @@
 // live; the roles that do work per group exist twice and take the groups alternately; and the issuing roles run as whole
 // warps with one elected lane (tcgen05.cuh): as single threads, at 100 to 250 cycles per mbarrier, TMA or tcgen05 instruction, 16
 // rows of x took 30.2 us for 28672 x 4096 where they take 28.4 now, 13.0 / 11.7 for 4096 x 4096, 21.3 / 19.5 for 4096 x 14336, RS-I8
-// 4096 x 14336 18.8 / 17.5, 32 rows and 4096 x 4096 19.6 / 15.3.
+// 4096 x 14336 18.8 / 17.5, 32 rows and 4096 x 4096 19.6 / 15.3.  With the expanded tiles in tensor memory 27.9, 10.9 and 18.2; with half
+// the instructions in the drain (two digits to an integer, integers to f32 by conversion) 24.7, 10.5 and 17.3 (32 rows, 14336 x 4096: 28.5 us at first, 24.1, now 18.6): the issue slots
+// that expansion and drain share are what bounds a group now.
 //   * raw weight tiles (128 rows x 64 bytes of nibbles, TMA by warp 8): 12 slots (7 with 32 rows of x) - they wait out the HBM latency;
 //   * digit planes of the same 128 columns (one 3-D TMA box, 128-byte swizzle, warp 4): 5 or 6 slots - L2 latency;
 //   * signed-byte weight tiles in tensor memory (lane = weight row, a column = four bytes of K): 4 slots, written by two sets of four
@@ -30,9 +32,8 @@
 //   buffer, issues the four MMAs (M = 128 weight rows, N = 4 n_block digit columns, K = 32 bytes each) and one commit on a
 //   ring of 16 `done` barriers; the producers, the expanding warps and the draining warps all derive what they wait for
 //   from that ring (the slot they want to refill was last used by the group `ring size` back).  Two sets of four warps
-//   drain: tcgen05.ld of the buffer, release it, integer -> f32 without conversion instructions (the sums are below 2^22:
-//   add them to the bits of 1.5 * 2^23 and subtract that constant), combine the digits, one FMA with the group scale into
-//   f32 accumulators in registers.  After the last group of a unit the second set hands its sums to the first through
+//   drain: tcgen05.ld of the buffer, release it, two digits to an integer, two integers to f32, combine them, one FMA with the
+//   group scale into f32 accumulators in registers.  After the last group of a unit the second set hands its sums to the first through
 //   shared memory, and the first stores the rows (or the split-K partial; the unit that arrives last adds the partials in
 //   split order, so results are bit-identical from call to call).
 // Because an accumulator lives for one group only, the pipeline runs on across unit boundaries without draining.
@@ -551,33 +552,30 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                         tcgen05_fence_after();
                         const int ng = min(GP, cur.g1 - cur.g);
                         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(bp.idx * GP * kN);
+                        // |D_i| <= 128 * 8 * 128 = 2^17, the top digit's <= 33 * 8 * 128: two digits together fit 32 bits, the upper two 24
+                        auto value = [](uint32_t d0, uint32_t d1, uint32_t d2, uint32_t d3) {
+                            return fmaf((float)((int)d2 + ((int)d3 << 8)), 65536.0f, (float)((int)d0 + ((int)d1 << 8)));
+                        };
 #pragma unroll
-                        for (int j = 0; j < GP; ++j) {
+                        for (int j = 0; j < GP; ++j) {  // (an item has at least one group)
 #pragma unroll
                             for (int m0 = 0; m0 < NB; m0 += 8) {
                                 uint32_t d0[8], d1[8], d2[8], d3[8];
-                                if (j < ng) {
+                                if (j == 0 || j < ng) {
                                     tmem_ld8(taddr + j * kN + m0, d0);
                                     tmem_ld8(taddr + j * kN + NB + m0, d1);
                                     tmem_ld8(taddr + j * kN + 2 * NB + m0, d2);
                                     tmem_ld8(taddr + j * kN + 3 * NB + m0, d3);
-                                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                                    tmem_load_wait();
                                 }
                                 if (j == GP - 1 && m0 + 8 >= NB) {  // everything of this buffer is in registers: hand it back
                                     tcgen05_fence_before();
                                     __syncwarp();
                                     if (lane == 0) mbar_arrive(&tmem_free[bp.idx]);
                                 }
-                                if (j < ng) {
-                                    // |D_i| <= 128 * 8 * 128 = 2^17: the integer added to the bits of 1.5 * 2^23 is that float plus the integer
-                                    const float kMagic = 12582912.0f;
+                                if (j == 0 || j < ng) {
 #pragma unroll
-                                    for (int t8 = 0; t8 < 8; ++t8) {
-                                        const float f0 = __uint_as_float(0x4b400000u + d0[t8]) - kMagic, f1 = __uint_as_float(0x4b400000u + d1[t8]) - kMagic;
-                                        const float f2 = __uint_as_float(0x4b400000u + d2[t8]) - kMagic, f3 = __uint_as_float(0x4b400000u + d3[t8]) - kMagic;
-                                        const float t = fmaf(fmaf(fmaf(f3, 256.0f, f2), 256.0f, f1), 256.0f, f0);
-                                        acc[m0 + t8] = fmaf(t, sc[j], acc[m0 + t8]);
-                                    }
+                                    for (int t8 = 0; t8 < 8; ++t8) acc[m0 + t8] = fmaf(value(d0[t8], d1[t8], d2[t8], d3[t8]), sc[j], acc[m0 + t8]);
                                 }
                             }
                         }

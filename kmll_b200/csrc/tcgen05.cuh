@@ -137,6 +137,7 @@ __device__ inline void tmem_store_x16(uint32_t taddr, const uint32_t (&d)[16]) {
           "r"(d[11]), "r"(d[12]), "r"(d[13]), "r"(d[14]), "r"(d[15]), "r"(taddr)
         : "memory");
 }
+__device__ inline void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ inline void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 }  // namespace kmll
