@@ -1067,9 +1067,9 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(const float* 
     }
 }
 
-// ---- prefill on the tensor cores --------------------------------------------------------------------------
-// The same causal attention as prefill_attention_kernel for the decoder's batched prefill, where it was more than half of
-// the time (2048-token prompt, Mistral-7B shape: 114 of 204 ms on CUDA cores).  One block = one query head x 64 query rows,
+// ---- prefill on mma.sync ----------------------------------------------------------------------------------
+// The same causal attention as prefill_attention_kernel for the decoder's batched prefill where prompt_attention.cu does not serve: an
+// f32 cache without planes of its rows (partial rotation, keys wider than the feed-forward).  One block = one query head x 64 query rows,
 // four warps of 16 rows each; key tiles of 64 positions.  Both contractions run as bf16 MMAs with f32 accumulation, every
 // f32 operand split into a bf16 head and remainder and three of the four partial products kept (16 mantissa bits per
 // operand, a relative 2^-17 per product); with a bf16 cache K and V are exact and two products remain.
