@@ -366,7 +366,9 @@ int kmll_top_k_f32(kmll_stream_t stream, const float* logits, size_t n, int k, u
  *                              below silu_rows go through SiLU
  *   kmll_polynorm_linear_bf16  a N(x) + b N(x^2) + c N(x^3) + e, coef = (a, b, c, e) bf16, N = division by the root mean square
  *   kmll_gated_linear_bf16     x over its root mean square (all of x, times norm_weight; or per head_len entries when norm_weight
- *                              is null) times silu (gate_sigmoid = 0) or sigmoid (1) of gate */
+ *                              is null) times silu (gate_sigmoid = 0) or sigmoid (1) of gate
+ * These three, kmll_normed_linear_bf16 and kmll_mixer_output_linear_bf16 start to read `w` while the kernel in front of them on the
+ * stream is still running: that kernel must not write `w`.  It may write any other operand, norm weights among them. */
 int kmll_linear_bf16(kmll_stream_t stream, const float* x, const uint16_t* w, int pitch, int rows, int cols, const uint16_t* norm_weight, float norm_offset,
                      float eps, const float* residual, int silu_rows, float* y);
 int kmll_polynorm_linear_bf16(kmll_stream_t stream, const float* x, const uint16_t* coef, float eps, const uint16_t* w, int pitch, int rows, int cols,

@@ -252,6 +252,7 @@ struct Bf16Matvec {
     int silu_rows;       // rows below this index go through SiLU
     int pair_act;        // not 0: rows 2 i and 2 i + 1 are a gate and its value, y[i] = act(gate) * value
     float out_scale;     // factor on every result (ahead of the residual)
+    int norm_constant;   // the norm weights (norm, seg[].norm_w) are a model's: read ahead of the dependency wait, like w
     // arg-max over the rows (packed != null): partials of kMatvecMaxBlocks entries, a zeroed counter; state != null: the decode
     // step ends here (next_top, position, step)
     uint32_t* part_tok;

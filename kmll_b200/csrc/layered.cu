@@ -414,6 +414,7 @@ Bf16Matvec matvec(const Mat& m, const float* x, float* out) {
     v.w = m.w; v.rows = m.rows; v.K = m.cols; v.ldw = m.ld;
     v.x = x; v.y = out;
     v.out_scale = 1.0f;
+    v.norm_constant = 1;
     return v;
 }
 NormArgs norm_args(const Layered* L, const uint16_t* w, const uint16_t* b) { return NormArgs{L->cfg.norm, w, b, L->cfg.norm_offset, L->cfg.norm_eps}; }

@@ -86,8 +86,9 @@ __global__ void __launch_bounds__(kVThreads, 2) bf16_matvec_kernel(const MatvecA
         for (int r = 0; r < kVDepth; ++r) request(0, 0, r);
 
     // ---- x -> shared memory through the prologue; columns K .. are zeros.  The whole grid waits for this behind its predecessor with no
-    // more than the ring's copies in flight, so whole pieces of four columns are loaded together, and the norm's weights, which are
-    // constants, before the dependency wait.
+    // more than the ring's copies in flight, so whole pieces of four columns are loaded together, and a model's norm weights, which are
+    // constants, before the dependency wait.  An operator's caller may have written them with the launch in front: those are read behind it.
+    if (a.norm_constant == 0) pdl_wait();
     const int kpad = p.kpieces * kVPiece;
     if (p.wide_norm != 0) {
         float4 v[kVHeld];
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(kVThreads, 2) bf16_matvec_kernel(const MatvecA
                 if (layer) nb[i] = *reinterpret_cast<const uint2*>(a.norm.b + k);
             }
         }
-        pdl_wait();
+        if (a.norm_constant != 0) pdl_wait();
 #pragma unroll
         for (int i = 0; i < kVHeld; ++i) {
             const int k = (tid + i * kVThreads) * 4;
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(kVThreads, 2) bf16_matvec_kernel(const MatvecA
             if (g.norm == KMLL_OUT_NORM_JOINT) w[i] = *reinterpret_cast<const uint2*>(g.norm_w + (k - g.begin));
             else if (g.norm == KMLL_OUT_NORM_HEAD_WEIGHTED) w[i] = *reinterpret_cast<const uint2*>(g.norm_w + ((k - g.begin) & 127));
         }
-        pdl_wait();
+        if (a.norm_constant != 0) pdl_wait();
         float s[kMaxSegments] = {};
 #pragma unroll
         for (int i = 0; i < kVHeldGated; ++i) {
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kVThreads, 2) bf16_matvec_kernel(const MatvecA
             }
             *reinterpret_cast<float4*>(xs + vec_slot(k, p.half)) = make_float4(y[0], y[1], y[2], y[3]);
         }
-    } else {
+    } else if (a.norm_constant != 0) {
         pdl_wait();
     }
     if (p.wide_norm != 0 || p.wide_gated != 0) {

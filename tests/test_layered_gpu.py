@@ -529,6 +529,41 @@ def test_bf16_linear_operators(cuda):
         assert float((got.double() - w0 @ torch.from_numpy(n).cuda()).abs().max()) <= 4e-5 * cols ** 0.5
 
 
+def test_norm_weights_of_the_launch_in_front(cuda):
+    """Norm weights that the launch directly in front writes - a long one, which ends with them - are the ones that the projection
+    uses, in every form that loads them in whole pieces.  Bounds as in test_operators_against_64_bits."""
+    import torch
+
+    from kmll_b200 import ops
+
+    cols, rows, eps = 2048, 160, 1e-3
+    gen = torch.Generator(device="cuda").manual_seed(21)
+    w = (torch.randn(rows, cols, generator=gen, device="cuda") / cols ** 0.5).bfloat16()
+    x, gate = (torch.randn(cols, generator=gen, device="cuda") for _ in range(2))
+    xd, gd, w0 = x.double(), gate.double(), w.double()
+    source = torch.zeros(1 << 25, device="cuda")
+    linear = rt.MixerSpec(rt.MIXER_GATED_LINEAR, cols // 128, 128, 128, out_norm=rt.OUT_NORM_HEAD_WEIGHTED, gate_act=rt.ACT_SILU)
+    centred = xd - xd.mean()
+    normed = xd / (xd.square().mean() + eps).sqrt()
+    by_head = (xd.view(-1, 128) / (xd.view(-1, 128).square().mean(1, keepdim=True) + eps).sqrt()).reshape(-1)
+    silu = gd * torch.sigmoid(gd)
+    forms = [(lambda n: ops.linear_bf16(x, w, norm_weight=n, eps=eps), lambda n: normed * n),
+             (lambda n: ops.normed_linear_bf16(x, w, rt.NORM_LAYER, n, n, eps), lambda n: centred / (centred.square().mean() + eps).sqrt() * n + n),
+             (lambda n: ops.gated_linear_bf16(x, gate, w, eps, norm_weight=n), lambda n: normed * n * silu),
+             (lambda n: ops.mixer_output_linear_bf16([linear], x, [n[:128]], [gate], w, eps), lambda n: by_head * n[:128].repeat(cols // 128) * silu)]
+    for i in range(12):
+        source[-cols:] = torch.randn(cols, generator=gen, device="cuda") + 1.0
+        for call, value in forms:
+            got = call(ops.f32_to_bf16(source)[-cols:])
+            want = w0 @ value(source[-cols:].bfloat16().double())
+            assert float((got.double() - want).abs().max()) <= 4e-5 * cols ** 0.5, i
+    # written long before: the same values
+    n = ops.f32_to_bf16(source)[-cols:]
+    torch.cuda.synchronize()
+    for call, value in forms:
+        assert float((call(n).double() - w0 @ value(n.double())).abs().max()) <= 4e-5 * cols ** 0.5
+
+
 # more than 256 rows of x: pairs of blocks.  One k-tile (one accumulator), a ragged last one, one row of weights, ragged tiles on both
 # sides, several units per pair
 @pytest.mark.parametrize("tokens,rows,cols", [(257, 130, 72), (300, 2, 64), (513, 520, 200), (640, 257, 1000), (1030, 6000, 136), (2500, 384, 4104)])
