@@ -10,7 +10,8 @@
 //                   by tcgen05.ld, twice - a first pass for the maximum, a second for the weights -, and the weights go back as bf16
 //                   planes in the place of the scores.  The two are independent streams, each with its own maximum, sum and
 //                   O in tensor memory, and are merged at the end.
-//   warps 8, 9      TMA of the key tiles and of the value tiles (values as they lie: the B operand of P V is MN-major)
+//   warps 8, 9      TMA of the key tiles and of the value tiles (values as they lie: the B operand of P V is MN-major); warp 9 also looks
+//                   through the values of tiles that some row does not see in full (PaHeld)
 //   warp 10         issues S = Q K^T (both operands in shared memory) and O += P V (P from tensor memory)
 // Bound by the tensor cores with f32 operands (48 MMAs of 61 cycles a tile; a fifth of the issuer's time is waiting), by the second pass of
 // the softmax (3460 cycles of its warps per tile, exponentials and conversions) with bf16 ones.  Measured against the mma.sync
@@ -42,7 +43,7 @@ constexpr int kPaBox = 128 * 128;  // a TMA box: 128 rows of 64 bf16 entries in 
 constexpr uint32_t kPaTmemO = 256;
 
 // Shared memory: planes of Q [128 rows][DQ] as 64-entry wide blocks; ring of stages with the boxes of K ([128 keys][DQ], NK planes) and of V
-// ([128 keys][DV]); each stream's (maximum, sum) per row; barriers.  NQ, NK: planes of Q and of K and V.
+// ([128 keys][DV]); each stream's (maximum, sum) per row; barriers; PaHeld.  NQ, NK: planes of Q and of K and V.
 template <int DQ, int DV, int NQ, int NK>
 struct PaShape {
     static constexpr int kQPlane = kPaRows * DQ * 2, kKBoxes = NK * DQ / 64, kVBoxes = NK * DV / 64;
@@ -50,7 +51,8 @@ struct PaShape {
     static constexpr int kStages = kOffK + 2 * (kKBoxes + kVBoxes) * kPaBox <= 216 * 1024 ? 2 : 1;
     static constexpr int kOffV = kOffK + kStages * kKBoxes * kPaBox, kOffStat = kOffV + kStages * kVBoxes * kPaBox;
     static constexpr int kOffBars = kOffStat + 2 * kPaRows * 8;
-    static constexpr int kSmemBytes = kOffBars + 128 + 1024;  // + slack for the 1024-byte alignment
+    static constexpr int kOffHeld = kOffBars + 128;           // PaHeld: [3 tiles][DV][128 bits]
+    static constexpr int kSmemBytes = kOffHeld + 3 * DV * 16 + 1024;  // + slack for the 1024-byte alignment
     static constexpr int kStagePitch = DV / 2 + 4;            // rows of half of O on their way out, over the operands
     static_assert(DQ % 64 == 0 && (DV == 64 || DV == 128) && kSmemBytes <= 227 * 1024, "shape");
     static_assert(8 * 32 * kStagePitch * 4 <= kOffStat, "the rows of O fit over the operands");
@@ -69,11 +71,42 @@ __device__ inline void pa_split8(const float (&v)[8], uint4& hi, uint4& lo) {
 __device__ inline uint64_t pa_desc_mn(uint32_t smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(kPaBox >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
+// Values that are not finite.  A key that a row does not attend has weight 0 there, and 0 * infinity is NaN.  So in the tiles that some
+// row does not see in full - at most three: the first (window) and the last two (causal) - such entries become zeros ahead of the
+// MMAs and are noted, a bit per (column, key); at the end an output whose row attends one of them becomes NaN.
+struct PaHeld {
+    // slot of tile j; the keys of the tile in the slot
+    static __device__ inline int slot(int j, int tiles) { return j == tiles - 1 ? 0 : j == tiles - 2 ? 1 : 2; }
+    static __device__ inline int tile(int slot, int tiles) { return slot == 2 ? 0 : tiles - 1 - slot; }
+    // The exponent of a half of w is all ones: bit 15 of that half here.  (Of two planes the first one tells: the remainder is finite with it.)
+    static __device__ inline uint32_t not_finite(uint32_t w) { return (w & 0x7f807f80u) + 0x00800080u; }
+    // key r of the tile, whose 128-byte rows of the first box start at `box`
+    template <int DV, int NK>
+    static __device__ inline void hold_back(unsigned char* box, int r, uint32_t* bits) {
+#pragma unroll 1
+        for (int col = 0; col < DV; ++col) {
+            unsigned char* const at = box + (col >> 6) * kPaBox + r * 128 + ((((col >> 3) & 7) ^ (r & 7)) << 4) + (col & 7) * 2;
+            if ((*reinterpret_cast<const uint16_t*>(at) & 0x7f80u) != 0x7f80u) continue;
+            for (int n = 0; n < NK; ++n) *reinterpret_cast<uint16_t*>(at + n * (DV / 64) * kPaBox) = 0u;
+            atomicOr(bits + col * 4 + (r >> 5), 1u << (r & 31));
+        }
+    }
+    // whether a bit of keys a .. b is set (either may lie outside the tile)
+    static __device__ inline bool any(const uint32_t* bits, int a, int b) {
+        for (int w = 0; w < 4; ++w) {
+            const int lo = max(a - w * 32, 0), hi = min(b - w * 32, 31);
+            if (lo <= hi && (bits[w] & (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo)) != 0u) return true;
+        }
+        return false;
+    }
+};
 // What a block attends: row r of the block is position pos0 + r and sees the keys max(0, pos - window + 1) .. pos (window 0: from 0);
 // keys first .. last are walked in tiles.
 struct PaRange {
     int pos0, live_rows, first, last, window;
     float scale2;  // log2(e) times the score scale, positive
+    // some row does not see some key of the tile that starts at t0
+    __device__ bool partly(int t0) const { return t0 + kPaKeys - 1 > pos0 || (window > 0 && t0 < pos0 + kPaRows - window); }
 };
 
 // Src: kDQ, kDV, kNQ, kNK; q_planes(row, c8, planes): eight entries of a query row; load_k(lead, box, pos, dst, bar), load_v: the TMA of one box
@@ -90,13 +123,19 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
     uint64_t* const pv_done = p_ready + 2;        // [2] O has taken the tile
     uint64_t* const k_full = pv_done + 2;         // [kStages]
     uint64_t* const v_full = k_full + kStages;    // [kStages]
-    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(v_full + kStages);
+    uint64_t* const v_clean = v_full + kStages;   // [3] PaHeld: the tile of the slot has been looked through
+    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(v_clean + 3);
+    uint32_t* const any_held = tmem_slot + 1;
+    uint32_t* const held = reinterpret_cast<uint32_t*>(smem + S::kOffHeld);
     const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp_index();
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) { mbar_init(&s_full[b], 1); mbar_init(&p_ready[b], 4); mbar_init(&pv_done[b], 1); }
         for (int st = 0; st < kStages; ++st) { mbar_init(&k_full[st], 1); mbar_init(&v_full[st], 1); }
+        for (int i = 0; i < 3; ++i) mbar_init(&v_clean[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        *any_held = 0u;
     }
+    for (int i = tid; i < 3 * DV * 4; i += kPaThreads) held[i] = 0u;
     if (warp == 10) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -126,6 +165,27 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
         uint64_t* const done = keys ? s_full : pv_done;
         const int boxes = keys ? S::kKBoxes : S::kVBoxes;
         const uint32_t lead = elect_lead();
+        // (This warp has seen every earlier use of the stage end, so the parity of v_full means tile j.)
+        auto look_through = [&](int j) {
+            if (!rg.partly(rg.first + j * kPaKeys)) return true;
+            if (!warp_wait(&v_full[j % kStages], (uint32_t)(j / kStages) & 1u)) return false;
+            unsigned char* const box = smem + S::kOffV + (j % kStages) * S::kVBoxes * kPaBox;
+            uint32_t bad = 0u;
+#pragma unroll 8
+            for (int i = lane; i < 8 * kPaKeys * (DV / 64); i += 32) {
+                const uint4 w = reinterpret_cast<const uint4*>(box)[i];
+                bad |= PaHeld::not_finite(w.x) | PaHeld::not_finite(w.y) | PaHeld::not_finite(w.z) | PaHeld::not_finite(w.w);
+            }
+            const int slot = PaHeld::slot(j, tiles);
+            if (__any_sync(0xffffffffu, (bad & 0x80008000u) != 0u)) {
+                for (int r = lane; r < kPaKeys; r += 32) PaHeld::hold_back<DV, NK>(box, r, held + slot * DV * 4);
+                *any_held = 1u;
+                fence_proxy_async_smem();
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&v_clean[slot]);
+            return true;
+        };
         for (int j = 0; j < tiles; ++j) {
             const int st = j % kStages, before = j - kStages;
             ok = before < 0 || warp_wait(&done[before & 1], (uint32_t)(before >> 1) & 1u);
@@ -136,7 +196,11 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
                 if (keys) src.load_k(lead, b, rg.first + j * kPaKeys, dst + b * kPaBox, &full[st]);
                 else src.load_v(lead, b, rg.first + j * kPaKeys, dst + b * kPaBox, &full[st]);
             }
+            // (with two stages a tile behind, so that the next one's copies are under way)
+            if (!keys && j >= kStages - 1) ok = look_through(j - (kStages - 1));
+            if (!ok) break;
         }
+        for (int j = max(tiles - (kStages - 1), 0); j < tiles && !keys && ok; ++j) ok = look_through(j);
         // after a time-out: what was requested has landed before the block ends
         if (!ok)
             for (int st = 0; st < kStages; ++st) mbar_wait<false>(&full[st], (uint32_t)((tiles - 1 - st) / kStages) & 1u);
@@ -172,6 +236,7 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
         for (int j = 0; j < tiles && ok; ++j) {
             const int st = j % kStages;
             ok = warp_wait(&v_full[st], (uint32_t)(j / kStages) & 1u) && warp_wait(&p_ready[j & 1], (uint32_t)(j >> 1) & 1u);
+            if (ok && rg.partly(rg.first + j * kPaKeys)) ok = warp_wait(&v_clean[PaHeld::slot(j, tiles)], 0u);
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t p = (uint32_t)(j & 1) * 128u, d = kPaTmemO + (uint32_t)(j & 1) * 128u;
@@ -201,7 +266,7 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
         int n = 0;  // tiles of this stream so far
         for (int j = stream; j < tiles; j += 2, ++n) {
             const int t0 = rg.first + j * kPaKeys;
-            const bool masked = t0 + kPaKeys - 1 > rg.pos0 || (rg.window > 0 && t0 < rg.pos0 + kPaRows - rg.window);  // some row does not see some key
+            const bool masked = rg.partly(t0);
             ok = warp_wait(&s_full[stream], (uint32_t)n & 1u);
             if (!ok) break;
             tcgen05_fence_after();
@@ -311,6 +376,12 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    if (*any_held != 0u)
+        for (int i = tid; i < 3 * rg.live_rows * DV; i += kPaThreads) {
+            const int slot = i / (rg.live_rows * DV), row = (i / DV) % rg.live_rows, col = i % DV;
+            const int pos = rg.pos0 + row, t0 = rg.first + PaHeld::tile(slot, tiles) * kPaKeys;  // (no bits are set in a slot without a tile)
+            if (PaHeld::any(held + (slot * DV + col) * 4, (rg.window > 0 ? pos - rg.window + 1 : 0) - t0, pos - t0)) out[(size_t)row * ldo + col] = __int_as_float(0x7fffffff);
+        }
     if (warp == 10) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(512u) : "memory");
 }
 

@@ -259,6 +259,37 @@ def test_latent_prompt_over_tiles(cuda, window):
     m.close()
 
 
+@pytest.mark.parametrize("window", [100, 512])
+def test_latent_prompt_keeps_values_out_of_rows_that_do_not_attend_them(cuda, window):
+    """A token whose value overflows to infinity in two columns: the rows in front of it and those whose window has left it are bit for
+    bit what they are with another token in its place, those that attend it are not.  (The output projection's two columns bring values
+    of about 1e34 back to the size of the residual.)"""
+    n = 390
+    cfg = config([latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=64, window=window, scale=192 ** -0.5)], width=128, positions=512)
+    t = lo.random_tensors(cfg, 3)
+    t["embed"][:, 0] = t["pos"][:, 0] = 0.0
+    t["embed"][1] = 0.0
+    t["embed"][1, 0] = 11.0  # an entry of its own, which latent entry 3 is made of
+    t["l0.mix.dkv"][3] *= 1e-3
+    t["l0.mix.dkv"][3, 0] = 4.0
+    columns = [5, 255]
+    t["l0.mix.uv"][columns] = 0.0
+    t["l0.mix.uv"][columns, 3] = 3e38
+    t["l0.mix.o"][:, columns] *= 1e-34
+    m = Model(cfg, "bfloat16", tensors=t)
+    tokens = np.random.default_rng(window).integers(2, cfg["vocab"], n)
+    want = m.run(tokens)
+    assert np.isfinite(want).all()
+    for at in (5, 127, 128, 200, 289, 389):
+        marked = tokens.copy()
+        marked[at] = 1
+        got = m.run(marked)
+        seen = (np.arange(n) >= at) & (np.arange(n) < at + window)
+        np.testing.assert_array_equal(got[~seen], want[~seen], err_msg=str(at))
+        assert (got[seen] != want[seen]).any(axis=1).all(), at
+    m.close()
+
+
 # ---- one key that stands out ---------------------------------------------------------------------------------------------------
 MARK, ASK = 1, 2  # token MARK leaves a key that token ASK looks for
 

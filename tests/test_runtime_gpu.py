@@ -119,6 +119,46 @@ def test_prompt_attention_tiles_match_oracle(cuda, heads, kv, hd, window, kv_bf1
     dec.close()
 
 
+@pytest.mark.parametrize("heads,kv,hd", [(4, 2, 64), (4, 1, 128)])
+@pytest.mark.parametrize("kv_bf16", [False, True])
+def test_prompt_attention_keeps_values_out_of_rows_that_do_not_attend_them(cuda, heads, kv, hd, kv_bf16):
+    """Token MARK's value overflows to infinity in two columns of a head.  Just in front of the last row's window, in a tile that
+    rows of its block do attend, the last row is bit for bit what it is with another token there; inside the window it is not.
+    The output projection's scales bring the two columns, about 1e36, back to the size of the residual."""
+    window, mark, columns = 100, 1, [5, hd - 1]
+    cfg = tiny(rt.FORMAT_RS_I8, True, n_layers=1, n_heads=heads, n_kv_heads=kv, head_dim=hd, max_seq_len=400, sliding_window=window, kv_bf16=kv_bf16)
+    dec = make(cfg)
+    rng = np.random.default_rng(hd)
+    table = (rng.normal(0, 1, (cfg.vocab_size, cfg.dim)).astype(F).view(np.uint32) >> 16).astype(np.uint16)
+    table[:, 0] = 0
+    table[mark] = 0
+    table[mark, 0] = 0x4180  # 16: the norm leaves the whole row in this entry
+    dec.set_tensor(-1, rt.T_EMBEDDING, table)
+    values, scales = dec.get_tensor(0, rt.T_WV)
+    values[columns] = rng.integers(-1, 2, (2, cfg.dim))
+    values[columns, 0] = 127
+    scales[columns] = 5e35
+    dec.set_tensor(0, rt.T_WV, values, scales)
+    values, scales = dec.get_tensor(0, rt.T_WO)
+    dec.set_tensor(0, rt.T_WO, values, np.full_like(scales, 1e-37))
+    prompt = rng.integers(2, cfg.vocab_size, 390)
+
+    def last(n, at):
+        p = prompt[:n].copy()
+        if at is not None:
+            p[at] = mark
+        dec.prefill(p)
+        return dec.last_hidden()
+
+    for n, outside in ((390, (285, 289)), (384, (157, 200, 283))):
+        want = last(n, None)
+        assert np.all(np.isfinite(want))
+        for at in outside:
+            np.testing.assert_array_equal(last(n, at), want, err_msg=str((n, at)))
+        assert not np.array_equal(last(n, n - 100), want)
+    dec.close()
+
+
 WIDE_FEED_FORWARD = """
 import json, sys
 import numpy as np
