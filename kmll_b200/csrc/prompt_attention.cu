@@ -145,6 +145,9 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    tcgen05_fence_before();
+    __syncthreads();  // (columns first, then the dependents: tcgen05.cuh)
+    tcgen05_fence_after();
     pdl_wait();
     for (int i = tid; i < kPaRows * C8; i += kPaThreads) {  // (rows beyond the prompt are zeros)
         const int r = i / C8, c8 = i - r * C8;
@@ -156,9 +159,7 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
         for (int n = 0; n < NQ; ++n) *reinterpret_cast<uint4*>(smem + n * S::kQPlane + pa_place(r, c8)) = pl[n];
     }
     fence_proxy_async_smem();
-    tcgen05_fence_before();
     __syncthreads();
-    tcgen05_fence_after();
     const int tiles = (rg.last - rg.first) / kPaKeys + 1;
     const uint32_t base = smem_u32(smem);
     bool ok = true;

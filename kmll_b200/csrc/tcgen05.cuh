@@ -41,6 +41,8 @@ __device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity) {
 __device__ inline void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ inline void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ inline void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Tensor memory is allocated before the block releases its dependents, that is, a block barrier stands between tcgen05.alloc and
+// pdl_wait(): a dependent block that held the columns while it waits for this grid would keep this grid in alloc, the one wait without a bound.
 // shared-memory matrix descriptor: K-major operand tile with 128-byte rows in the 128-byte swizzle (what TMA writes with
 // CU_TENSOR_MAP_SWIZZLE_128B): groups of 8 rows are 1024 bytes apart; version 1 (sm_100); layout type 2 = SWIZZLE_128B
 __device__ inline uint64_t gemm_smem_desc(uint32_t smem_addr) {
