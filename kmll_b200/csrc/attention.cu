@@ -1068,8 +1068,8 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(const float* 
 }
 
 // ---- prefill on mma.sync ----------------------------------------------------------------------------------
-// The same causal attention as prefill_attention_kernel for the decoder's batched prefill where prompt_attention.cu does not serve: an
-// f32 cache without planes of its rows (partial rotation, keys wider than the feed-forward).  One block = one query head x 64 query rows,
+// The same causal attention as prefill_attention_kernel for the decoder's batched prefill where prompt_attention.cu does not serve - an
+// f32 cache without planes of its rows (partial rotation, keys wider than the feed-forward) - or does not pay (short prompts, narrow windows).  One block = one query head x 64 query rows,
 // four warps of 16 rows each; key tiles of 64 positions.  Both contractions run as bf16 MMAs with f32 accumulation, every
 // f32 operand split into a bf16 head and remainder and three of the four partial products kept (16 mantissa bits per
 // operand, a relative 2^-17 per product); with a bf16 cache K and V are exact and two products remain.
@@ -1381,7 +1381,8 @@ int prefill_attention_launch(cudaStream_t stream, const float* q_batch, const fl
     static const bool mma_allowed = [] { const char* v = getenv("KMLL_PREFILL_MMA"); return !(v != nullptr && v[0] == '0'); }();
     const void* k_rows = kv_bf16 ? static_cast<const void*>(k_cache) : k_planes;
     const void* v_rows = kv_bf16 ? static_cast<const void*>(v_cache) : v_planes;
-    if (tensor_cores && mma_allowed && k_rows != nullptr && prompt_attention_serves(q_batch, k_rows, v_rows, out, prompt_len, n_heads, head_dim))
+    if (tensor_cores && mma_allowed && k_rows != nullptr && prompt_attention_pays(prompt_len, window, head_dim, kv_bf16) &&
+        prompt_attention_serves(q_batch, k_rows, v_rows, out, head_dim))
         return prompt_attention_launch(stream, q_batch, k_rows, v_rows, prompt_len, n_heads, n_kv_heads, head_dim, out, kv_bf16, window);
     if (tensor_cores && mma_allowed && (head_dim == 64 || head_dim == 128)) {
         const dim3 grid_mma(n_heads, (prompt_len + 63) / 64);

@@ -168,7 +168,8 @@ int prepare_prefill_offset(cudaStream_t stream, const float* q, const float* k, 
 int write_kv_row(cudaStream_t stream, const float* x, int position, int token_len, int head_dim, float* cache, int kv_bf16);
 // Prompt attention on the tensor cores (prompt_attention.cu): rows of q in f32, 16-byte aligned operands.  `k`, `v`: rows of bf16,
 // [position][n_kv_heads * head_dim] (kv_bf16: the caches) or [position][2][n_kv_heads * head_dim], the two planes of an f32 row.
-bool prompt_attention_serves(const void* q, const void* k, const void* v, const void* out, int prompt_len, int n_heads, int head_dim);
+bool prompt_attention_serves(const void* q, const void* k, const void* v, const void* out, int head_dim);
+bool prompt_attention_pays(int prompt_len, int window, int head_dim, int kv_bf16);  // it is the faster of the two kernels
 int prompt_attention_launch(cudaStream_t stream, const float* q_batch, const void* k, const void* v, int prompt_len, int n_heads, int n_kv_heads,
                             int head_dim, float* out, int kv_bf16, int window);
 // tensor map of a row-major bf16 matrix [rows, inner] with boxes of box_rows rows of 64 entries in the 128-byte swizzle

@@ -515,9 +515,18 @@ int latent_prompt_launch(cudaStream_t stream, const LatentArgs& a) {
     return KMLL_OK;
 }
 
-bool prompt_attention_serves(const void* q, const void* k, const void* v, const void* out, int prompt_len, int n_heads, int head_dim) {
-    (void)prompt_len;
-    (void)n_heads;
+// A block here has 128 rows and costs 11 to 15 us however few keys they see; one of the mma.sync kernel has 64 and costs 3 to 5 a key tile of 64.  So
+// that kernel keeps short prompts and narrow windows.  Both with the rotation in front, which writes the planes of an f32 cache; 8 to
+// 32 heads, here / there in us: heads of 128, 128 tokens 20.2 / 18.4 and 129 tokens 20.2 / 20.9 (32 heads, f32 cache; bf16 20.4 / 19.0 and 19.9 / 19.9); 1024
+// tokens and windows of 64 (two tiles there) 28.3 / 26.5, of 72 (three) 27.9 / 29.0, of 256 32.0 / 46.0.  Heads of 64: 129 tokens 15.9 / 14.8, 192 15.5 /
+// 16.0, 200 16.6 / 18.9; 1024 tokens, f32 cache, windows of 128 19.0 / 19.7, 192 23.7 / 23.6 (2000 tokens 40.4 / 35.3), 256 23.2 / 26.5; bf16 cache, 32 heads, 256 38.3 / 30.7,
+// 384 40.4 / 34.1, 512 39.9 / 39.8 (2000 tokens 73.6 / 77.0).
+bool prompt_attention_pays(int prompt_len, int window, int head_dim, int kv_bf16) {
+    const int shortest = head_dim == 128 ? 129 : 193, narrowest = head_dim == 128 ? 66 : kv_bf16 ? 512 : 256;
+    return prompt_len >= shortest && (window <= 0 || window >= prompt_len || window >= narrowest);
+}
+
+bool prompt_attention_serves(const void* q, const void* k, const void* v, const void* out, int head_dim) {
     const uintptr_t bits = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out);
     return (head_dim == 64 || head_dim == 128) && (bits & 15u) == 0;
 }

@@ -1318,7 +1318,8 @@ int kmll_decoder_prefill(kmll_decoder_t dec, kmll_stream_t stream, const uint32_
             }
             KMLL_TRY(apply_qk_norm(d, s, L, qb, kb, n));
             // An f32 cache's rows as bf16 planes for the attention: in the buffers of gate and up, which are written behind it
-            uint16_t* kp = c.fused && !c.kv_bf16 && d->hidden_l >= kv_len ? reinterpret_cast<uint16_t*>(gb) : nullptr;
+            const bool split = c.fused && !c.kv_bf16 && d->hidden_l >= kv_len && prompt_attention_pays(n, c.sliding_window, c.head_dim, 0);
+            uint16_t* kp = split ? reinterpret_cast<uint16_t*>(gb) : nullptr;
             uint16_t* vp = kp != nullptr ? reinterpret_cast<uint16_t*>(ub) : nullptr;
             bool planes = false;
             KMLL_TRY(prepare_prefill_offset(s, qb, kb, vb, d->freqs, c.rotary_dim / 2, n, q_len, kv_len, c.head_dim, 0, qrb, L.key_cache,

@@ -99,11 +99,11 @@ def test_f32_prompt_attention_matches_oracle(cuda, n, heads, kv, hd, window, kv_
 
 
 @pytest.mark.parametrize("heads,kv,hd", [(4, 2, 64), (4, 1, 128), (8, 8, 128)])
-@pytest.mark.parametrize("window,kv_bf16", [(0, False), (0, True), (1, False), (100, True), (130, False), (300, False)])
+@pytest.mark.parametrize("window,kv_bf16", [(0, False), (0, True), (1, False), (66, False), (100, True), (130, False), (300, False)])
 def test_prompt_attention_tiles_match_oracle(cuda, heads, kv, hd, window, kv_bf16):
     """Attention on tensor memory: prompts that end around the 128 rows of a block and the 128 keys of a tile, one to four tiles (one and
-    two streams of tiles), windows that start inside a tile; (8, 8, 128) has keys wider than the feed-forward, so an f32 cache has
-    no room for planes and keeps the other kernel.  Bounds as in the tests above."""
+    two streams of tiles), windows that start inside a tile; the other kernel on the other side of its lines (length, window), and for
+    (8, 8, 128) with an f32 cache: keys wider than the feed-forward leave no room for planes.  Bounds as in the tests above."""
     n = 390
     cfg = tiny(rt.FORMAT_RS_I8, True, n_layers=1, n_heads=heads, n_kv_heads=kv, head_dim=hd, max_seq_len=n + 8, sliding_window=window, kv_bf16=kv_bf16)
     dec = make(cfg)
@@ -111,7 +111,7 @@ def test_prompt_attention_tiles_match_oracle(cuda, heads, kv, hd, window, kv_bf1
     prompt = np.random.default_rng(heads + hd + window).integers(0, cfg.vocab_size, n)
     for at, token in enumerate(prompt, 1):
         ora.forward(int(token))
-        if at in (1, 2, 64, 127, 128, 129, 255, 256, 257, 383, 384, 385, 390):
+        if at in (1, 2, 64, 127, 128, 129, 192, 193, 255, 256, 257, 383, 384, 385, 390):
             dec.prefill(prompt[:at])
             got = dec.last_hidden()
             scale = max(float(np.max(np.abs(ora.hidden))), 1.0)
@@ -119,14 +119,13 @@ def test_prompt_attention_tiles_match_oracle(cuda, heads, kv, hd, window, kv_bf1
     dec.close()
 
 
-@pytest.mark.parametrize("heads,kv,hd", [(4, 2, 64), (4, 1, 128)])
-@pytest.mark.parametrize("kv_bf16", [False, True])
-def test_prompt_attention_keeps_values_out_of_rows_that_do_not_attend_them(cuda, heads, kv, hd, kv_bf16):
+@pytest.mark.parametrize("heads,kv,hd,kv_bf16,window", [(4, 2, 64, False, 260), (4, 2, 64, True, 520), (4, 1, 128, False, 100), (4, 1, 128, True, 100)])
+def test_prompt_attention_keeps_values_out_of_rows_that_do_not_attend_them(cuda, heads, kv, hd, kv_bf16, window):
     """Token MARK's value overflows to infinity in two columns of a head.  Just in front of the last row's window, in a tile that
     rows of its block do attend, the last row is bit for bit what it is with another token there; inside the window it is not.
     The output projection's scales bring the two columns, about 1e36, back to the size of the residual."""
-    window, mark, columns = 100, 1, [5, hd - 1]
-    cfg = tiny(rt.FORMAT_RS_I8, True, n_layers=1, n_heads=heads, n_kv_heads=kv, head_dim=hd, max_seq_len=400, sliding_window=window, kv_bf16=kv_bf16)
+    mark, columns, whole = 1, [5, hd - 1], (window // 128 + 3) * 128
+    cfg = tiny(rt.FORMAT_RS_I8, True, n_layers=1, n_heads=heads, n_kv_heads=kv, head_dim=hd, max_seq_len=whole + 8, sliding_window=window, kv_bf16=kv_bf16)
     dec = make(cfg)
     rng = np.random.default_rng(hd)
     table = (rng.normal(0, 1, (cfg.vocab_size, cfg.dim)).astype(F).view(np.uint32) >> 16).astype(np.uint16)
@@ -141,7 +140,7 @@ def test_prompt_attention_keeps_values_out_of_rows_that_do_not_attend_them(cuda,
     dec.set_tensor(0, rt.T_WV, values, scales)
     values, scales = dec.get_tensor(0, rt.T_WO)
     dec.set_tensor(0, rt.T_WO, values, np.full_like(scales, 1e-37))
-    prompt = rng.integers(2, cfg.vocab_size, 390)
+    prompt = rng.integers(2, cfg.vocab_size, whole + 6)
 
     def last(n, at):
         p = prompt[:n].copy()
@@ -150,12 +149,12 @@ def test_prompt_attention_keeps_values_out_of_rows_that_do_not_attend_them(cuda,
         dec.prefill(p)
         return dec.last_hidden()
 
-    for n, outside in ((390, (285, 289)), (384, (157, 200, 283))):
+    for n, before in ((whole + 6, (5, 1)), (whole, (127, 84, 1))):
         want = last(n, None)
         assert np.all(np.isfinite(want))
-        for at in outside:
-            np.testing.assert_array_equal(last(n, at), want, err_msg=str((n, at)))
-        assert not np.array_equal(last(n, n - 100), want)
+        for back in before:
+            np.testing.assert_array_equal(last(n, n - window - back), want, err_msg=str((n, back)))
+        assert not np.array_equal(last(n, n - window), want)
     dec.close()
 
 
