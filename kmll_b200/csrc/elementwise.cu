@@ -413,7 +413,9 @@ __global__ void embedding_kernel(const uint16_t* __restrict__ table, int dim, co
 }
 
 // Rows of a prompt, one block each: four entries per thread and step, so the 16-byte stores keep HBM busy (an entry per thread:
-// 2048 x 4096 38 us, now 10).
+// 2048 x 4096 38 us, now 10).  Narrow rows leave most of a block idle and keep the other form: 65536 rows of 128 entries 68 us here, 35 there,
+// of 16 68 / 5, of 256 69 / 69, of 512 69 / 137; 512 rows of 256 1.6 / 1.8.
+constexpr int kWideEmbedding = 256;
 __global__ void __launch_bounds__(256) embedding_rows_kernel(const uint16_t* __restrict__ table, int dim, const uint32_t* __restrict__ tokens, int vocab,
                                                              float* __restrict__ out) {
     pdl_wait();
@@ -894,7 +896,7 @@ int kmll_embedding_tokens(kmll_stream_t s, const uint16_t* table, int vocab, int
     KMLL_REQUIRE(vocab > 0 && dim > 0 && token_count >= 0, "embedding_tokens: shape mismatch");
     if (token_count == 0) return KMLL_OK;
     const size_t total = (size_t)token_count * dim;
-    if ((dim & 3) == 0 && (reinterpret_cast<uintptr_t>(table) & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    if (dim >= kWideEmbedding && (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(table) & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
         KMLL_LAUNCH_CHECK(launch(embedding_rows_kernel, dim3((unsigned)token_count), dim3(256), 0, as_stream(s), true, table, dim, tokens, vocab, out), "embedding_tokens");
         return KMLL_OK;
     }

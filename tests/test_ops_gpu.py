@@ -570,9 +570,9 @@ def test_embedding_vs_oracle(cuda):
         ops.embedding_tokens_bf16(t, dev(toks), 5, 96)  # token buffer too short
 
 
-@pytest.mark.parametrize("dim", [1, 5, 8, 1020, 1028, 4100])
+@pytest.mark.parametrize("dim", [1, 5, 8, 252, 256, 257, 1020, 1028, 4100])
 def test_embedding_rows_of_any_width(cuda, dim):
-    """Rows in pieces of four entries (fewer pieces than threads, more, a ragged last round) and rows that are not: exact."""
+    """Rows in pieces of four entries (fewer pieces than threads, more, a ragged last round), narrow rows and rows that are not: exact."""
     rng = np.random.default_rng(dim)
     table = oracle.bf16_from_f32(rng.normal(0, 1, (37, dim)).astype(F))
     toks = rng.integers(0, 37, 11).astype(np.uint32)
