@@ -570,6 +570,7 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
     if (warp == 0) {
         const uint32_t lead = elect_lead();
         PairRing ring(stages);
+        int issued = 0;
         for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
             const int tile = item / p.ksplit, kt0 = (item % p.ksplit) * kt_per, kt1 = min(kt0 + kt_per, KT);
             const int row0 = (tile / p.x_tiles) * kHRows, t0 = (tile % p.x_tiles) * p.n_block;
@@ -581,8 +582,10 @@ __global__ void __launch_bounds__(kHThreads, 1) linear_gemm_bf16_kernel(const Ge
                 lead_expect_tx(lead, &full[s], (uint32_t)stage_bytes);
                 lead_tma_2d(lead, st, &map_w, kt * kHKT, row0, &full[s]);
                 lead_tma_2d(lead, st + a_bytes, &map_x, kt * kHKT, t0, &full[s]);
+                ++issued;
             }
         }
+        if (!ok) ring_landed(full, issued, stages);
     } else if (warp == 1) {
         const uint32_t lead = elect_lead();
         PairRing ring(stages);

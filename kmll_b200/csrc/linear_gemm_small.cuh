@@ -378,6 +378,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
         if (cur.start(p, blockIdx.x, G)) {
             const uint32_t lead = elect_lead();
             RingPos<S::kRawSlots> rp;
+            int it = 0;
             PROF_DECL;
             do {
                 PROF_W0;
@@ -388,7 +389,9 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                 lead_expect_tx(lead, &raw_full[rp.idx], (uint32_t)S::kRawBytes);
                 lead_tma_2d(lead, smem_base + (uint32_t)rp.idx * S::kRawBytes, map, cur.g * 64, (cur.tile - p.mat[mi].tile_start) * 128, &raw_full[rp.idx]);
                 rp.next();
+                ++it;
             } while (cur.advance(p, G, GP));
+            if (!ok) ring_landed(raw_full, it, S::kRawSlots);
             if (lane == 0) PROF_END(0);
         }
     } else if (warp == 19) {
@@ -411,6 +414,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
                 xp.next();
                 ++it;
             } while (cur.advance(p, G, GP));
+            if (!ok) ring_landed(x_full, it, S::kXSlots);
             if (lane == 0) PROF_END(1);
         }
     } else if (warp >= 16) {
@@ -740,6 +744,7 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
                 sp.next();
                 ++it;
             } while (cur.advance(p, G));
+            if (!ok) ring_landed(full, it, S::kStages);
         }
     } else if (warp == 0 || warp == 11) {
         const int set = warp == 0 ? 0 : 1;

@@ -71,11 +71,6 @@ __device__ inline void pa_split8(const float (&v)[8], uint4& hi, uint4& lo) {
 __device__ inline uint64_t pa_desc_mn(uint32_t smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(kPaBox >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// The last of the first `issued` tiles that uses stage st of `stages`, -1: none.
-__host__ __device__ constexpr int pa_last_use(int issued, int st, int stages) { return issued <= st ? -1 : st + (issued - 1 - st) / stages * stages; }
-static_assert(pa_last_use(0, 0, 1) == -1 && pa_last_use(1, 0, 1) == 0 && pa_last_use(7, 0, 1) == 6, "one stage");
-static_assert(pa_last_use(0, 0, 2) == -1 && pa_last_use(1, 0, 2) == 0 && pa_last_use(1, 1, 2) == -1 && pa_last_use(2, 1, 2) == 1, "two stages, first uses");
-static_assert(pa_last_use(5, 0, 2) == 4 && pa_last_use(5, 1, 2) == 3 && pa_last_use(6, 0, 2) == 4 && pa_last_use(6, 1, 2) == 5, "two stages, later uses");
 // Values that are not finite.  A key that a row does not attend has weight 0 there, and 0 * infinity is NaN.  So in the tiles that some
 // row does not see in full - at most three: the first (window) and the last two (causal) - such entries become zeros ahead of the
 // MMAs and are noted, a bit per (column, key); at the end an output whose row attends one of them becomes NaN.
@@ -209,11 +204,7 @@ __device__ inline void prompt_attention_block(const Src& src, const PaRange& rg,
             if (!ok) break;
         }
         for (int j = max(tiles - (kStages - 1), 0); j < tiles && !keys && ok; ++j) ok = look_through(j);
-        // what was requested has landed before the block ends, after a time-out too: the last use of each stage that was begun
-        for (int st = 0; st < kStages; ++st) {
-            const int last = pa_last_use(issued, st, kStages);
-            if (last >= 0 && !warp_wait(&full[st], (uint32_t)(last / kStages) & 1u)) ok = false;
-        }
+        ok = ring_landed(full, issued, kStages) && ok;  // (after a time-out too)
     } else if (warp == 10) {
         constexpr uint32_t idesc_s = gemm_idesc_bf16(128, kPaKeys), idesc_o = gemm_idesc_bf16(128, DV) | (1u << 16);  // V is MN-major
         const uint64_t dq = gemm_smem_desc(base), dk = gemm_smem_desc(base + S::kOffK), dv = pa_desc_mn(base + S::kOffV);

@@ -69,6 +69,21 @@ __device__ inline uint32_t elect_lead() {
 }
 // all lanes leave a bounded wait together
 __device__ inline bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait<false>(bar, parity)) != 0; }
+// The last of the first `issued` uses of a ring of `stages` that is one of stage st; -1: none.
+__host__ __device__ constexpr int ring_last_use(int issued, int st, int stages) { return issued <= st ? -1 : st + (issued - 1 - st) / stages * stages; }
+static_assert(ring_last_use(0, 0, 1) == -1 && ring_last_use(1, 0, 1) == 0 && ring_last_use(7, 0, 1) == 6, "one stage");
+static_assert(ring_last_use(0, 0, 2) == -1 && ring_last_use(1, 0, 2) == 0 && ring_last_use(1, 1, 2) == -1 && ring_last_use(2, 1, 2) == 1, "two stages, first uses");
+static_assert(ring_last_use(5, 0, 2) == 4 && ring_last_use(5, 1, 2) == 3 && ring_last_use(20, 1, 9) == 19 && ring_last_use(20, 2, 9) == 11, "later uses");
+// A block does not end with copies under way: whoever began the copies of the first `issued` uses of a ring waits, before it leaves its
+// role after a time-out, for the last one of each stage.  (It has seen the uses before end, so the parity is that one's.)
+__device__ inline bool ring_landed(uint64_t* full, int issued, int stages) {
+    bool ok = true;
+    for (int st = 0; st < stages; ++st) {
+        const int last = ring_last_use(issued, st, stages);
+        if (last >= 0) ok = warp_wait(&full[st], (uint32_t)(last / stages) & 1u) && ok;
+    }
+    return ok;
+}
 __device__ inline void lead_mma_f16(uint32_t lead, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
