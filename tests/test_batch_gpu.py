@@ -53,29 +53,41 @@ def test_batch_matches_single_sequence(cuda, fmt, batch):
 @pytest.mark.parametrize("fmt", [rt.FORMAT_RS_I8, rt.FORMAT_W4G128])
 @pytest.mark.parametrize("vocab,batch", [(641, 7), (4100, 9), (16388, 2)])
 def test_batch_arg_max_over_ragged_rows(cuda, fmt, vocab, batch):
-    """Logits rows that are and are not whole 16-byte pieces (fewer pieces than threads, more, a last round of one): the step's
-    token is the arg-max that the single-sequence decoder finds for the same prompt, and so is its logit."""
+    """Logits rows that are and are not whole 16-byte pieces (fewer pieces than threads, more, a last round of one).  Behind token
+    `start` five rows of the output matrix - two, their negatives, one more - repeat to the end, in front of it the logits are zero: a
+    positive maximum with exact ties in other pieces and other threads, whose lowest token is one of the five at `start`.  Every token
+    is the one that the single-sequence decoder takes."""
     cfg = _cfg(fmt, vocab_size=vocab)
     dec = rt.Decoder(cfg)
     dec.init_random(11, 0.05, False)
+    values, scales = dec.get_tensor(-1, rt.T_OUTPUT)
     rng = np.random.default_rng(vocab)
     prompts = [rng.integers(0, vocab, 9) for _ in range(batch)]
-    singles = []
-    for p in prompts:
-        dec.prefill(p)
-        singles.append([v.copy() for v in dec.generate_greedy(3)])
-    bd = rt.BatchDecoder(dec, batch)
-    for slot, p in enumerate(prompts):
-        dec.prefill(p)
-        bd.adopt(slot)
-    tokens, logits = bd.generate_greedy(3)
-    for slot, (ref_t, ref_l) in enumerate(singles):
-        for i in range(3):
-            tol = 2e-3 * max(1.0, abs(float(ref_l[i])))  # two kernels of f32 sums over 256 and 512 columns, as above
-            assert abs(float(logits[slot, i]) - float(ref_l[i])) <= tol, (slot, i)
-            if int(tokens[slot, i]) != int(ref_t[i]):  # a near-tie: the sequences part
-                break
-    bd.close()
+    taken = set()
+    for start in (0, 1027 if vocab > 1032 else 130, vocab // 2 + 1, vocab - 5):
+        place = (np.arange(vocab) - start) % 5
+        s = scales[place // 2].copy()  # rows 0, -0, 1, -1, 2
+        negative = np.isin(place, (1, 3))
+        s[negative] = s[negative] ^ np.uint16(0x8000) if s.dtype == np.uint16 else -s[negative]
+        s[:start] = 0
+        dec.set_tensor(-1, rt.T_OUTPUT, values[place // 2], s)
+        singles = []
+        for p in prompts:
+            dec.prefill(p)
+            singles.append([v.copy() for v in dec.generate_greedy(5)])
+        bd = rt.BatchDecoder(dec, batch)
+        for slot, p in enumerate(prompts):
+            dec.prefill(p)
+            bd.adopt(slot)
+        tokens, logits = bd.generate_greedy(5)
+        for slot, (ref_t, ref_l) in enumerate(singles):
+            assert [int(t) for t in tokens[slot]] == [int(t) for t in ref_t], (start, slot)
+            assert all(start <= int(t) < start + 5 for t in tokens[slot]), (start, slot)
+            # two kernels of f32 sums over 256 and 512 columns, as above
+            assert np.all(np.abs(logits[slot] - ref_l) <= 2e-3 * np.maximum(1.0, np.abs(ref_l))), (start, slot)
+            taken |= {int(t) - start for t in tokens[slot]}
+        bd.close()
+    assert len(taken) >= 3  # several elements of a piece
     dec.close()
 
 

@@ -595,6 +595,127 @@ def test_norm_weights_of_the_launch_in_front(cuda):
         assert float((call(n).double() - w0 @ value(n.double())).abs().max()) <= 4e-5 * cols ** 0.5
 
 
+@pytest.mark.parametrize("cols", [256, 384, 4096, 4224, 8192, 8320])
+def test_mixer_output_of_whole_heads(cuda, cols):
+    """The output projection of mixers whose heads are runs of 128 columns (all of x in whole pieces), of 8192 columns, of more and with
+    heads of 256 (one column at a time): every norm, gates by column and by head, one and two mixers, x on and off a 16-byte
+    boundary.  Bound: f32 sums of `cols` products around 1, as in test_bf16_linear_operators."""
+    import torch
+
+    from kmll_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    eps, rows = 1e-3, 70
+    w = (torch.randn(rows, cols, generator=gen, device="cuda") / cols ** 0.5).bfloat16()
+    res = torch.randn(rows, generator=gen, device="cuda")
+    act = {rt.ACT_SILU: torch.nn.functional.silu, rt.ACT_SIGMOID: torch.sigmoid}
+
+    def attention(heads, vdim):
+        return rt.MixerSpec(rt.MIXER_ATTENTION, heads, 64, vdim, gate_act=rt.ACT_SIGMOID, out_scale=0.6)
+
+    def linear(heads, norm, vdim=128):
+        return rt.MixerSpec(rt.MIXER_GATED_LINEAR, heads, 64, vdim, gate_act=rt.ACT_SILU, out_scale=1.3, out_norm=norm)
+
+    norms = (rt.OUT_NORM_PER_HEAD, rt.OUT_NORM_JOINT, rt.OUT_NORM_HEAD_WEIGHTED, rt.OUT_NORM_NONE)
+    n = cols // 128
+    cases = [[linear(n, norm)] for norm in norms] + [[attention(n, 128)]]
+    cases += [[attention(1, 128), linear(n - 1, norm)] for norm in norms] + [[linear(n - 1, norm), attention(1, 128)] for norm in norms]
+    cases += [[linear(1, a), linear(n - 1, b)] for a in norms for b in norms]
+    if n % 2 == 0:
+        cases += [[linear(n // 2, norm, 256)] for norm in norms] + [[attention(n // 2, 256)]]
+        if n > 2:
+            cases += [[attention(1, 256), linear(n - 2, norm)] for norm in norms]
+    for case, mixers in enumerate(cases):
+        x = torch.randn(cols + 1, generator=gen, device="cuda")
+        x = x[1:] if case % 4 == 3 else x[:cols]
+        weights, gates, parts, at = [], [], [], 0
+        for m in mixers:
+            o = x[at:at + m.heads * m.vdim].double().view(m.heads, m.vdim)
+            at += m.heads * m.vdim
+            whole = m.mixer == rt.MIXER_ATTENTION
+            norm = rt.OUT_NORM_NONE if whole else m.out_norm
+            gates.append(torch.randn(m.heads if whole else m.heads * m.vdim, generator=gen, device="cuda"))
+            weight = None
+            if norm in (rt.OUT_NORM_JOINT, rt.OUT_NORM_HEAD_WEIGHTED):
+                weight = (torch.randn(m.vdim * (m.heads if norm == rt.OUT_NORM_JOINT else 1), generator=gen, device="cuda") + 1.0).bfloat16()
+            weights.append(weight)
+            if norm == rt.OUT_NORM_JOINT:
+                o = o / (o.square().mean() + eps).sqrt() * weight.double().view(m.heads, m.vdim)
+            elif norm != rt.OUT_NORM_NONE:
+                o = o / (o.square().mean(1, keepdim=True) + eps).sqrt()
+                if weight is not None:
+                    o = o * weight.double()
+            parts.append((o * act[m.gate_act](gates[-1].double()).view(m.heads, -1) * m.out_scale).reshape(-1))
+        got = ops.mixer_output_linear_bf16(mixers, x, weights, gates, w, eps, residual=res)
+        want = w.double() @ torch.cat(parts) + res.double()
+        assert float((got.double() - want).abs().max()) <= 4e-5 * cols ** 0.5, (case, mixers)
+
+
+@pytest.mark.parametrize("cols", [4096, 4104, 8200])
+def test_norm_of_long_and_unaligned_rows(cuda, cols):
+    """Norms over what a thread can hold in whole pieces (4096 columns), over more, and of an x that is off a 16-byte boundary."""
+    import torch
+
+    from kmll_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    w = (torch.randn(50, cols, generator=gen, device="cuda") / cols ** 0.5).bfloat16()
+    nw, nb = (torch.randn(cols, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    coef = torch.randn(4, generator=gen, device="cuda").bfloat16()
+    for off in (0, 1):
+        x = (torch.randn(cols + 1, generator=gen, device="cuda") * 2 + 0.5)[off:off + cols]
+        X = x.double()
+        for got, n in ((ops.linear_bf16(x, w, norm_weight=nw, norm_offset=1.0, eps=1e-3), lo.rms_norm_zero_centred(X.cpu().numpy(), nw.double().cpu().numpy(), 1e-3)),
+                       (ops.normed_linear_bf16(x, w, rt.NORM_LAYER, nw, nb, 1e-3),
+                        ((X - X.mean()) / (X.var(unbiased=False) + 1e-3).sqrt() * nw.double() + nb.double()).cpu().numpy()),
+                       (ops.polynorm_linear_bf16(x, coef, 1e-3, w), lo.poly_norm(X.cpu().numpy(), coef.double().cpu().numpy(), 1e-3))):
+            assert float((got.double() - w.double() @ torch.from_numpy(n).cuda()).abs().max()) <= 6e-5 * cols ** 0.5, off
+
+
+@pytest.mark.parametrize("tokens,position,window", [(1, 0, 0), (130, 0, 0), (300, 0, 1000), (257, 130, 0), (390, 250, 300), (128, 900, 200), (5, 700, 129)])
+def test_latent_prompt_operator_with_growing_scores(cuda, tokens, position, window):
+    """Latent attention of a prompt against 64-bit sums over the same bf16 operands.  Keys of the later tiles are longer, so row maxima grow
+    by many powers of two from tile to tile, in some rows more than in others; a last case in each head has keys that shrink instead.
+    Bound: a score is a sum of exact products in f32, 12 steps of 16 columns that each lose 2^-23 of the sum of magnitudes, and its weight
+    follows it; a weight is two bf16 planes (2^-16).  Both enter sum and divisor, hence the two."""
+    import torch
+
+    from kmll_b200 import ops
+
+    heads, dim, rot, vdim, rank, max_seq = 3, 128, 64, 128, 64, 1100
+    gen = torch.Generator(device="cuda").manual_seed(tokens + window)
+    seen = position + tokens
+    first = max(0, position - window + 1) if window else 0
+    length = torch.linspace(0.2, 6.0, seen, device="cuda")
+    k = torch.randn(seen, heads, dim, generator=gen, device="cuda") * torch.stack([length, length, length.flip(0)], 1)[:, :, None]
+    v = torch.randn(seen, heads, vdim, generator=gen, device="cuda")
+    expanded = torch.cat([k.reshape(seen, -1), v.reshape(seen, -1)], 1).bfloat16()[first:].contiguous()
+    cache = torch.zeros(max_seq, rank + rot, device="cuda", dtype=torch.bfloat16)
+    cache[:seen, rank:] = torch.randn(seen, rot, generator=gen, device="cuda").bfloat16()
+    angle = torch.rand(max_seq, rot // 2, generator=gen, device="cuda") * 6.28
+    turn = (torch.stack([angle.cos(), angle.sin()], 2) * 16).round().contiguous() / 16  # (rotated entries are exact in f32, whatever the order)
+    x = torch.randn(tokens, heads * (dim + rot) + 8, generator=gen, device="cuda").bfloat16()
+    scale = 192 ** -0.5 * 1.7
+    out = ops.latent_attention_prefill(x, position, heads, dim, rot, vdim, rank, window, scale, turn, cache, expanded, first).double()
+    q = x[:, :heads * (dim + rot)].float().view(tokens, heads, dim + rot)
+    c, s = (turn[position:seen, None, :, i] for i in range(2))
+    u, z = q[:, :, dim:dim + rot // 2], q[:, :, dim + rot // 2:]
+    q = torch.cat([q[:, :, :dim], u * c - z * s, z * c + u * s], 2).bfloat16().double()
+    both = expanded.double()
+    K, V = both[:, :heads * dim].view(-1, heads, dim), both[:, heads * dim:].view(-1, heads, vdim)
+    K = torch.cat([K, cache[first:seen, None, rank:].double().expand(-1, heads, -1)], 2)
+    scores = torch.einsum("thd,shd->hts", q, K) * scale
+    at, of = torch.arange(position, seen, device="cuda")[:, None], torch.arange(first, seen, device="cuda")[None]
+    hidden = (of > at) | (of <= at - window if window else torch.zeros_like(of, dtype=torch.bool))
+    weights = torch.softmax(scores.masked_fill(hidden, float("-inf")), 2)
+    want = torch.einsum("hts,shd->thd", weights, V)
+    spread = torch.einsum("hts,shd->thd", weights, V.abs())
+    size = torch.einsum("thd,shd->hts", q.abs(), K.abs()) * scale
+    slack = (size.masked_fill(hidden, 0.0).amax(2) * 12 * 2.0 ** -23 + 2.0 ** -16).T[:, :, None]
+    rel = ((out.view(tokens, heads, vdim) - want).abs() / (spread * slack * 2)).amax()
+    assert float(rel) <= 1.0, float(rel)
+
+
 # more than 256 rows of x: pairs of blocks.  One k-tile (one accumulator), a ragged last one, one row of weights, ragged tiles on both
 # sides, several units per pair
 @pytest.mark.parametrize("tokens,rows,cols", [(257, 130, 72), (300, 2, 64), (513, 520, 200), (640, 257, 1000), (1030, 6000, 136), (2500, 384, 4104)])

@@ -119,6 +119,60 @@ def test_prompt_attention_tiles_match_oracle(cuda, heads, kv, hd, window, kv_bf1
     dec.close()
 
 
+# strength (by MARK token) of the mark in each key tile, 0: none.  Each stream of tiles (even, odd) sees its maximum grow late, early, in every
+# tile, not at all; equal marks in one stream and in both
+PEAKS = [(0, 0, 0, 0, 1), (0, 0, 0, 1, 0), (4, 3, 2, 1, 0), (1, 2, 3, 4, 0), (0, 1, 1, 0, 0), (1, 0, 0, 0, 1), (4, 0, 2, 0, 1), (0, 4, 0, 2, 1), (4, 4, 3, 3, 3)]
+
+
+@pytest.mark.parametrize("heads,kv,hd", [(4, 2, 64), (4, 1, 128)])
+@pytest.mark.parametrize("kv_bf16", [False, True])
+def test_prompt_attention_with_keys_that_stand_out(cuda, heads, kv, hd, kv_bf16):
+    """Scores of token ASK's query with the keys of MARK tokens are 60, 30, 15 and 7.5 (85, 42, 21 and 10 powers of two), of everything
+    else about 0: the running maximum grows by more than 2^8 in the tiles that PEAKS says, in the rows that ask and not in the others
+    of their warps, and the two streams meet with maxima far apart.  The scores come from one pair of entries that the rotation
+    turns by 5e-4 at most; rounding of q and k moves them by 60 * 2^-16, so weights and attention by 1e-3 of themselves, a tenth of that of
+    the hidden state (a mark's value is a tenth of it at most): the bounds of the tests above."""
+    n, ask, pair = 640, 5, hd // 2 - 1
+    cfg = tiny(rt.FORMAT_RS_I8, True, n_layers=1, n_heads=heads, n_kv_heads=kv, head_dim=hd, max_seq_len=n + 8, kv_bf16=kv_bf16)
+    dec = make(cfg)
+    rng = np.random.default_rng(hd + kv_bf16)
+    table = (rng.normal(0, 1, (cfg.vocab_size, cfg.dim)).astype(F).view(np.uint32) >> 16).astype(np.uint16)
+    table[:, 1:6] = 0
+    table[1:6] = 0
+    table[np.arange(1, 6), np.arange(1, 6)] = 0x4180  # 16: the norm leaves the whole row in this entry
+    dec.set_tensor(-1, rt.T_EMBEDDING, table)
+    dec.set_tensor(0, rt.T_ATTENTION_NORM, np.full(cfg.dim, 0x3f80, dtype=np.uint16))
+    for tensor, count in ((rt.T_WQ, heads), (rt.T_WK, kv)):
+        values, scales = dec.get_tensor(0, tensor)
+        for h in range(count):
+            rows = [h * hd + pair, h * hd + hd - 1]
+            values[rows] = 0
+            if tensor == rt.T_WQ:
+                values[rows[0], ask] = 127
+            else:
+                values[rows[0], 1:5] = (127, 64, 32, 16)
+            scales[rows] = (60 * hd ** 0.5) ** 0.5 / (127 * 16)
+        dec.set_tensor(0, tensor, values, scales)
+    for peaks in PEAKS:
+        prompt = rng.integers(6, cfg.vocab_size, n)
+        prompt[rng.random(n) < 0.3] = ask
+        for tile, mark in enumerate(peaks):
+            if mark:
+                prompt[tile * 128 + int(rng.integers(3, 120))] = mark
+        ora = OracleDecoder(cfg, dec)
+        ends = {257, 300, 384, 385, 500, 512, 513, 600, 638, 640}
+        for at, token in enumerate(prompt, 1):
+            if at in ends:
+                token = prompt[at - 1] = ask if at != 638 else 7
+            ora.forward(int(token))
+            if at in ends:
+                dec.prefill(prompt[:at])
+                scale = max(float(np.max(np.abs(ora.hidden))), 1.0)
+                worst = float(np.max(np.abs(dec.last_hidden() - ora.hidden))) / scale
+                assert worst <= (BF16_KV_BOUND["hid_tol"] if kv_bf16 else 2e-4), (peaks, at, worst)
+    dec.close()
+
+
 @pytest.mark.parametrize("heads,kv,hd,kv_bf16,window", [(4, 2, 64, False, 260), (4, 2, 64, True, 520), (4, 1, 128, False, 100), (4, 1, 128, True, 100)])
 def test_prompt_attention_keeps_values_out_of_rows_that_do_not_attend_them(cuda, heads, kv, hd, kv_bf16, window):
     """Token MARK's value overflows to infinity in two columns of a head.  Just in front of the last row's window, in a tile that
