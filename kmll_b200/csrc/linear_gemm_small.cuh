@@ -21,8 +21,8 @@
 // 4096 x 14336 18.8 / 17.5, 32 rows and 4096 x 4096 19.6 / 15.3.  With the expanded tiles in tensor memory 27.9, 10.9 and 18.2; with half
 // the instructions in the drain (two digits to an integer, integers to f32 by conversion) 24.7, 10.5 and 17.3 (32 rows, 14336 x 4096: 28.5 us at first, 24.1, now 18.6): the issue slots
 // that expansion and drain share are what bounds a group now.
-//   * raw weight tiles (128 rows x 64 bytes of nibbles, TMA by warp 8): 12 slots (7 with 32 rows of x) - they wait out the HBM latency;
-//   * digit planes of the same 128 columns (one 3-D TMA box, 128-byte swizzle, warp 4): 5 or 6 slots - L2 latency;
+//   * raw weight tiles (128 rows x 64 bytes of nibbles a group): as many slots as fit - they wait out the HBM latency;
+//   * digit planes of the same 128 columns (one 3-D TMA box a group, 128-byte swizzle): 4 slots - L2 latency;
 //   * signed-byte weight tiles in tensor memory (lane = weight row, a column = four bytes of K): 4 slots, written by two sets of four
 //     expanding warps (seven integer instructions per word; the even and odd columns of a word come out as two runs, the
 //     digit planes are stored in that column order).  In shared memory they were written and read through the port that the
@@ -38,7 +38,8 @@
 //   split order, so results are bit-identical from call to call).
 // Because an accumulator lives for one group only, the pipeline runs on across unit boundaries without draining.
 // Tensor maps cover this GPU's memory only; no multicast.  Every wait is bounded (mbar_wait); a time-out raises the device
-// status word, and the block frees its tensor memory and returns.  There is no blocking hardware barrier inside the loops.
+// status word, and the block waits for the copies it began, frees its tensor memory and returns.  There is no blocking hardware barrier
+// inside the loops, so a time-out in one warp can never leave another warp waiting forever.
 // Compiled with -DKMLL_ROLE_PROFILE, block 0 records per role the cycles spent waiting and in all (the figures above).
 #pragma once
 
@@ -366,9 +367,8 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
     const uint32_t smem_base = smem_u32(ssmem);
     bool ok = true;
     // the `done` barrier and parity that report the completion of item number n of this block
-    auto done_wait = [&](int n) { return mbar_wait<false>(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
     auto done_warp_wait = [&](int n) { return warp_wait(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
-    static_assert(kBtDoneRing == 16, "done_wait shifts by 4");
+    static_assert(kBtDoneRing == 16, "done_warp_wait shifts by 4");
     UnitCursor cur;
 
     if (warp == 18) {
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
             if (lane == 0) PROF_END(1);
         }
     } else if (warp >= 16) {
-        // ---- MMA issuers: one thread of each of two warps, alternate items (their accumulators are different buffers, so
+        // ---- MMA issuers: two warps, alternate items (their accumulators are different buffers, so
         // no order is needed between them).  Per item: the tiles are expanded, the digit planes have landed, the accumulator
         // buffer has been read out; four MMAs per group; one commit.
         const int set = warp - 16;
@@ -659,8 +659,8 @@ __global__ void __launch_bounds__(kBtThreads, 1) linear_gemm_small_kernel(const 
 // The int8 weights are MMA operands exactly as they lie in memory: TMA writes 128 rows x 128 bytes with the 128-byte
 // swizzle and the tensor core reads them; no thread touches a weight.  One row scale per output, so the s32 accumulators
 // run over the whole K range of a unit (|sum| <= 127 * 128 * K < 2^31 for K <= 131072) and are read once per unit.
-// Two MMA-issuing threads take the groups alternately; each keeps its OWN accumulator (the first MMA of a unit overwrites,
-// and nothing orders the two threads), the drain adds the two.  Buffers alternate with the unit's parity, so the MMAs of
+// Two MMA-issuing warps take the groups alternately; each keeps its OWN accumulator (the first MMA of a unit overwrites,
+// and nothing orders the two), the drain adds the two.  Buffers alternate with the unit's parity, so the MMAs of
 // the next unit run while the previous one is read out.
 //   warps 0, 11: MMA     warp 4: TMA digit planes     warp 8: TMA weights     warps 12..15: drain     others: idle
 template <int NB>
@@ -715,14 +715,16 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t smem_base = smem_u32(ssmem);
     bool ok = true;
-    auto done_wait = [&](int n) { return mbar_wait<false>(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
     auto done_warp_wait = [&](int n) { return warp_wait(&done[n & (kBtDoneRing - 1)], (uint32_t)(n >> 4) & 1u); };
     UnitCursor cur;
 
     if (warp == 4 || warp == 8) {
         // ---- TMA producers: a stage is free when the group that used it last (kStages back) has been multiplied.
-        // (Two alternating threads per stream were tried: no faster, and one run of a 250-tile matrix ended in a launch
-        // failure whose cause was not found by reading; the single-thread form below is the one that has run every shape.)
+        // (One warp per stream, which requests in order.  Two alternating ones were tried, no faster, and one run of a 250-tile matrix ended
+        // in a launch failure.  Nothing ordered their requests, so an issuer could wait by the parity of a slot's use after next before the
+        // use between, the other issuer's, had been requested: it multiplied what lay there and reported the slot free, copies were
+        // requested into a slot that others were still bound for, and at the end some were under way that nobody waited for.  The
+        // issuers below look back at that use.)
         const bool digits = warp == 4;
         if (digits) pdl_wait();  // the digit planes come from the previous kernel; the weights never change
         if (cur.start(p, blockIdx.x, G)) {
@@ -792,7 +794,7 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
         uint32_t drain_phase = 0;
         pdl_wait();
         if (cur.start(p, blockIdx.x, G)) {
-            int it = 0, unit_no = 0;
+            int unit_no = 0;
             bool more = true;
             while (more && ok) {
                 const int tile = cur.tile, z = cur.z;
@@ -800,13 +802,11 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
                 const int mi = (p.nmat > 2 && tile >= p.mat[2].tile_start) ? 2 : (p.nmat > 1 && tile >= p.mat[1].tile_start) ? 1 : 0;
                 const SmallMat& mt = p.mat[mi];
                 const int row = (tile - mt.tile_start) * 128 + rl;
-                const int it_first = it;
-                it += n_items;
                 for (int k = 0; k < n_items && more; ++k) more = cur.advance(p, G);
                 const int par = unit_no & 1;
                 if (!warp_wait(&unit_done[par], (uint32_t)(unit_no >> 1) & 1u)) { ok = false; break; }
                 tcgen05_fence_after();
-                // which thread took the first group of the unit decides nothing here: both accumulators are simply added
+                // which warp took the first group of the unit decides nothing here: both accumulators are simply added
                 const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((par * 2 + 0) * kN);
                 const uint32_t tb = ta + (uint32_t)kN;
                 float acc[NB];
@@ -830,7 +830,6 @@ __global__ void __launch_bounds__(512, 1) linear_gemm_small_i8_kernel(const Smal
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&tmem_free[par]);
-                (void)it_first;
                 const float rscale = row < mt.rows ? mt.row_scales[row] : 0.0f;
                 if (p.ksplit == 1) {
                     small_store<NB, 8>(p, mt, row, rscale, acc);

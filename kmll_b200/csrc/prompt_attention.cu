@@ -14,14 +14,14 @@
 //                   through the values of tiles that some row does not see in full (PaHeld)
 //   warp 10         issues S = Q K^T (both operands in shared memory) and O += P V (P from tensor memory)
 // Bound by the tensor cores with f32 operands (48 MMAs of 61 cycles a tile; a fifth of the issuer's time is waiting), by the second pass of
-// the softmax (3460 cycles of its warps per tile, exponentials and conversions) with bf16 ones.  Measured against the mma.sync
-// kernel, 32 heads of 128: 2048 tokens, f32 cache 364 -> 112 us, bf16 cache -> 98 us.  A block costs ~5 us beside its
-// tiles (Q planes, first copies, rows out): 1 token 11 us, 640 tokens 27 us with launch gaps.  Built before and slower: eight
+// the softmax (3460 cycles of its warps per tile, exponentials and conversions) with bf16 ones; all threads are held to 168 registers, and
+// the softmax spills 12 to 60 bytes of them.  Profiled against the mma.sync kernel, 32 heads of 128: 2000 tokens, f32 cache 363 -> 125 us, bf16
+// cache 279 -> 108; 512 tokens 48 -> 24 and 41 -> 21.  A block costs 11 to 15 us beside its tiles (prompt_attention_pays).  Built before and slower: eight
 // warps that convert keys and values of an f32 cache themselves, every block again, instead of TMA of planes written once (262 us).
 // Order of the MMAs: S0 S1, P0V0 S2, P1V1 S3, ...  O is rescaled only when a row's maximum has grown by more than 2^8 since the last
 // time (larger weights cost no precision: every plane is relative), which after the first tiles hardly happens.
-// Blocks with the most keys start first.  Every wait is bounded; a time-out raises the status word, and the block frees its
-// tensor memory and returns.
+// Blocks with the most keys start first.  Every wait is bounded; a time-out raises the status word, and the block waits for the copies it
+// began, frees its tensor memory and returns.
 #include <cuda.h>
 
 #include "internal.cuh"

@@ -22,9 +22,8 @@ __device__ inline bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait; false = timed out (the caller raises the status word and unwinds).  There is no
-// blocking hardware barrier anywhere in the kernel, so a time-out in one warp can never leave
-// another warp waiting forever.
+// Bounded wait; false = timed out (the caller raises the status word and unwinds).  Roles meet at hardware barriers only where every warp
+// comes by, time-out or not: ahead of the roles' loops and behind them.
 template <bool BACKOFF = true>
 __device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
